@@ -6,6 +6,7 @@
 // runtime's library API.
 #include <cuda_runtime.h>
 #include <dlfcn.h>
+#include <math.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <string.h>
@@ -247,6 +248,9 @@ extern "C" int spinsim_plan_create(const spinsim_plan_desc* desc, const void* fi
     p->m.rotating = d.rotating ? 1 : 0;
     p->m.hypercubes = h;
     p->m.precision = ldexp(1.0, 2 * h);  // 4 ** h, I:1550
+    // The symmetric splitting of N = 4^h factors differs from the exponential by less than
+    // |g|^3 / (8 N^2); at |g|^3 <= 2^-53 N^2 that is an eighth of a rounding error.
+    p->m.lt_norm2_max = pow(ldexp(1.0, 4 * h - 53), 2.0 / 3.0);
     p->m.lanes = d.lanes;
     if (d.threads_per_block) p->block = d.threads_per_block;
 
@@ -919,7 +923,10 @@ static void fill_evolve_tiles(const spinsim_plan* p, const Instance* inst, int32
     std::vector<Run> runs;
     runs.reserve(2 * (size_t)n);
     for (int i = 0; i < n; i++) {
-        const double step_cost = inst[i].dim == 3 ? 4.0 + 0.5 * p->m.hypercubes : 1.0;
+        // a spin-one step costs about a spin-half one (SU(2) elements), more with a quadratic shift, and
+        // its squarings with the eight-generator exponential
+        const double step_cost =
+            inst[i].dim == 2 ? 1.0 : p->m.expo_one == EXPO_LIE_TROTTER_8 ? 4.0 + 0.5 * p->m.hypercubes : 1.5;
         const int64_t full = inst[i].n_out / per_warp, rest = inst[i].n_out % per_warp;
         if (full) runs.push_back({step_cost * inst[i].n_fine * per_warp, i, per_warp, 0, full});
         if (rest) runs.push_back({step_cost * inst[i].n_fine * rest, i, (int32_t)rest, full * per_warp, 1});

@@ -88,6 +88,7 @@ struct MethodConfig {
     int32_t hypercubes;     // ceil(number_of_squares / 2), >= 0  (I:1547-1549)
     int32_t lanes;          // lanes sharing one output interval (1, 2, 4, 8, 16, 32)
     double precision;       // 4 ** hypercubes  (I:1550)
+    double lt_norm2_max;    // largest |g|^2 whose Lie-Trotter exponential is the exponential to rounding (expo64.cuh)
 };
 
 // Launch arguments of the time-evolution kernels.

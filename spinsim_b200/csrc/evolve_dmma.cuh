@@ -89,15 +89,6 @@ SS_D Su2d su2d_mul(const Su2d& b, const Su2d& a) {
     return o;
 }
 
-SS_D Su2d shfl_down_su2(const Su2d& v, int delta) {
-    Su2d o;
-    o.am1.re = __shfl_down_sync(0xffffffffu, v.am1.re, delta);
-    o.am1.im = __shfl_down_sync(0xffffffffu, v.am1.im, delta);
-    o.beta.re = __shfl_down_sync(0xffffffffu, v.beta.re, delta);
-    o.beta.im = __shfl_down_sync(0xffffffffu, v.beta.im, delta);
-    return o;
-}
-
 static_assert(kDmmaTile == kScanTile, "a CTA tile is one state scan tile (its warps' row products are its partials)");
 
 // Recurrence r = ((channel * kBulkTones + tone) * kDmmaSegments + segment) * 2 + Gauss point of an
