@@ -90,6 +90,13 @@ MINB_TIGHT = (5, 6)
 DMMA_MINB = (3, 4, 5, 6)
 
 
+def user_minb(v):
+    """Resident CTAs a user-field kernel's register allocation must allow: four (128 registers; the
+    spin-one Rabi sweep's time evolution 179 -> 131 us against 208 registers and two CTAs), except for
+    the eight-generator exponential, whose 3 x 3 temporaries would spill in its inner loop."""
+    return 2 if v[3] == 2 else 4
+
+
 def gen_sources():
     os.makedirs(GEN, exist_ok=True)
     units = []  # (kind, name, source path)
@@ -112,7 +119,7 @@ def gen_sources():
         src = os.path.join(GEN, f"u_{name}.cu")
         body = ("#define SPINSIM_USER_FIELD 1\n"
                 '#include "evolve_kernel.cuh"\n'
-                f'extern "C" __global__ void __launch_bounds__(spinsim::kEvolveThreadsMax, 2) '
+                f'extern "C" __global__ void __launch_bounds__(spinsim::kEvolveThreadsMax, {user_minb(v)}) '
                 f"spinsim_evolve_user(spinsim::EvolveArgs a) {{\n"
                 f"    spinsim::evolve_body<{tmpl(v, 0)}>(a);\n}}\n")
         write_if_changed(src, body)

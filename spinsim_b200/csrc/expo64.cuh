@@ -145,9 +145,8 @@ SS_D void su2_step64(const MethodConfig& m, Su2d& p, const double* g) {
 
 // ------------------------------------------------------------------ spin one
 // matrix_exponential_lie_trotter for spin one (I:1768-1808); exp(i p) = (x + i y) / a replaces
-// p = atan2(y, x).  The exponential minus one.  Out of line: taken by the steps with a quadratic
-// shift that are too large for their number of squarings (spin_one_step64).
-inline __device__ __noinline__ Mat<3> expo_lt_one_m1(const double* g, int hypercubes, double precision) {
+// p = atan2(y, x).  The exponential minus one.
+SS_D Mat<3> expo_lt_one_m1(const double* g, int hypercubes, double precision) {
     double a = sqrt(g[0] * g[0] + g[1] * g[1]);
     c64 ep = c64{1.0, 0.0};  // exp(i p)
     if (a > 0) {
@@ -270,25 +269,34 @@ SS_D Mat<3> spin_one_exp_m1_64(double x, double y, double z, double q) {
     return e;
 }
 
+// u <- (1 + e) u, column by column in place
+SS_D void spin_one_apply64(Mat<3>& u, const Mat<3>& e) {
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        const c64 c0 = u.a[0][j], c1 = u.a[1][j], c2 = u.a[2][j];
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+            u.a[i][j] = cfma(e.a[i][2], c2, cfma(e.a[i][1], c1, cfma(e.a[i][0], c0, u.a[i][j])));
+    }
+}
+
+// A step by the reference's squarings.  Out of line, the product by value: taken only by steps that are
+// too large for their number of squarings, so its registers and stack stay out of the common loop.
+inline __device__ __noinline__ Mat<3> spin_one_squarings_step64(Mat<3> u, double x, double y, double z, double q,
+                                                               int hypercubes, double precision) {
+    const double g[4] = {x, y, z, q};
+    spin_one_apply64(u, expo_lt_one_m1(g, hypercubes, precision));
+    return u;
+}
+
 // One exponential of a spin-one step with a quadratic shift (I:1768-1808), applied to the interval's
 // product u.  As in su2_step64, the exponential itself where the Lie-Trotter product agrees with it to
 // rounding (|g|^2 <= lt_norm2_max; the reversed sign of the shift in the factor's [0][2] phase is
 // of the same order as the splitting's error, a^2 q / (6 N^2)), else the reference's squarings.
 SS_D void spin_one_step64(const MethodConfig& m, Mat<3>& u, const double* g) {
     const double r2 = fma(g[0], g[0], fma(g[1], g[1], fma(g[2], g[2], g[3] * g[3])));
-    const Mat<3> e = r2 <= m.lt_norm2_max ? spin_one_exp_m1_64(g[0], g[1], g[2], g[3])
-                                          : expo_lt_one_m1(g, m.hypercubes, m.precision);
-    Mat<3> o;
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            c64 acc = u.a[i][j];
-#pragma unroll
-            for (int k = 0; k < 3; k++) acc = cfma(e.a[i][k], u.a[k][j], acc);
-            o.a[i][j] = acc;
-        }
-    u = o;
+    if (r2 <= m.lt_norm2_max) spin_one_apply64(u, spin_one_exp_m1_64(g[0], g[1], g[2], g[3]));
+    else u = spin_one_squarings_step64(u, g[0], g[1], g[2], g[3], m.hypercubes, m.precision);
 }
 
 // matrix_exponential_lie_trotter_8 (I:1810-1925).  As in the reference, the third block
