@@ -13,9 +13,8 @@
  *      time[N] f64, time_evolution U[N][d][d] c128, state[N][d] c128, spin[N][3] f64.
  *  - `stream` is a cudaStream_t (NULL = legacy default stream).  All work is stream-ordered.  The
  *    single-instance entry points (spinsim_evaluate, spinsim_time_evolution, spinsim_state,
- *    spinsim_state_static, spinsim_piece_*) and spinsim_batch_launch only launch kernels: their
- *    descriptors travel as launch arguments and are written into the workspace on the device, so
- *    they never wait for the stream and can be captured into a CUDA graph (host arrays such as psi0
+ *    spinsim_state_static, spinsim_piece_*) and spinsim_batch_launch only launch kernels: a single
+ *    call's descriptors travel as launch arguments, so they never wait for the stream and can be captured into a CUDA graph (host arrays such as psi0
  *    are read during the call).  Host waits: spinsim_plan_create (module load; with a user field,
  *    the link), spinsim_batch_prepare (copies from pageable host memory, which wait for the stream;
  *    spinsim_batch_prepare_staged copies from the caller's page-locked staging instead), and the
@@ -176,6 +175,15 @@ int spinsim_evaluate_with_norms(const spinsim_plan* plan, const spinsim_field* f
                                 double dt_out, int64_t n_out, const double* psi0, double* time_dev, double* u_dev,
                                 double* state_dev, double* spin_dev, float* step_norms_dev, void* workspace_dev,
                                 size_t workspace_bytes, void* stream);
+
+/* spinsim_evaluate_with_norms of a user-field plan with its sweep parameters in host memory (at most
+ * SPINSIM_MAX_CALL_PARAMS of them, read during the call): they travel with the launch, so the call needs no
+ * copy and no device buffer for them. */
+#define SPINSIM_MAX_CALL_PARAMS 64
+int spinsim_evaluate_params(const spinsim_plan* plan, const double* params, int32_t n_params, double t0, double dt_int,
+                            double dt_out, int64_t n_out, const double* psi0, double* time_dev, double* u_dev,
+                            double* state_dev, double* spin_dev, float* step_norms_dev, void* workspace_dev,
+                            size_t workspace_bytes, void* stream);
 
 /* get_time_evolution alone (I:855-896): writes time_dev[N] and u_dev[N][d][d]. */
 int spinsim_time_evolution(const spinsim_plan* plan, const spinsim_field* field, double t0, double dt_int,

@@ -401,35 +401,36 @@ class Simulator:
         if psi0.size != d:
             raise ValueError(f"state_init must have {d} entries")
         dev = self._torch_device
-        sweep = torch.as_tensor(np.asarray(sweep_parameters, np.float64).reshape(-1), device=dev)
-        if sweep.numel() == 0:
-            sweep = torch.zeros(1, dtype=torch.float64, device=dev)
+        # a user field's sweep parameters travel with the launch; more than that go through device memory
+        params = np.ascontiguousarray(np.asarray(sweep_parameters, np.float64).reshape(-1))
+        if not params.size:
+            params = np.zeros(1)
+        by_value = self._builtin is None and params.size <= _lib.MAX_CALL_PARAMS
+        sweep = None if by_value or self._builtin is not None else torch.as_tensor(params, device=dev)
         time = torch.empty(n, dtype=torch.float64, device=dev)
         u = torch.empty((n, d, d), dtype=torch.complex128, device=dev)
         state = torch.empty((n, d), dtype=torch.complex128, device=dev)
         spin = torch.empty((n, 3), dtype=torch.float64, device=dev)
         ws_bytes = self._lib.spinsim_evaluate_workspace_size(self._plan, n)
         ws = torch.empty(max(ws_bytes, 256), dtype=torch.uint8, device=dev)
-        field = self._field_struct(sweep)
         stream = torch.cuda.current_stream(dev).cuda_stream
-        if self.precision == Precision.FP32_BULK:
-            norms = torch.zeros(max(n, 1), dtype=torch.float32, device=dev)
-            _lib.check(self._lib.spinsim_evaluate_with_norms(
-                self._plan, ctypes.byref(field), float(time_start), float(dt_int), float(time_step_output), n,
-                psi0.ctypes.data_as(ctypes.c_void_p), time.data_ptr(), u.data_ptr(), state.data_ptr(),
-                spin.data_ptr(), norms.data_ptr(), ws.data_ptr(), ws.numel(), stream))
+        bulk = self.precision == Precision.FP32_BULK
+        norms = torch.zeros(max(n, 1), dtype=torch.float32, device=dev) if bulk else None
+        call = (float(time_start), float(dt_int), float(time_step_output), n, psi0.ctypes.data, time.data_ptr(),
+                u.data_ptr(), state.data_ptr(), spin.data_ptr(), norms.data_ptr() if bulk else None, ws.data_ptr(),
+                ws.numel(), stream)
+        if by_value:
+            _lib.check(self._lib.spinsim_evaluate_params(self._plan, params.ctypes.data, params.size, *call))
+        else:
+            _lib.check(self._lib.spinsim_evaluate_with_norms(self._plan, ctypes.byref(self._field_struct(sweep)), *call))
+        error = 0.0
+        if bulk:
             steps = n * int(math.floor(float(time_step_output) / float(dt_int) + 0.5))
             bound = magnus_method_bound(self.get_field, dt_int, steps)
             lt = self._lie_trotter_hypercubes()
 
             def error():
                 return bulk_error_estimate(norms[:n].double().sum().item(), d, bound, steps, lt)
-        else:
-            _lib.check(self._lib.spinsim_evaluate(
-                self._plan, ctypes.byref(field), float(time_start), float(dt_int), float(time_step_output), n,
-                psi0.ctypes.data_as(ctypes.c_void_p), time.data_ptr(), u.data_ptr(), state.data_ptr(),
-                spin.data_ptr(), ws.data_ptr(), ws.numel(), stream))
-            error = 0.0
         return Results(time, u, state, self.spin_calculator, spin=spin, keep=(sweep, ws, self._builtin), error=error)
 
     def spin_calculator(self, state):

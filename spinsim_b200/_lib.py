@@ -16,6 +16,7 @@ ERR_CUDA = -2
 ERR_LINK = -3
 ERR_UNSUPPORTED = -4
 ERR_WORKSPACE = -5
+MAX_CALL_PARAMS = 64  # SPINSIM_MAX_CALL_PARAMS
 
 c_i32 = ctypes.c_int32
 c_i64 = ctypes.c_int64
@@ -83,6 +84,8 @@ _SIGNATURES = [
     ("spinsim_evaluate_with_norms", ctypes.c_int,
      [c_vp, ctypes.POINTER(Field), c_dbl, c_dbl, c_dbl, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp,
       ctypes.c_size_t, c_vp]),
+    ("spinsim_evaluate_params", ctypes.c_int,
+     [c_vp, c_vp, c_i32, c_dbl, c_dbl, c_dbl, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, ctypes.c_size_t, c_vp]),
     ("spinsim_time_evolution", ctypes.c_int,
      [c_vp, ctypes.POINTER(Field), c_dbl, c_dbl, c_dbl, c_i64, c_vp, c_vp, c_vp, ctypes.c_size_t, c_vp]),
     ("spinsim_state_workspace_size", ctypes.c_size_t, [c_i32, c_i64]),

@@ -108,7 +108,7 @@ def gen_sources():
                 src = os.path.join(GEN, f"k_{name}.cu")
                 t = tmpl(v, field, minb)
                 body = (f'#include "evolve_kernel.cuh"\n'
-                        f"namespace spinsim {{\ntemplate __global__ void evolve_kernel<{t}>(EvolveArgs);\n}}\n"
+                        f"namespace spinsim {{\ntemplate __global__ void evolve_kernel<{t}>(const __grid_constant__ EvolveArgs);\n}}\n"
                         f'extern "C" const void* spinsim_kget_{name}(void) {{\n'
                         f"    return (const void*)&spinsim::evolve_kernel<{t}>;\n}}\n")
                 write_if_changed(src, body)
@@ -120,7 +120,7 @@ def gen_sources():
         body = ("#define SPINSIM_USER_FIELD 1\n"
                 '#include "evolve_kernel.cuh"\n'
                 f'extern "C" __global__ void __launch_bounds__(spinsim::kEvolveThreadsMax, {user_minb(v)}) '
-                f"spinsim_evolve_user(spinsim::EvolveArgs a) {{\n"
+                f"spinsim_evolve_user(const __grid_constant__ spinsim::EvolveArgs a) {{\n"
                 f"    spinsim::evolve_body<{tmpl(v, 0)}>(a);\n}}\n")
         write_if_changed(src, body)
         units.append(("lto", name, src))

@@ -28,6 +28,7 @@ static_assert(sizeof(spinsim_table) == sizeof(TableChannel), "table layout");
 static_assert(sizeof(spinsim_field) == sizeof(FieldDesc), "field layout");
 static_assert(sizeof(spinsim_instance) == sizeof(Instance), "instance layout");
 static_assert(offsetof(spinsim_instance, psi0) == offsetof(Instance, psi0), "instance psi0");
+static_assert(SPINSIM_MAX_CALL_PARAMS == kSingleParams, "parameters by value");
 static_assert(offsetof(spinsim_field, bias) == offsetof(FieldDesc, bias), "field bias");
 
 // ------------------------------------------------------------------ errors
@@ -427,6 +428,7 @@ int pick_lanes(const spinsim_plan* p, int64_t intervals, int max_fine) {
 struct ScanPlan {
     int64_t n_tiles = 0;
     int64_t tiles_half = 0;  // tiles [0, tiles_half) are spin half, the rest spin one
+    int64_t max_tiles = 0;   // of the longest instance
     int32_t n_instances = 0;
 };
 
@@ -434,7 +436,11 @@ void count_scan_plan(const Instance* inst, int n_inst, ScanPlan* sp) {
     int64_t count = 0;
     for (int dim = 2; dim <= 3; dim++) {
         for (int i = 0; i < n_inst; i++)
-            if (inst[i].dim == dim) count += (inst[i].n_out + kScanTile - 1) / kScanTile;
+            if (inst[i].dim == dim) {
+                const int64_t tiles = (inst[i].n_out + kScanTile - 1) / kScanTile;
+                count += tiles;
+                sp->max_tiles = std::max(sp->max_tiles, tiles);
+            }
         count = (count + kScanTilesPerWarp - 1) / kScanTilesPerWarp * kScanTilesPerWarp;
         if (dim == 2) sp->tiles_half = count;
     }
@@ -468,6 +474,7 @@ struct ScanBuffers {
     double *tile_product, *tile_prefix;
     int64_t n_tiles;
     int64_t tiles_half;  // tiles [0, tiles_half) are spin half, the rest spin one
+    int64_t max_tiles;   // of the longest instance
     int32_t n_instances;
 };
 
@@ -476,6 +483,7 @@ struct ScanBuffers {
 void carve_scan_desc(Carver& c, const ScanPlan& sp, ScanBuffers* b) {
     b->n_tiles = sp.n_tiles;
     b->tiles_half = sp.tiles_half;
+    b->max_tiles = sp.max_tiles;
     b->n_instances = sp.n_instances;
     b->tiles = c.take<Tile>((size_t)std::max<int64_t>(1, sp.n_tiles));
     b->begin = c.take<int32_t>((size_t)std::max<int32_t>(1, sp.n_instances));
@@ -493,6 +501,7 @@ void carve_scan_single(Carver& c, int64_t n_out, int32_t dim, ScanBuffers* b) {
     b->begin = b->end = nullptr;
     b->n_tiles = scan_tiles_of(n_out);
     b->tiles_half = dim == 2 ? b->n_tiles : 0;
+    b->max_tiles = b->n_tiles;
     b->n_instances = 1;
     carve_scan_scratch(c, b->n_tiles, b);
 }
@@ -505,38 +514,32 @@ int upload(void* dst, const void* src, size_t bytes, cudaStream_t s) {
 
 enum ScanStages { SCAN_PREFIX = 1, SCAN_APPLY = 2, SCAN_ALL = 3 };
 
-// A single call's descriptors, written on the device from the launch's arguments (no host copy).
-int put_descriptors(Instance* inst_dst, const Instance& inst, FieldDesc* field_dst, const FieldDesc* field,
-                    cudaStream_t s) {
-    DescriptorArgs a;
-    memset(&a, 0, sizeof(a));
-    a.inst = inst;
-    if (field) memcpy(&a.field, field, sizeof(FieldDesc));
-    a.inst_dst = inst_dst;
-    a.field_dst = field ? field_dst : nullptr;
-    put_descriptors_kernel<<<1, 32, 0, s>>>(a);
-    CUDA_TRY(cudaGetLastError());
-    return SPINSIM_OK;
-}
-
-// The state scan's launches (scan.cuh).  b.tiles == null: one instance (inst_dev[0], n_out steps)
-// with implicit tiles.
-// A kernel launch that may start before the preceding kernel in the stream has completed
+// A kernel launch (of clusters of `cluster` CTAs) that may start before the preceding kernel in the stream has completed
 // (programmatic stream serialization): the kernel itself waits for that kernel's results
 // (grid_dependency_wait) where it first needs them.
 template <typename... K, typename... A>
-cudaError_t launch_early(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+cudaError_t launch_early_cluster(void (*kernel)(K...), unsigned cluster, dim3 grid, dim3 block, size_t smem,
+                                 cudaStream_t s, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = 1;
+    at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <typename... K, typename... A>
+cudaError_t launch_early(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    return launch_early_cluster(kernel, 1, grid, block, smem, s, args...);
 }
 
 // Multiprocessors of the current device (looked up once per device; not a stream operation).
@@ -552,11 +555,57 @@ int device_sm_count(int* out) {
     return SPINSIM_OK;
 }
 
+// Output steps of a single instance up to which the whole scan is one launch of one cluster: one step per
+// thread to 2048, up to kClusterSteps beyond.  Measured against the three launches (spin half / one): 100
+// steps 9.4 / 16.7 -> 3.1 / 5.7 us, 4001 steps 12.9 / 22.6 -> 7.0 / 10.9, 8192 steps 13 / 22 (with the
+// cluster prefix) against 10.9 / 17.6; at 16,384 steps the three launches win, 14.4 / 24.9 against 18.6 / 35.8.
+constexpr int64_t kScanShort = (int64_t)kClusterSteps * kClusterMax * kClusterThreads;
+
+int launch_scan_short(const ScanArgs& a, int32_t dim, cudaStream_t s) {
+    constexpr int64_t threads = (int64_t)kClusterMax * kClusterThreads;
+    const int32_t per = (int32_t)((a.single_n_out + threads - 1) / threads);
+    const int64_t ctas = (a.single_n_out + (int64_t)per * kClusterThreads - 1) / ((int64_t)per * kClusterThreads);
+    unsigned c = 1;
+    while (c < ctas) c *= 2;
+    auto kernel = dim == 2 ? scan_short_kernel<2> : scan_short_kernel<3>;
+    CUDA_TRY(launch_early_cluster(kernel, c, dim3(c), dim3(kClusterThreads), 0, s, a, per));
+    return SPINSIM_OK;
+}
+
+// The tile prefixes: a warp per instance, or, where some instance has many tiles, a cluster per instance
+// with about four tiles per thread of the longest (fewer CTAs where that would be many of them).  A warp
+// takes 1.1 us for each 32 tiles of the longest instance from SU(2) partials, and 1.7 or 3 us from 2 x 2 or
+// 3 x 3 products; a cluster kernel takes about 6 us and 0.5 us for each tile of its longest thread, in waves
+// of three CTAs per SM (one of 6250 tiles 165 -> 10 us).  The shorter of the two is launched.
+int launch_prefix(const ScanArgs& a, const ScanBuffers& b, const bool* has_dim, int sm, cudaStream_t s) {
+    unsigned c = 1;
+    while (c < (unsigned)kClusterMax && (int64_t)c * 4 * kClusterThreads < b.max_tiles &&
+           (int64_t)2 * c * b.n_instances <= 16 * (int64_t)sm)
+        c *= 2;
+    const double per_chunk = a.partials ? 1.1 : has_dim[1] ? 3.0 : 1.7;
+    const double by_warp = per_chunk * (double)((b.max_tiles + 31) / 32);
+    const double per_thread = (double)((b.max_tiles + c * kClusterThreads - 1) / (c * kClusterThreads));
+    const double waves = (double)(((int64_t)c * b.n_instances + 3 * sm - 1) / (3 * sm));
+    const double by_cluster = (has_dim[0] + has_dim[1]) * waves * (6.0 + 0.5 * per_thread);
+    if (by_warp <= by_cluster) {
+        const unsigned warps_per_block = kScanBlock / 32;
+        const unsigned grid = (unsigned)((b.n_instances + warps_per_block - 1) / warps_per_block);
+        CUDA_TRY(launch_early(scan_prefix_kernel, dim3(grid), dim3(kScanBlock), 0, s, a));
+        return SPINSIM_OK;
+    }
+    const dim3 grid(c * (unsigned)b.n_instances);
+    if (has_dim[0]) CUDA_TRY(launch_early_cluster(scan_prefix_cluster_kernel<2>, c, grid, dim3(kClusterThreads), 0, s, a));
+    if (has_dim[1]) CUDA_TRY(launch_early_cluster(scan_prefix_cluster_kernel<3>, c, grid, dim3(kClusterThreads), 0, s, a));
+    return SPINSIM_OK;
+}
+
+// The state scan's launches (scan.cuh).  b.tiles == null: one instance (`single`, on the host) with
+// implicit tiles.
 // partials: the tensor-path time evolution has written each tile's warp partials into b.tile_product
 // (the tile products kernels are then not launched).
 // rows (partials mode, may be null): each output step's operator as its SU(2) pair, which the apply
 // reads in place of u.
-int launch_scan(const Instance* inst_dev, int64_t single_n_out, const ScanBuffers& b, const double* u, double* state,
+int launch_scan(const Instance* inst_dev, const Instance* single, const ScanBuffers& b, const double* u, double* state,
                 double* spin, cudaStream_t s, int stages = SCAN_ALL, double* total = nullptr, bool partials = false,
                 const double* rows = nullptr) {
     if (b.n_tiles == 0) return SPINSIM_OK;
@@ -574,11 +623,13 @@ int launch_scan(const Instance* inst_dev, int64_t single_n_out, const ScanBuffer
     a.state = state;
     a.spin = spin;
     a.total = total;
-    a.single_n_out = single_n_out;
+    if (single) {
+        a.single = *single;
+        a.single_n_out = single->n_out;
+        if (stages == SCAN_ALL && !total && single->n_out <= kScanShort) return launch_scan_short(a, single->dim, s);
+    }
     a.partials = partials ? 1 : 0;
     a.rows = partials ? rows : nullptr;
-    const unsigned warps_per_block = kScanBlock / 32;
-    const unsigned grid_inst = (unsigned)((b.n_instances + warps_per_block - 1) / warps_per_block);
     // tile kernels: one launch per spin dimension over its run of tiles
     const int64_t lo[2] = {0, b.tiles_half}, hi[2] = {b.tiles_half, b.n_tiles};
     const int warps[2] = {ScanShared<2>::kWarps, ScanShared<3>::kWarps};
@@ -590,14 +641,18 @@ int launch_scan(const Instance* inst_dev, int64_t single_n_out, const ScanBuffer
     constexpr int t2 = ScanShared<2>::kThreads, t3 = ScanShared<3>::kThreads;
     constexpr size_t m2 = ScanShared<2>::kBytes, m3 = ScanShared<3>::kBytes;
     int sm = 0;
+    int rc = device_sm_count(&sm);
+    if (rc) return rc;
     if (stages & SCAN_PREFIX) {
-        if (grid[0] && !partials) scan_products_kernel<2><<<grid[0], t2, m2, s>>>(a, lo[0], hi[0]);
-        if (grid[1] && !partials) scan_products_kernel<3><<<grid[1], t3, m3, s>>>(a, lo[1], hi[1]);
-        CUDA_TRY(launch_early(scan_prefix_kernel, dim3(grid_inst), dim3(kScanBlock), 0, s, a));
+        if (grid[0] && !partials)
+            CUDA_TRY(launch_early(scan_products_kernel<2>, dim3(grid[0]), dim3(t2), m2, s, a, lo[0], hi[0]));
+        if (grid[1] && !partials)
+            CUDA_TRY(launch_early(scan_products_kernel<3>, dim3(grid[1]), dim3(t3), m3, s, a, lo[1], hi[1]));
+        const bool has_dim[2] = {grid[0] != 0, grid[1] != 0};
+        rc = launch_prefix(a, b, has_dim, sm, s);
+        if (rc) return rc;
     }
     if (stages & SCAN_APPLY) {  // persistent: at most the CTAs the device holds at once
-        int rc = device_sm_count(&sm);
-        if (rc) return rc;
         const int apply_warps[2] = {ApplyShared<2>::kWarps, ApplyShared<3>::kWarps};  // the same in both modes
         static_assert(ApplyShared<2, true>::kWarps == ApplyShared<2>::kWarps &&
                           ApplyShared<3, true>::kWarps == ApplyShared<3>::kWarps, "apply CTA sizes");
@@ -667,6 +722,16 @@ int launch_evolve(const spinsim_plan* p, EvolveArgs a, int64_t tiles, cudaStream
     return SPINSIM_OK;
 }
 
+// The tensor path's per-instance constants (evolve_dmma.cuh), which the time evolution then reads; for a
+// single call also its descriptors (inst_out, field_out), from the arguments.
+int launch_dmma_consts(EvolveArgs* a, DmmaConsts* out, int32_t n, Instance* inst_out, FieldDesc* field_out,
+                       cudaStream_t s) {
+    void* args[] = {a, &out, &n, &inst_out, &field_out};
+    CUDA_TRY(cudaLaunchKernel(spinsim_kget_dmma_consts(), dim3((unsigned)n), dim3(kDmmaRecurrences), args, 0, s));
+    a->dmma_consts = out;
+    return SPINSIM_OK;
+}
+
 int check_field(const spinsim_plan* p, const spinsim_field* f) {
     if (!f) return fail(SPINSIM_ERR_INVALID, "field is null");
     if (p->desc.field_kind == SPINSIM_FIELD_TABLE && !f->tables)
@@ -701,30 +766,34 @@ static int make_instance(const spinsim_plan* p, double t0, double dt_int, double
     return SPINSIM_OK;
 }
 
-// Workspace of a single-instance call: its instance and field descriptors (written on the device by
-// put_descriptors) and the state scan's scratch (its tiles are implicit).
-static size_t single_workspace(int64_t n_out, bool with_scan, bool with_rows = false) {
+// Workspace of a single-instance call: the state scan's scratch (its descriptors are launch arguments, its
+// tiles implicit) and, on the tensor path, its descriptors, constants and SU(2) rows.
+static size_t single_workspace(int64_t n_out, bool with_scan, bool with_rows = false, bool tensor = false) {
     Carver c(nullptr);
-    c.take<Instance>(1);
-    c.take<FieldDesc>(1);
     if (with_scan) {
         ScanBuffers b;
         carve_scan_single(c, n_out, 2, &b);
     }
     if (with_rows) c.take<double>(4 * (size_t)std::max<int64_t>(1, n_out));
+    if (tensor) {
+        c.take<Instance>(1);
+        c.take<FieldDesc>(1);
+        c.take<DmmaConsts>(1);
+    }
     return c.used + 256;
 }
 
 extern "C" size_t spinsim_evaluate_workspace_size(const spinsim_plan* plan, int64_t n_out) {
     if (!plan || n_out < 0 || plan->desc.spin_dim == 0) return 0;
-    return single_workspace(n_out, true, plan->cta_tiles);  // the tensor path's SU(2) rows for the scan
+    return single_workspace(n_out, true, plan->cta_tiles, plan->cta_tiles);  // the tensor path's SU(2) rows for the scan
 }
 
 static int evaluate_impl(const spinsim_plan* p, const spinsim_field* field, double t0, double dt_int, double dt_out,
                          int64_t n_out, const double* psi0, double* time, double* u, double* state, double* spin,
-                         float* norms, void* ws, size_t ws_bytes, cudaStream_t s, bool with_scan) {
+                         float* norms, void* ws, size_t ws_bytes, cudaStream_t s, bool with_scan,
+                         const double* params = nullptr, int32_t n_params = 0) {
     if (!p) return fail(SPINSIM_ERR_INVALID, "plan is null");
-    int rc = check_field(p, field);
+    int rc = params ? (field ? SPINSIM_OK : fail(SPINSIM_ERR_INVALID, "field is null")) : check_field(p, field);
     if (rc) return rc;
     Instance inst;
     rc = make_instance(p, t0, dt_int, dt_out, n_out, psi0, &inst);
@@ -734,24 +803,24 @@ static int evaluate_impl(const spinsim_plan* p, const spinsim_field* field, doub
     if (with_scan && !psi0) return fail(SPINSIM_ERR_INVALID, "psi0 is null");
     if (!ws || ((uintptr_t)ws & 255)) return fail(SPINSIM_ERR_WORKSPACE, "workspace must be non-null and 256-byte aligned");
     const bool with_rows = with_scan && p->cta_tiles;
-    const size_t need = single_workspace(n_out, with_scan, with_rows);
+    const size_t need = single_workspace(n_out, with_scan, with_rows, p->cta_tiles);
     if (ws_bytes < need) return fail(SPINSIM_ERR_WORKSPACE, "workspace of %zu bytes is below the %zu needed", ws_bytes, need);
 
     Carver c(ws);
-    Instance* inst_dev = c.take<Instance>(1);
-    FieldDesc* field_dev = c.take<FieldDesc>(1);
     ScanBuffers b;
     if (with_scan) carve_scan_single(c, n_out, inst.dim, &b);
     double* rows = with_rows ? c.take<double>(4 * (size_t)std::max<int64_t>(1, n_out)) : nullptr;
-    rc = put_descriptors(inst_dev, inst, field_dev, reinterpret_cast<const FieldDesc*>(field), s);
-    if (rc) return rc;
 
     EvolveArgs a;
     memset(&a, 0, sizeof(a));
     a.m = p->m;
     a.m.lanes = pick_lanes(p, n_out, inst.n_fine);
-    a.instances = inst_dev;
-    a.fields = field_dev;
+    a.single = inst;
+    memcpy(&a.single_field, field, sizeof(FieldDesc));
+    if (params) {
+        a.n_single_params = n_params;
+        memcpy(a.single_params, params, sizeof(double) * (size_t)n_params);
+    }
     a.tiles = nullptr;
     const int per_tile = tile_intervals(p, a.m.lanes);
     a.n_tiles = (n_out + per_tile - 1) / per_tile;
@@ -760,14 +829,22 @@ static int evaluate_impl(const spinsim_plan* p, const spinsim_field* field, doub
     a.u = u;
     a.step_norms = p->desc.precision == SPINSIM_PRECISION_FP32_BULK ? norms : nullptr;
     // the tensor path writes the scan's tile partials as it goes (its CTA tiles are the scan tiles)
-    const bool partials = with_scan && p->cta_tiles &&
+    const bool partials = with_scan && p->cta_tiles && n_out > kScanShort &&
                           tones_on_tensor_path(*reinterpret_cast<const FieldDesc*>(field), inst.dim);
     a.tile_partials = partials ? b.tile_product : nullptr;
     a.scan_begin = nullptr;
     a.rows = partials ? rows : nullptr;
-    rc = launch_evolve(p, a, a.n_tiles, s);
+    if (p->cta_tiles) {
+        Instance* inst_dev = c.take<Instance>(1);
+        FieldDesc* field_dev = c.take<FieldDesc>(1);
+        rc = launch_dmma_consts(&a, c.take<DmmaConsts>(1), 1, inst_dev, field_dev, s);
+        if (rc) return rc;
+        a.instances = inst_dev;
+        a.fields = field_dev;
+    }
+    rc = launch_evolve(p, a, a.n_tiles, s, p->cta_tiles);
     if (rc || !with_scan) return rc;
-    return launch_scan(inst_dev, n_out, b, u, state, spin, s, SCAN_ALL, nullptr, partials, a.rows);
+    return launch_scan(nullptr, &inst, b, u, state, spin, s, SCAN_ALL, nullptr, partials, a.rows);
 }
 
 extern "C" int spinsim_evaluate(const spinsim_plan* plan, const spinsim_field* field, double t0, double dt_int,
@@ -785,6 +862,21 @@ extern "C" int spinsim_evaluate_with_norms(const spinsim_plan* plan, const spins
                                            void* stream) {
     return evaluate_impl(plan, field, t0, dt_int, dt_out, n_out, psi0, time_dev, u_dev, state_dev, spin_dev,
                          step_norms_dev, workspace_dev, workspace_bytes, (cudaStream_t)stream, true);
+}
+
+extern "C" int spinsim_evaluate_params(const spinsim_plan* plan, const double* params, int32_t n_params, double t0,
+                                       double dt_int, double dt_out, int64_t n_out, const double* psi0,
+                                       double* time_dev, double* u_dev, double* state_dev, double* spin_dev,
+                                       float* step_norms_dev, void* workspace_dev, size_t workspace_bytes,
+                                       void* stream) {
+    if (!plan) return fail(SPINSIM_ERR_INVALID, "plan is null");
+    if (plan->desc.field_kind != SPINSIM_FIELD_USER) return fail(SPINSIM_ERR_INVALID, "the plan has no user field");
+    if (!params || n_params < 1 || n_params > kSingleParams)
+        return fail(SPINSIM_ERR_INVALID, "between 1 and %d sweep parameters travel with the call", kSingleParams);
+    spinsim_field field;
+    memset(&field, 0, sizeof(field));
+    return evaluate_impl(plan, &field, t0, dt_int, dt_out, n_out, psi0, time_dev, u_dev, state_dev, spin_dev,
+                         step_norms_dev, workspace_dev, workspace_bytes, (cudaStream_t)stream, true, params, n_params);
 }
 
 extern "C" int spinsim_time_evolution(const spinsim_plan* plan, const spinsim_field* field, double t0, double dt_int,
@@ -807,13 +899,9 @@ static int state_scan(int32_t dim, const double* u_dev, int64_t n_out, const dou
     if (psi0)
         for (int i = 0; i < 2 * dim; i++) inst.psi0[i] = psi0[i];
     Carver c(workspace);
-    Instance* inst_dev = c.take<Instance>(1);
-    c.take<FieldDesc>(1);
     ScanBuffers b;
     carve_scan_single(c, n_out, dim, &b);
-    int rc = put_descriptors(inst_dev, inst, nullptr, nullptr, s);
-    if (rc) return rc;
-    return launch_scan(inst_dev, n_out, b, u_dev, state_dev, spin_dev, s, stages, total_dev);
+    return launch_scan(nullptr, &inst, b, u_dev, state_dev, spin_dev, s, stages, total_dev);
 }
 
 extern "C" size_t spinsim_state_workspace_size(int32_t dim, int64_t n_out) {
@@ -1268,15 +1356,12 @@ extern "C" int spinsim_batch_launch(const spinsim_batch* b, double* time_dev, do
     a.rows = b->partials ? b->rows : nullptr;
     a.scan_begin = b->scan.begin;
     if (b->consts != nullptr && b->scan.n_instances > 0) {  // the tensor path's per-instance constants first
-        DmmaConsts* out = b->consts;
-        int32_t n = b->scan.n_instances;
-        void* cargs[] = {&a, &out, &n};
-        CUDA_TRY(cudaLaunchKernel(spinsim_kget_dmma_consts(), dim3((unsigned)n), dim3(kDmmaRecurrences), cargs, 0, s));
-        a.dmma_consts = b->consts;
+        int rc = launch_dmma_consts(&a, b->consts, b->scan.n_instances, nullptr, nullptr, s);
+        if (rc) return rc;
     }
     int rc = launch_evolve(p, a, b->n_tiles, s, a.dmma_consts != nullptr);
     if (rc || !state_dev) return rc;
-    rc = launch_scan(b->inst_dev, 0, b->scan, u_dev, state_dev, spin_dev, s, SCAN_ALL, nullptr, b->partials, a.rows);
+    rc = launch_scan(b->inst_dev, nullptr, b->scan, u_dev, state_dev, spin_dev, s, SCAN_ALL, nullptr, b->partials, a.rows);
     return rc;
 }
 

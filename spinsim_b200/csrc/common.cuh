@@ -91,10 +91,13 @@ struct MethodConfig {
     double lt_norm2_max;    // largest |g|^2 whose Lie-Trotter exponential is the exponential to rounding (expo64.cuh)
 };
 
+// Sweep parameters of a single call that travel as launch arguments (more go through device memory).
+constexpr int kSingleParams = 64;
+
 // Launch arguments of the time-evolution kernels.
 struct EvolveArgs {
     MethodConfig m;
-    const Instance* instances;
+    const Instance* instances;  // null: one instance, described by the arguments themselves (single, ...)
     const FieldDesc* fields;
     const Tile* tiles;       // null: single instance, implicit tiles of 32 / lanes intervals (a CTA's 32 on the tensor path)
     int64_t n_tiles;
@@ -111,6 +114,10 @@ struct EvolveArgs {
                                            // earlier in the launch (null: each tile computes them)
     double* rows;  // tensor path: per output step (indexed like time), the interval's lab-frame operator
                    // as its SU(2) pair (a, b), 4 doubles, for the state scan (null: not written)
+    Instance single;         // instances == null: the instance,
+    FieldDesc single_field;  // its field,
+    int32_t n_single_params; // and, when not 0, its sweep parameters (in place of single_field.params)
+    double single_params[kSingleParams];
 };
 
 // State scan tiles (scan.cuh): consecutive output steps of one instance per tile, and the doubles

@@ -139,13 +139,20 @@ SS_D int32_t dmma_magnus(const FieldDesc& f, double dt) {
 #ifdef SPINSIM_DMMA_CONSTS_KERNEL
 // The per-instance constants of the tensor path (DmmaConsts), one CTA of kDmmaRecurrences threads
 // per instance, launched before the time evolution so its tiles load them instead of recomputing
-// them (384 FP64 sincos and the step test per tile).
-__global__ void __launch_bounds__(kDmmaRecurrences) dmma_consts_kernel(EvolveArgs a, DmmaConsts* out, int32_t n) {
+// them (384 FP64 sincos and the step test per tile).  A single call (inst_out not null): the instance and
+// field come with the arguments and are also written to device memory for the time evolution.
+__global__ void __launch_bounds__(kDmmaRecurrences) dmma_consts_kernel(const __grid_constant__ EvolveArgs a,
+                                                                       DmmaConsts* out, int32_t n, Instance* inst_out,
+                                                                       FieldDesc* field_out) {
     grid_dependency_release();  // the time evolution may start its tiles' set-up meanwhile
     const int32_t i = blockIdx.x;
     if (i >= n) return;
-    const Instance& inst = a.instances[i];
-    const FieldDesc& f = a.fields[inst.field];
+    const Instance& inst = inst_out != nullptr ? a.single : a.instances[i];
+    const FieldDesc& f = inst_out != nullptr ? a.single_field : a.fields[inst.field];
+    if (inst_out != nullptr && threadIdx.x == 0) {
+        *inst_out = a.single;
+        *field_out = a.single_field;
+    }
     if (!tones_on_tensor_path(f, inst.dim)) return;
     DmmaConsts& c = out[i];
     const int r = threadIdx.x;
@@ -449,6 +456,7 @@ __device__ __noinline__ void dmma_tile_fallback(const MethodConfig& m, const Ins
 template <int DIMS>
 SS_D void evolve_dmma_body(const EvolveArgs& a, DmmaShared& sh) {
     int64_t tile_id = blockIdx.x;
+    if (a.tiles == nullptr) grid_dependency_wait();  // a single call: its descriptors come from dmma_consts_kernel
     int32_t reserved = -1;  // thread 0: the next tile, taken from the queue while this one runs
     for (;;) {
         if (a.tile_counter != nullptr) {

@@ -3,7 +3,8 @@
 // persistent) launch.
 //
 // A warp takes one Tile (up to 32 / lanes consecutive output intervals of one instance).  Without a
-// tile list the launch covers a single instance with one tile per warp.  With a tile list and a
+// tile list the launch covers a single instance, whose descriptors are launch arguments, with one tile
+// per warp.  With a tile list and a
 // counter, warps pull tiles from a global atomic queue until it is empty; tiles are ordered
 // longest-first on the host, so instances of very different durations share one launch without a
 // long tail.  No warp ever waits for another warp.
@@ -24,6 +25,21 @@ SS_D void evolve_body(const EvolveArgs& a) {
     const int group = lane / lanes;
     const int lane_in_group = lane - group * lanes;
     const int per_warp = (SYNTH ? 32 * kSynthIntervals : 32) / lanes;
+    const FieldDesc* one_field = &a.single_field;
+    if constexpr (FIELD == FIELD_USER) {
+        // A single call's sweep parameters: a copy in shared memory, which the user's field may index freely.
+        __shared__ FieldDesc shared_field;
+        __shared__ double shared_params[kSingleParams];
+        if (a.instances == nullptr) {
+            for (int i = threadIdx.x; i < a.n_single_params; i += blockDim.x) shared_params[i] = a.single_params[i];
+            if (threadIdx.x == 0) {
+                shared_field.params = a.n_single_params ? shared_params : a.single_field.params;
+                shared_field.n_params = a.n_single_params ? a.n_single_params : a.single_field.n_params;
+            }
+            __syncthreads();
+            one_field = &shared_field;
+        }
+    }
     const int64_t warp_global = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int64_t tile_id = warp_global;
     for (;;) {
@@ -37,14 +53,14 @@ SS_D void evolve_body(const EvolveArgs& a) {
         if (a.tiles != nullptr) {
             tile = a.tiles[tile_id];
         } else {
-            const int64_t n = a.instances[0].n_out;
+            const int64_t n = a.single.n_out;
             const int64_t first = tile_id * per_warp;
             tile.instance = 0;
             tile.first = first;
             tile.count = (int)((n - first) < per_warp ? (n - first) : per_warp);
         }
-        const Instance& inst = a.instances[tile.instance];
-        const FieldDesc& f = a.fields[inst.field];
+        const Instance& inst = a.instances != nullptr ? a.instances[tile.instance] : a.single;
+        const FieldDesc& f = a.instances != nullptr ? a.fields[inst.field] : *one_field;
         double* time_out = a.time + inst.out_offset;
         double* u_out = a.u + inst.u_offset;
         float* norms_out = a.step_norms != nullptr ? a.step_norms + inst.out_offset : nullptr;
@@ -85,7 +101,7 @@ SS_D void evolve_body(const EvolveArgs& a) {
 // MINB = minimum resident CTAs per SM that the register allocation must allow (128-thread CTAs):
 // 2 leaves the full register file to one thread (255), 3 caps at 168, 4 at 128 registers.
 template <int DIMS, int INTEG, int EXPO_H, int EXPO_O, int FIELD, int PREC, int MINB>
-__global__ void __launch_bounds__(kEvolveThreadsMax, MINB) evolve_kernel(EvolveArgs a) {
+__global__ void __launch_bounds__(kEvolveThreadsMax, MINB) evolve_kernel(const __grid_constant__ EvolveArgs a) {
     evolve_body<DIMS, INTEG, EXPO_H, EXPO_O, FIELD, PREC>(a);
 }
 

@@ -14,11 +14,13 @@
 //      SU(2) pairs instead, and A is not launched; B then scans SU(2) pairs (partials mode).
 //   B  scan_prefix_kernel: a warp per instance scans the instance's tile products 32 at a time and
 //      stores every tile's exclusive prefix (and, when asked, the instance's whole product).
+//      Instances of many tiles: scan_prefix_cluster_kernel, a cluster of CTAs per instance.
 //   C  scan_apply_kernel: each group scans its lanes' products (lane j: U[4j+3] ... U[0] of the
 //      tile), applies the exclusive part times the tile's prefix to psi0 and steps through its
 //      four output steps writing state and spin (get_spin, I:899-959), fused.
 // The tile list holds the spin-half tiles, then the spin-one tiles, each run padded to whole warps
-// (count 0); the tile kernels are launched once per spin dimension over its run of tiles.
+// (count 0); the tile kernels are launched once per spin dimension over its run of tiles.  A single
+// short instance takes one launch for all of it (scan_short_kernel).
 #pragma once
 #include "common.cuh"
 
@@ -103,9 +105,10 @@ struct ScanArgs {
                                 // the tensor-path time evolution, in place of the tile products
     const double* rows;         // partials mode: each output step's operator as its SU(2) pair (4 doubles,
                                 // indexed like time), which the apply reads in place of u; may be null
+    Instance single;            // instances == null: the one instance
 };
 
-SS_D const Instance& scan_instance(const ScanArgs& a, int32_t i) { return a.instances[i]; }
+SS_D const Instance& scan_instance(const ScanArgs& a, int32_t i) { return a.instances != nullptr ? a.instances[i] : a.single; }
 
 // Tile k, or an empty tile (count 0) past the end of the list.
 SS_D Tile scan_tile(const ScanArgs& a, int64_t k) {
@@ -120,15 +123,6 @@ SS_D Tile scan_tile(const ScanArgs& a, int64_t k) {
     t.count = (int32_t)(rest < kScanTile ? rest : kScanTile);
     return t;
 }
-
-// Writes a single call's instance (and field) descriptors into its workspace from the launch's own
-// arguments: no host-to-device copy, so the call stays stream-ordered and capturable.
-struct DescriptorArgs {
-    Instance inst;
-    FieldDesc field;
-    Instance* inst_dst;
-    FieldDesc* field_dst;  // may be null
-};
 
 #ifdef __CUDACC__
 // Shared memory of a scan CTA for spin dimension D: per warp, its four tiles' operators; the apply
@@ -219,19 +213,13 @@ SS_D void products_group(const ScanArgs& a, const Tile& tile, int64_t k, int j, 
 }
 
 #ifdef SPINSIM_SCAN_KERNELS  // the launches themselves are defined once, in the C ABI's unit
-__global__ void put_descriptors_kernel(DescriptorArgs a) {
-    if (threadIdx.x == 0) {
-        *a.inst_dst = a.inst;
-        if (a.field_dst != nullptr) *a.field_dst = a.field;
-    }
-}
-
 extern __shared__ __align__(16) double scan_smem[];
 
 // Tiles [tile_lo, tile_hi) of spin dimension D (the tile list keeps each dimension's tiles together).
 template <int D>
-__global__ void __launch_bounds__(ScanShared<D>::kThreads) scan_products_kernel(ScanArgs a, int64_t tile_lo,
-                                                                               int64_t tile_hi) {
+__global__ void __launch_bounds__(ScanShared<D>::kThreads) scan_products_kernel(const __grid_constant__ ScanArgs a,
+                                                                               int64_t tile_lo, int64_t tile_hi) {
+    grid_dependency_wait();  // the operators of the preceding kernel
     const int64_t w0 =
         tile_lo + (((int64_t)blockIdx.x * ScanShared<D>::kThreads + threadIdx.x) >> 5) * kScanTilesPerWarp;
     const int lane = threadIdx.x & 31;
@@ -318,7 +306,7 @@ SS_D void prefix_warp_su2(const ScanArgs& a, int32_t i, int lane) {
 }
 
 #ifdef SPINSIM_SCAN_KERNELS
-__global__ void __launch_bounds__(kScanBlock) scan_prefix_kernel(ScanArgs a) {
+__global__ void __launch_bounds__(kScanBlock) scan_prefix_kernel(const __grid_constant__ ScanArgs a) {
     grid_dependency_wait();  // the tile products (or partials) of the preceding kernel
     const int32_t i = (int32_t)(((int64_t)blockIdx.x * kScanBlock + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
@@ -333,6 +321,183 @@ __global__ void __launch_bounds__(kScanBlock) scan_prefix_kernel(ScanArgs a) {
     }
 }
 
+#endif
+
+// ---------------------------------------------------------------------------------- long prefixes, short instances
+// Both kernels below scan one instance with a cluster of CTAs of kClusterThreads threads: thread by
+// thread, then by warp, then over the CTAs' totals in distributed shared memory.
+
+constexpr int kClusterThreads = 256;
+constexpr int kClusterWarps = kClusterThreads / 32;
+constexpr int kClusterMax = 8;            // CTAs per cluster (the portable limit)
+constexpr int kClusterSteps = 4;          // scan_short_kernel: at most this many output steps per thread
+
+template <int D>
+struct ClusterShared {
+    Mat<D> warp_total[kClusterWarps];
+    Mat<D> warp_enter[kClusterWarps];
+    Mat<D> cta_total;
+};
+
+SS_D unsigned cluster_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+    return r;
+}
+SS_D unsigned cluster_size() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(r));
+    return r;
+}
+SS_D void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
+SS_D void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
+
+// A matrix in the shared memory of CTA `rank` of the cluster, at the address of the caller's own copy.
+template <int D>
+SS_D Mat<D> remote_mat(const Mat<D>* own, unsigned rank) {
+    unsigned addr = (unsigned)__cvta_generic_to_shared(own), there;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(there) : "r"(addr), "r"(rank));
+    Mat<D> m;
+#pragma unroll
+    for (int i = 0; i < D; i++)
+#pragma unroll
+        for (int j = 0; j < D; j++)
+            asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];\n"
+                         : "=d"(m.a[i][j].re), "=d"(m.a[i][j].im)
+                         : "r"(there + 16u * (unsigned)(i * D + j)));
+    return m;
+}
+
+template <int D>
+SS_D void mat_vec(const Mat<D>& m, c64 (&v)[D]) {
+    c64 o[D];
+#pragma unroll
+    for (int r = 0; r < D; r++) {
+        c64 acc = m.a[r][0] * v[0];
+#pragma unroll
+        for (int c = 1; c < D; c++) acc = cfma(m.a[r][c], v[c], acc);
+        o[r] = acc;
+    }
+#pragma unroll
+    for (int r = 0; r < D; r++) v[r] = o[r];
+}
+
+// The warps' totals are in sh.warp_total: the CTA's total for the other CTAs (warp 0: a tree, later
+// warps from the left).  Every thread of the CTA calls this; on return the cluster's totals are visible.
+template <int D>
+SS_D void cluster_exchange(ClusterShared<D>& sh) {
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        Mat<D> m;
+        if (threadIdx.x < kClusterWarps) m = sh.warp_total[threadIdx.x];
+        else set_identity(m);
+#pragma unroll
+        for (int s = 1; s < kClusterWarps; s <<= 1) {
+            const Mat<D> later = shfl_down_mat(m, s);
+            if ((threadIdx.x & (2 * s - 1)) == 0) m = matmul(later, m);
+        }
+        if (threadIdx.x == 0) sh.cta_total = m;
+    }
+    __syncthreads();
+    cluster_arrive();
+    cluster_wait();
+}
+
+#ifdef SPINSIM_SCAN_KERNELS
+// Long instances' tile prefixes: cluster i / C scans instance i's tile products (see prefix_warp, which
+// takes a chunk of 32 tiles at a time in one warp and is as long as the instance).  Thread t of the
+// cluster multiplies `per` consecutive tiles, the products are scanned, and the thread steps through its
+// tiles again writing their exclusive prefixes.  Latency-bound; one instance of 200,000 output steps
+// (6250 tiles) took one warp 165 us.
+template <int D>
+__global__ void __launch_bounds__(kClusterThreads) scan_prefix_cluster_kernel(const __grid_constant__ ScanArgs a) {
+    __shared__ ClusterShared<D> sh;
+    grid_dependency_wait();
+    const unsigned ctas = cluster_size(), rank = cluster_rank();
+    const int32_t i = (int32_t)(blockIdx.x / ctas);
+    if (scan_instance(a, i).dim != D) return;  // the whole cluster
+    const int32_t b = a.tile_begin != nullptr ? a.tile_begin[i] : 0;
+    const int32_t e = a.tile_end != nullptr ? a.tile_end[i] : (int32_t)a.n_tiles;
+    const int32_t per = (e - b + (int32_t)ctas * kClusterThreads - 1) / ((int32_t)ctas * kClusterThreads);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t k0 = min((int64_t)e, b + ((int64_t)rank * kClusterThreads + threadIdx.x) * per);
+    const int64_t k1 = min((int64_t)e, k0 + per);
+    auto tile_of = [&](int64_t k) {
+        if (a.partials) return su2p_to_mat<D>(tile_product_of(load_partials(a, k, true)));
+        return load_mat<D>(a.tile_product + k * kScanMat);
+    };
+    Mat<D> m;
+    set_identity(m);
+    for (int64_t k = k0; k < k1; k++) m = matmul(tile_of(k), m);
+    m = warp_scan<D>(m, lane);
+    if (lane == 31) sh.warp_total[w] = m;
+    m = shfl_up_mat(m, 1);
+    if (lane == 0) set_identity(m);
+    cluster_exchange(sh);
+    if (threadIdx.x < kClusterWarps) {  // what enters warp w: the earlier warps' and CTAs' totals
+        Mat<D> enter;
+        set_identity(enter);
+        for (unsigned r = 0; r < rank; r++) enter = matmul(remote_mat(&sh.cta_total, r), enter);
+        for (int v = 0; v < (int)threadIdx.x; v++) enter = matmul(sh.warp_total[v], enter);
+        sh.warp_enter[threadIdx.x] = enter;
+    }
+    __syncthreads();
+    cluster_arrive();  // the other CTAs' totals have been read
+    m = matmul(m, sh.warp_enter[w]);
+    for (int64_t k = k0; k < k1; k++) {
+        store_mat<D>(a.tile_prefix + k * kScanMat, m);
+        m = matmul(tile_of(k), m);
+    }
+    if (a.total != nullptr && k0 < k1 && k1 == e) store_mat<D>(a.total + (int64_t)i * 2 * D * D, m);
+    cluster_wait();
+}
+
+// The whole state scan of one short instance (8192 output steps at most) in one launch of one
+// cluster: thread t holds `per` consecutive output steps, reads their operators, takes part in the scan of
+// the threads' products and steps through its states, writing state and spin (get_state, get_spin).  At
+// these sizes the scan is the latency of its launches: products, prefix and apply, 20 to 25 us one after
+// another for 5000 output steps.
+template <int D>
+__global__ void __launch_bounds__(kClusterThreads) scan_short_kernel(const __grid_constant__ ScanArgs a, int32_t per) {
+    constexpr int MD = 2 * D * D;
+    __shared__ ClusterShared<D> sh;
+    grid_dependency_wait();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned rank = cluster_rank();
+    const int64_t first = ((int64_t)rank * kClusterThreads + threadIdx.x) * per;
+    const int count = (int)max((int64_t)0, min((int64_t)per, a.single_n_out - first));
+    const double* u = a.u + first * MD;
+    Mat<D> m;
+    set_identity(m);
+    for (int i = 0; i < count; i++) m = i == 0 ? load_mat<D>(u) : matmul(load_mat<D>(u + i * MD), m);
+    m = warp_scan<D>(m, lane);
+    if (lane == 31) sh.warp_total[w] = m;
+    m = shfl_up_mat(m, 1);
+    if (lane == 0) set_identity(m);
+    cluster_exchange(sh);
+    c64 psi[D];
+#pragma unroll
+    for (int r = 0; r < D; r++) psi[r] = c64{a.single.psi0[2 * r], a.single.psi0[2 * r + 1]};
+    for (unsigned r = 0; r < rank; r++) mat_vec(remote_mat(&sh.cta_total, r), psi);
+    cluster_arrive();  // the other CTAs' totals have been read
+    for (int v = 0; v < w; v++) mat_vec(sh.warp_total[v], psi);
+    mat_vec(m, psi);
+    for (int i = 0; i < count; i++) {
+        double2* st = reinterpret_cast<double2*>(a.state) + (first + i) * D;
+#pragma unroll
+        for (int r = 0; r < D; r++) st[r] = make_double2(psi[r].re, psi[r].im);
+        if (a.spin != nullptr) {
+            double s3[3];
+            spin_of<D>(psi, s3);
+            double* sp = a.spin + (first + i) * 3;
+            sp[0] = s3[0];
+            sp[1] = s3[1];
+            sp[2] = s3[2];
+        }
+        if (i + 1 < count) mat_vec(load_mat<D>(u + i * MD), psi);
+    }
+    cluster_wait();
+}
 #endif
 
 // The group's tile: lane j computes the states of output steps 4j .. 4j + 3 into hist (n of them),
@@ -578,7 +743,7 @@ SS_D void apply_tiles(const ScanArgs& a, int64_t w0, int64_t tile_hi, int lane, 
 // this one waits for before it starts; otherwise it follows the other spin's apply kernel, which has
 // already waited for them, so it starts at once and waits for that kernel only before it completes.
 template <int D, bool ROWS>
-__global__ void __launch_bounds__(ApplyShared<D, ROWS>::kThreads) scan_apply_kernel(ScanArgs a, int64_t tile_lo,
+__global__ void __launch_bounds__(ApplyShared<D, ROWS>::kThreads) scan_apply_kernel(const __grid_constant__ ScanArgs a, int64_t tile_lo,
                                                                                    int64_t tile_hi, int32_t after_prefix) {
     using S = ApplyShared<D, ROWS>;
     if (after_prefix) grid_dependency_wait();
