@@ -25,7 +25,7 @@ import numpy as np
 _lock = threading.Lock()
 DEFAULT_CANDIDATES = [
     {"lanes": lanes, "threads_per_block": tpb, "max_registers": regs}
-    for regs in (0, 168, 128) for lanes in (1, 2) for tpb in (64, 128)
+    for regs in (255, 168, 128) for lanes in (1, 2) for tpb in (64, 128)
 ]
 # FP32-bulk tone fields: tensor-path kernel at 80 and 96 (6 and 5 CTAs per SM), 128 and 168 registers; the warp
 # synthesis at 168 and 128 registers with 64- or 128-thread CTAs.

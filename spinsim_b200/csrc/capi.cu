@@ -182,6 +182,12 @@ static int tile_intervals(const spinsim_plan* p, int lanes) {
     return p->cta_tiles ? kDmmaTile : 32 * p->intervals_per_lane / lanes;
 }
 
+// The plan's warps take 32 consecutive output intervals, one per lane: a tile of the state scan, whose product
+// they write.
+static bool warps_write_products(const spinsim_plan* p, int lanes) {
+    return !p->cta_tiles && !p->lockstep && lanes == 1;
+}
+
 extern "C" const char* spinsim_version(void) { return "spinsim_b200 0.1.0 (sm_100a)"; }
 
 extern "C" int spinsim_last_error(char* buf, size_t n) {
@@ -282,11 +288,14 @@ extern "C" int spinsim_plan_create(const spinsim_plan_desc* desc, const void* fi
         p->m.lanes = 1;
     } else if (d.field_kind != SPINSIM_FIELD_USER) {
         // Register budget: the kernel built for MINB resident 128-thread CTAs per SM whose cap is the
-        // largest that fits max_registers (0 = no cap): 6 -> 80, 5 -> 96, 4 -> 128, 3 -> 168
-        // registers, 2 uncapped.  Budgets of 80 and 96 exist only for some kernels; without one the
-        // next larger budget is taken.
+        // largest that fits max_registers: 6 -> 80, 5 -> 96, 4 -> 128, 3 -> 168 registers, 2 uncapped.
+        // Budgets of 80 and 96 exist only for some kernels; without one the next larger budget is taken.
+        // By default 128, except for the eight-generator exponential, whose 3 x 3 temporaries would
+        // spill, and 96 for FP32-bulk tables, bound by latency: a launch of 400 pulse trains takes 723 us
+        // at 168, 637 at 128, 568 at 96 and 512 at 80, where an interpolated table's steps spill too much.
         const int mr = d.max_registers;
-        const int want_minb = mr <= 0 ? 2 : mr <= 80 ? 6 : mr <= 96 ? 5 : mr <= 128 ? 4 : mr <= 168 ? 3 : 2;
+        const bool bulk_table = d.field_kind == SPINSIM_FIELD_TABLE && d.precision == SPINSIM_PRECISION_FP32_BULK;
+        const int want_minb = mr <= 0 ? (eo == EXPO_LIE_TROTTER_8 ? 2 : bulk_table ? 5 : 4) : mr <= 80 ? 6 : mr <= 96 ? 5 : mr <= 128 ? 4 : mr <= 168 ? 3 : 2;
         for (int minb = want_minb; minb >= 2 && !p->func; minb--) {
             for (const BuiltinEntry& b : kBuiltin) {
                 if (b.dims == d.spin_dim && b.integ == d.integration && b.expo_h == eh && b.expo_o == eo &&
@@ -603,11 +612,12 @@ int launch_prefix(const ScanArgs& a, const ScanBuffers& b, const bool* has_dim, 
 // implicit tiles.
 // partials: the tensor-path time evolution has written each tile's warp partials into b.tile_product
 // (the tile products kernels are then not launched).
+// products: the time evolution has written the tile products themselves.
 // rows (partials mode, may be null): each output step's operator as its SU(2) pair, which the apply
 // reads in place of u.
 int launch_scan(const Instance* inst_dev, const Instance* single, const ScanBuffers& b, const double* u, double* state,
                 double* spin, cudaStream_t s, int stages = SCAN_ALL, double* total = nullptr, bool partials = false,
-                const double* rows = nullptr) {
+                const double* rows = nullptr, bool products = false) {
     if (b.n_tiles == 0) return SPINSIM_OK;
     ScanArgs a;
     memset(&a, 0, sizeof(a));
@@ -644,9 +654,9 @@ int launch_scan(const Instance* inst_dev, const Instance* single, const ScanBuff
     int rc = device_sm_count(&sm);
     if (rc) return rc;
     if (stages & SCAN_PREFIX) {
-        if (grid[0] && !partials)
+        if (grid[0] && !partials && !products)
             CUDA_TRY(launch_early(scan_products_kernel<2>, dim3(grid[0]), dim3(t2), m2, s, a, lo[0], hi[0]));
-        if (grid[1] && !partials)
+        if (grid[1] && !partials && !products)
             CUDA_TRY(launch_early(scan_products_kernel<3>, dim3(grid[1]), dim3(t3), m3, s, a, lo[1], hi[1]));
         const bool has_dim[2] = {grid[0] != 0, grid[1] != 0};
         rc = launch_prefix(a, b, has_dim, sm, s);
@@ -834,6 +844,8 @@ static int evaluate_impl(const spinsim_plan* p, const spinsim_field* field, doub
     a.tile_partials = partials ? b.tile_product : nullptr;
     a.scan_begin = nullptr;
     a.rows = partials ? rows : nullptr;
+    const bool products = with_scan && warps_write_products(p, a.m.lanes) && n_out > kScanShort;
+    a.tile_products = products ? b.tile_product : nullptr;
     if (p->cta_tiles) {
         Instance* inst_dev = c.take<Instance>(1);
         FieldDesc* field_dev = c.take<FieldDesc>(1);
@@ -844,7 +856,7 @@ static int evaluate_impl(const spinsim_plan* p, const spinsim_field* field, doub
     }
     rc = launch_evolve(p, a, a.n_tiles, s, p->cta_tiles);
     if (rc || !with_scan) return rc;
-    return launch_scan(nullptr, &inst, b, u, state, spin, s, SCAN_ALL, nullptr, partials, a.rows);
+    return launch_scan(nullptr, &inst, b, u, state, spin, s, SCAN_ALL, nullptr, partials, a.rows, products);
 }
 
 extern "C" int spinsim_evaluate(const spinsim_plan* plan, const spinsim_field* field, double t0, double dt_int,
@@ -1354,6 +1366,8 @@ extern "C" int spinsim_batch_launch(const spinsim_batch* b, double* time_dev, do
     a.step_norms = p->desc.precision == SPINSIM_PRECISION_FP32_BULK ? b->step_norms : nullptr;
     a.tile_partials = b->partials ? b->scan.tile_product : nullptr;  // the same kernel work with or without the scan
     a.rows = b->partials ? b->rows : nullptr;
+    const bool products = warps_write_products(p, b->lanes);
+    a.tile_products = products ? b->scan.tile_product : nullptr;
     a.scan_begin = b->scan.begin;
     if (b->consts != nullptr && b->scan.n_instances > 0) {  // the tensor path's per-instance constants first
         int rc = launch_dmma_consts(&a, b->consts, b->scan.n_instances, nullptr, nullptr, s);
@@ -1361,7 +1375,8 @@ extern "C" int spinsim_batch_launch(const spinsim_batch* b, double* time_dev, do
     }
     int rc = launch_evolve(p, a, b->n_tiles, s, a.dmma_consts != nullptr);
     if (rc || !state_dev) return rc;
-    rc = launch_scan(b->inst_dev, nullptr, b->scan, u_dev, state_dev, spin_dev, s, SCAN_ALL, nullptr, b->partials, a.rows);
+    rc = launch_scan(b->inst_dev, nullptr, b->scan, u_dev, state_dev, spin_dev, s, SCAN_ALL, nullptr, b->partials, a.rows,
+                     products);
     return rc;
 }
 

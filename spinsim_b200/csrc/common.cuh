@@ -109,6 +109,8 @@ struct EvolveArgs {
     double* tile_partials;   // tensor path: per scan tile (kScanTile output steps, kScanMat doubles), each
                              // warp's product of its rows as an SU(2) pair in the lab frame (4 doubles per
                              // warp, warp after warp); null: not written
+    double* tile_products;   // other plans with one lane per output step: per scan tile (kScanMat doubles), the
+                             // product of the tile's operators; null: not written
     const int32_t* scan_begin;  // per instance: its first scan tile (null: one instance, tile 0)
     const struct DmmaConsts* dmma_consts;  // tensor path: per instance, written by dmma_consts_kernel
                                            // earlier in the launch (null: each tile computes them)

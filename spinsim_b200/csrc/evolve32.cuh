@@ -242,28 +242,17 @@ SS_D void spin_one_euler_step(Mat<3>& u, const double* g, float* nsq) {
     apply_split3(u, lin, rest);
 }
 
-// P <- (1 + E) P in FP64 with E = -i g.sigma/2 (g the step's FP64 generator: the linear part, never
-// rounded to FP32) + rest (its FP32 remainder).
-SS_D void su2_apply_split(Su2d& p, double gx, double gy, double gz, const Su2f& rest) {
-    const c64 am1 = c64{(double)rest.am1.re, fma(-0.5, gz, (double)rest.am1.im)};
-    const c64 b = c64{fma(0.5, gy, (double)rest.beta.re), fma(-0.5, gx, (double)rest.beta.im)};
-    // alpha' = alpha_e alpha - conj(beta_e) beta ; beta' = beta_e alpha + conj(alpha_e) beta
-    const c64 alpha = c64{1.0 + p.am1.re, p.am1.im};
-    const c64 beta = p.beta;
-    // (alpha - 1) + am1 alpha - conj(b) beta and b alpha + conj(am1) beta + beta, each part one chain
-    // of four FMAs
-    c64 na, nb;
-    na.re = fma(-am1.im, alpha.im, fma(am1.re, alpha.re, fma(-b.im, beta.im, fma(-b.re, beta.re, p.am1.re))));
-    na.im = fma(am1.im, alpha.re, fma(am1.re, alpha.im, fma(b.im, beta.re, fma(-b.re, beta.im, p.am1.im))));
-    nb.re = fma(-b.im, alpha.im, fma(b.re, alpha.re, fma(am1.im, beta.im, fma(am1.re, beta.re, beta.re))));
-    nb.im = fma(b.im, alpha.re, fma(b.re, alpha.im, fma(-am1.im, beta.re, fma(am1.re, beta.im, beta.im))));
-    p.am1 = na;
-    p.beta = nb;
+// The step's element E = -i g.sigma/2 (g the step's FP64 generator: the linear part, never rounded to
+// FP32) + rest (its FP32 remainder), in FP64.
+SS_D Su2d su2_split(double gx, double gy, double gz, const Su2f& rest) {
+    return Su2d{c64{(double)rest.am1.re, fma(-0.5, gz, (double)rest.am1.im)},
+                c64{fma(0.5, gy, (double)rest.beta.re), fma(-0.5, gx, (double)rest.beta.im)}};
 }
 
 // One CF4 step as an SU(2) element: E = Ea + Eb + Eb Ea with Ea = exp(-i ga.sigma/2) - 1; its linear
-// part -i (ga + gb).sigma/2 in FP64, the series remainders and the product Eb Ea in FP32.
-SS_D void su2_cf4_step(Su2d& p, const double* ga, const double* gb, float* nsq) {
+// part -i (ga + gb).sigma/2 in FP64, the series remainders and the product Eb Ea in FP32.  *nsq
+// accumulates |g|^2 of both generators.
+SS_D Su2d su2_cf4_element(const double* ga, const double* gb, float* nsq) {
     float a[3], b[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
@@ -274,19 +263,19 @@ SS_D void su2_cf4_step(Su2d& p, const double* ga, const double* gb, float* nsq) 
     const Su2f ra = su2_exp_rest(a[0], a[1], a[2]);
     const Su2f rb = su2_exp_rest(b[0], b[1], b[2]);
     const Su2f prod = su2_prod(su2_full(b[0], b[1], b[2], rb), su2_full(a[0], a[1], a[2], ra));
-    su2_apply_split(p, ga[0] + gb[0], ga[1] + gb[1], ga[2] + gb[2], su2_add(su2_add(ra, rb), prod));
+    return su2_split(ga[0] + gb[0], ga[1] + gb[1], ga[2] + gb[2], su2_add(su2_add(ra, rb), prod));
 }
 
 // One Euler step (a single exponential of the generator g, I:759-791) in the same split: the linear
 // part in FP64, the remainder in FP32.
-SS_D void su2_euler_step(Su2d& p, const double* g, float* nsq) {
+SS_D Su2d su2_euler_element(const double* g, float* nsq) {
     float a[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
         a[c] = __double2float_rn(g[c]);
         *nsq = fmaf(a[c], a[c], *nsq);
     }
-    su2_apply_split(p, g[0], g[1], g[2], su2_exp_rest(a[0], a[1], a[2]));
+    return su2_split(g[0], g[1], g[2], su2_exp_rest(a[0], a[1], a[2]));
 }
 
 // ---------------------------------------------------------------------------------- generic bulk path
@@ -309,7 +298,7 @@ __device__ __noinline__ SpinOneProduct spin_one_quadratic_steps32(const FieldDes
                                                                   Generators4 g, int j, int j1, float nsq) {
     bool first = true;
     for (; j < j1; j++) {
-        if (!first) step_generators<FIELD, 4, 1, INTEG>(f, st, g.a, g.b);
+        if (!first) step_generators<FIELD, 4, INTEG>(f, st, g.a, g.b);
         first = false;
         if constexpr (INTEG == INTEG_EULER) spin_one_euler_step(u, g.a, &nsq);
         else spin_one_cf4_step(u, g.a, g.b, &nsq);
@@ -317,32 +306,25 @@ __device__ __noinline__ SpinOneProduct spin_one_quadratic_steps32(const FieldDes
     return SpinOneProduct{u, nsq};
 }
 
-template <int D, int INTEG, int EXPO, int FIELD>
+// Every lane of the warp calls this, as interval64 (whose DIMS and step loop these are).
+template <int DIMS, int INTEG, int FIELD>
 SS_D void interval32(const MethodConfig& m, const Instance& inst, const FieldDesc& f, int64_t index, bool active,
-                     int lane_in_group, double* time_out, double* u_out, float* norms_out) {
-    static_assert(EXPO != EXPO_LIE_TROTTER_8, "the FP32-bulk form has no eight-generator exponential");
-    constexpr int L = (D == 2) ? 3 : 4;
-    constexpr int P = (D == 2) ? 2 : 1;  // power of the frame winding in the xy transform (I:599-613)
+                     int lane_in_group, double* time_out, double* u_out, float* norms_out, double* product_out) {
+    constexpr int L = LieDim<DIMS, EXPO_LIE_TROTTER>::value;
+    const int dim = DIMS != 0 ? DIMS : inst.dim;
     const int lanes = m.lanes;
     const double dt = inst.dt_int, dt_out = inst.dt_out;
     const double t_c = __dadd_rn(inst.t0, __dmul_rn(dt_out, (double)(inst.interval0 + index)));  // I:818, unfused
-    double rw = 0.0;
-    if (active && m.rotating) {
-        double s0[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) s0[k] = 0.0;
-        sample_field<FIELD, L>(f, t_c + dt_out / 2, s0);
-        rw = s0[2];
-        if (D == 2) rw /= 2;
-    }
+    double prw = 0.0;
+    if (active && m.rotating) prw = sample_z<FIELD, L>(f, t_c + dt_out / 2);
+    const double rw = dim == 2 ? prw / 2 : prw;
     const int K = active ? inst.n_fine : 0;
     const int j0 = (int)(((int64_t)K * lane_in_group) / lanes);
     const int j1 = (int)(((int64_t)K * (lane_in_group + 1)) / lanes);
 
-    Steps<L> st;
-    set_integrator<INTEG>(st, dt);
-    st.template begin<P, INTEG>(m, rw, t_c, j0, K);
-    auto next_generators = [&](double* ga, double* gb) { step_generators<FIELD, L, P, INTEG>(f, st, ga, gb); };
+    const StepRule rule = step_rule<INTEG>(t_c, dt);
+    Steps<L> st(rule);
+    auto next_generators = [&](double* ga, double* gb) { step_generators<FIELD, L, INTEG>(f, st, ga, gb); };
 
     // Phase 1: every step an SU(2) element (spin half always; spin one while the quadratic shift
     // is zero); the interval product is an FP64 SU(2) element.  Software-pipelined: the next step's
@@ -352,39 +334,39 @@ SS_D void interval32(const MethodConfig& m, const Instance& inst, const FieldDes
     float nsq = 0.0f;  // sum of |g|^2 over this lane's steps (the error statement's scale)
     int j = j0;
     bool pending = false;
-    if (j < j1) next_generators(ga, gb);
+    auto quadratic_step = [&]() { return DIMS != 2 && dim == 3 && (ga[3] != 0.0 || gb[3] != 0.0); };
+    if constexpr (FIELD == FIELD_TABLE) {
+        auto element = [&](const double* a, const double* b, int n) {
+            float step = 0.0f;
+            const Su2d e = INTEG == INTEG_EULER ? su2_euler_element(a, &step) : su2_cf4_element(a, b, &step);
+            nsq = fmaf((float)n, step, nsq);
+            return e;
+        };
+        if (hold_steps<INTEG>(f, dim, m.rotating && prw != 0.0, rule, j0, j1, dt_out, su2, element)) j = j1;
+    }
+    if (j < j1) {
+        st.template begin<INTEG>(m, prw, j0, K);
+        next_generators(ga, gb);
+    }
     for (; j < j1; j++) {
-        if constexpr (D == 3) {
-            if (ga[3] != 0.0 || gb[3] != 0.0) {
-                pending = true;
-                break;
-            }
+        if (quadratic_step()) {
+            pending = true;
+            break;
         }
         double na[4] = {0.0, 0.0, 0.0, 0.0}, nb[4] = {0.0, 0.0, 0.0, 0.0};
         if (j + 1 < j1) next_generators(na, nb);
-        if constexpr (INTEG == INTEG_EULER) su2_euler_step(su2, ga, &nsq);
-        else su2_cf4_step(su2, ga, gb, &nsq);
+        if constexpr (INTEG == INTEG_EULER) su2_apply64(su2, su2_euler_element(ga, &nsq));
+        else su2_apply64(su2, su2_cf4_element(ga, gb, &nsq));
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             ga[k] = na[k];
             gb[k] = nb[k];
         }
     }
-    Mat<D> u;
-    {
-        const c64 alpha = c64{1.0 + su2.am1.re, su2.am1.im};
-        if constexpr (D == 3) {
-            u = su2_to_spin_one(alpha, su2.beta);
-        } else {
-            u.a[0][0] = alpha;
-            u.a[1][0] = su2.beta;
-            u.a[0][1] = c64{-su2.beta.re, su2.beta.im};
-            u.a[1][1] = conj(alpha);
-        }
-    }
     // Phase 2 (spin one with a quadratic shift): full 3x3 exponentials and an FP64 3x3 product.
     // The pending step's generators are in ga, gb.
-    if constexpr (D == 3) {
+    Mat<3> u;
+    if constexpr (DIMS != 2) {
         if (pending) {
             Generators4 g;
 #pragma unroll
@@ -392,35 +374,17 @@ SS_D void interval32(const MethodConfig& m, const Instance& inst, const FieldDes
                 g.a[k] = ga[k];
                 g.b[k] = gb[k];
             }
-            const SpinOneProduct r = spin_one_quadratic_steps32<INTEG, FIELD>(f, st, u, g, j, j1, nsq);
+            const SpinOneProduct r = spin_one_quadratic_steps32<INTEG, FIELD>(
+                f, st, su2_to_spin_one(c64{1.0 + su2.am1.re, su2.am1.im}, su2.beta), g, j, j1, nsq);
             u = r.u;
             nsq = r.nsq;
         }
     }
-
-    for (int s = 1; s < lanes; s <<= 1) {
-        const Mat<D> later = shfl_down_mat(u, s);
-        nsq += __shfl_down_sync(0xffffffffu, nsq, s);
-        if ((lane_in_group & (2 * s - 1)) == 0) u = matmul(later, u);
-    }
-    if (!active || lane_in_group != 0) return;
-    if (m.rotating) {  // leave the rotating frame, I:839-852
-        c64 wo;
-        sincos(rw * dt_out, &wo.im, &wo.re);
-        const c64 woc = conj(wo);
-#pragma unroll
-        for (int k = 0; k < D; k++) {
-            u.a[0][k] = u.a[0][k] * woc;
-            u.a[D - 1][k] = u.a[D - 1][k] * wo;
-        }
-    }
-    time_out[index] = t_c;
-    if (norms_out != nullptr) norms_out[index] = nsq;
-    double2* dst = reinterpret_cast<double2*>(u_out) + index * (D * D);
-#pragma unroll
-    for (int i = 0; i < D; i++)
-#pragma unroll
-        for (int k = 0; k < D; k++) dst[i * D + k] = make_double2(u.a[i][k].re, u.a[i][k].im);
+    for (int s = 1; s < lanes; s <<= 1) nsq += __shfl_down_sync(0xffffffffu, nsq, s);
+    const bool writes = active && lane_in_group == 0;
+    if (writes && norms_out != nullptr) norms_out[index] = nsq;
+    finish_steps<DIMS>(m, dim, su2, u, pending, lanes, lane_in_group, rw, dt_out, writes, t_c, index, time_out, u_out,
+                       product_out);
 }
 
 // ---------------------------------------------------------------------------------- tone synthesis
@@ -602,7 +566,7 @@ SS_D void intervals32_synth(const MethodConfig& m, const Instance& inst, const F
                 ga[c] = fma(c0, sa[i][c], c1 * sb[i][c]);
                 gb[c] = fma(c1, sa[i][c], c0 * sb[i][c]);
             }
-            su2_cf4_step(su2[i], ga, gb, &nsq[i]);
+            su2_apply64(su2[i], su2_cf4_element(ga, gb, &nsq[i]));
         }
     }
     __syncwarp();  // the shared slots are reused by the warp's next tile

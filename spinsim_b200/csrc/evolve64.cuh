@@ -12,10 +12,10 @@
 
 namespace spinsim {
 
-// Lie-algebra dimension of the field vector (I:547-554).
-template <int D, int EXPO>
+// Components of the field vector (I:547-554); spin half in a mixed-spin kernel (DIMS 0) ignores the fourth.
+template <int DIMS, int EXPO_ONE>
 struct LieDim {
-    static constexpr int value = (D == 2) ? 3 : (EXPO == EXPO_LIE_TROTTER_8 ? 8 : 4);
+    static constexpr int value = DIMS == 2 ? 3 : EXPO_ONE == EXPO_LIE_TROTTER_8 ? 8 : 4;
 };
 
 // transform_frame_* for the eight-generator exponential (I:582-618).  Division by the unit winding w is
@@ -38,52 +38,74 @@ SS_D void transform_frame_lt8(double* s, double rw, c64 w) {
 // (about one rounding a step) stays far below the phase's own argument rounding.
 constexpr int kPhasorSteps = 64;
 
-// What a step loop's field samples need: the frame phasors exp(-i P rw tau) at the step's two samples
-// and their rotation by one step, the interval's start and the step's number, the sample offsets and
-// weights, and the table cursors.  A sample's time is t_c + tau with tau = j dt + offset, rounded once
-// each: the reference's running sum of steps (I:836) agrees with it to its own rounding, and the frame's
-// phase (at tau) stays consistent with the field's (at t_c + tau), whose common part cancels in the
-// rotating frame.
+// Where an interval's steps sample the field and how they weight the samples: the interval's start, the
+// reference's sample offsets and weights of an integrator for steps of dt (I:624-686 Magnus CF4 at the two
+// Gauss points, I:693-752 Heun at the step's ends, I:759-791 Euler at its middle).  A sample's time is t_c + tau
+// with tau = j dt + offset, rounded once each: the reference's running sum of steps (I:836) agrees with it
+// to its own rounding, and the frame's phase (at tau) stays consistent with the field's (at t_c + tau), whose
+// common part cancels in the rotating frame.
+struct StepRule {
+    double t_c, dt, off_a, off_b, c0, c1;
+};
+
+template <int INTEG>
+SS_D StepRule step_rule(double t_c, double dt) {
+    const double a_lo = 0.5 * dt * (1.0 - 1.0 / kSqrt3);
+    const double a_hi = 0.5 * dt * (1.0 + 1.0 / kSqrt3);
+    const double w0 = (1.5 + kSqrt3) / 6.0, w1 = (1.5 - kSqrt3) / 6.0;
+    StepRule r;
+    r.t_c = t_c;
+    r.dt = dt;
+    r.off_a = INTEG == INTEG_CF4 ? a_lo : INTEG == INTEG_HEUN ? 0.0 : 0.5 * dt;
+    r.off_b = INTEG == INTEG_CF4 ? a_hi : dt;
+    r.c0 = INTEG == INTEG_CF4 ? dt * w0 : INTEG == INTEG_HEUN ? 0.5 * dt : dt;
+    r.c1 = INTEG == INTEG_CF4 ? dt * w1 : 0.0;
+    return r;
+}
+
+// What a step loop's field samples need: the rule, the step's number, the frame phasors exp(-i prw tau),
+// prw = P rw with P the power of the frame winding in the xy transform (I:599-613: 2 for spin half, 1 for
+// spin one), at the step's two samples and their rotation by one step, and the table cursors.
 template <int L>
-struct Steps {
+struct Steps : StepRule {
     c64 wa, wb, wrot;
-    double rw, t_c, j, dt, off_a, off_b, c0, c1;
+    double prw, j;
     bool rotating;
     TableCursor cur[L];
 
+    SS_D Steps(const StepRule& rule) : StepRule(rule) {}
     SS_D double tau(double off) const { return fma(j, dt, off); }
 
-    template <int P, int INTEG>
+    template <int INTEG>
     SS_D void start_phasors() {
-        sincos(-(double)P * rw * tau(off_a), &wa.im, &wa.re);
-        if (INTEG != INTEG_EULER) sincos(-(double)P * rw * tau(off_b), &wb.im, &wb.re);
+        sincos(-prw * tau(off_a), &wa.im, &wa.re);
+        if (INTEG != INTEG_EULER) sincos(-prw * tau(off_b), &wb.im, &wb.re);
     }
     // Steps from number `first` of an interval that starts at t (steps: how many it has; 0: none).
-    template <int P, int INTEG>
-    SS_D void begin(const MethodConfig& m, double interval_rw, double t, int first, int steps) {
-        rw = interval_rw;
-        t_c = t;
+    template <int INTEG>
+    SS_D void begin(const MethodConfig& m, double interval_prw, int first, int steps) {
+        prw = interval_prw;
         j = (double)first;
         rotating = m.rotating;
         wa = wb = wrot = c64{1.0, 0.0};
-        if (m.rotating && steps > 0) {
-            sincos(-(double)P * rw * dt, &wrot.im, &wrot.re);
-            start_phasors<P, INTEG>();
+        if (m.rotating && steps > 0 && prw != 0.0) {
+            sincos(-prw * dt, &wrot.im, &wrot.re);
+            start_phasors<INTEG>();
         }
 #pragma unroll
         for (int c = 0; c < L; c++) cur[c] = TableCursor{};  // for the increasing sample times of the steps
     }
     // Before the samples of step n of a lane that began at step n0: the phasors from sincos every
     // kPhasorSteps steps.
-    template <int P, int INTEG>
+    template <int INTEG>
     SS_D void restart(int n, int n0) {
-        if (rotating && (n - n0) % kPhasorSteps == 0) start_phasors<P, INTEG>();
+        if (rotating && prw != 0.0 && (n - n0) % kPhasorSteps == 0) start_phasors<INTEG>();
     }
 };
 
 // One step's field samples (FP64) -> frame transform -> the integrator's generators (FP64); the
 // step number and the frame phasors move on.
-template <int FIELD, int L, int P, int INTEG>
+template <int FIELD, int L, int INTEG>
 SS_D void step_generators(const FieldDesc& f, Steps<L>& st, double* ga, double* gb) {
     double s0[8], s1[8];  // a user field writes all eight channels
 #pragma unroll
@@ -94,17 +116,17 @@ SS_D void step_generators(const FieldDesc& f, Steps<L>& st, double* ga, double* 
     sample_field<FIELD, L>(f, st.t_c + st.tau(st.off_a), s0, st.cur);
     if (INTEG != INTEG_EULER) sample_field<FIELD, L>(f, st.t_c + st.tau(st.off_b), s1, st.cur);
     st.j += 1.0;
-    if (st.rotating) {  // xy times exp(-i P rw tau), z minus P rw
+    if (st.rotating) {  // xy times exp(-i prw tau), z minus prw
         const c64 xa = c64{s0[0], s0[1]} * st.wa;
         s0[0] = xa.re;
         s0[1] = xa.im;
-        s0[2] -= (double)P * st.rw;
+        s0[2] -= st.prw;
         st.wa = st.wa * st.wrot;
         if (INTEG != INTEG_EULER) {
             const c64 xb = c64{s1[0], s1[1]} * st.wb;
             s1[0] = xb.re;
             s1[1] = xb.im;
-            s1[2] -= (double)P * st.rw;
+            s1[2] -= st.prw;
             st.wb = st.wb * st.wrot;
         }
     }
@@ -119,18 +141,45 @@ struct Generators4 {
     double a[4], b[4];
 };
 
-// The reference's sample offsets and weights of an integrator for steps of dt (I:624-686 Magnus CF4 at
-// the two Gauss points, I:693-752 Heun at the step's ends, I:759-791 Euler at its middle).
-template <int INTEG, int L>
-SS_D void set_integrator(Steps<L>& st, double dt) {
-    const double a_lo = 0.5 * dt * (1.0 - 1.0 / kSqrt3);
-    const double a_hi = 0.5 * dt * (1.0 + 1.0 / kSqrt3);
-    const double w0 = (1.5 + kSqrt3) / 6.0, w1 = (1.5 - kSqrt3) / 6.0;
-    st.dt = dt;
-    st.off_a = INTEG == INTEG_CF4 ? a_lo : INTEG == INTEG_HEUN ? 0.0 : 0.5 * dt;
-    st.off_b = INTEG == INTEG_CF4 ? a_hi : dt;
-    st.c0 = INTEG == INTEG_CF4 ? dt * w0 : INTEG == INTEG_HEUN ? 0.5 * dt : dt;
-    st.c1 = INTEG == INTEG_CF4 ? dt * w1 : 0.0;
+// Steps j0 .. j1 - 1 of an interval whose field is piecewise constant and whose frame does not turn (pulse
+// trains), as runs: the steps between two knots share one element, and their product is its power by
+// squarings; a step with a knot between its samples is a run of its own.  element(ga, gb, n) is the element of
+// n steps of these generators.  False, with nothing done, unless every lane of the warp (which all call
+// this) can take this form.  Bound by latency (the knots' search and the runs' divergence).  A launch of 400
+// pulse trains (4.1e6 output steps of 20, FP32-bulk, 96 registers): 1806 -> 568 us.
+template <int INTEG, typename Element>
+SS_D bool hold_steps(const FieldDesc& f, int dim, bool turns, const StepRule& st, int j0, int j1, double dt_out, Su2d& p,
+                     Element element) {
+    if (__any_sync(0xffffffffu, turns)) return false;
+    HoldChannel ch[3];
+    const double first = __shfl_sync(0xffffffffu, st.t_c, 0);
+    if (!hold_channels(f, dim == 2 ? 3 : 4, first, first + 33.0 * dt_out, ch)) return false;
+    const double dt = st.dt, last = INTEG == INTEG_EULER ? st.off_a : st.off_b;
+    for (int j = j0, n; j < j1; j += n) {
+        const double ta = st.t_c + fma((double)j, dt, st.off_a), tb = st.t_c + fma((double)j, dt, last);
+        double sa[3], ga[3], gb[3];
+        double until = INFINITY;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            sa[c] = ch[c].at(f, c, ta);
+            until = fmin(until, ch[c].t_hi);
+        }
+        n = 1;
+        if (tb < until) {
+            // an estimate, made safe below: a run cut short goes on as another one
+            const float more = __fdividef((float)(until - tb), (float)dt);
+            n = more >= (float)(j1 - j) ? j1 - j : 1 + (int)more;
+            while (n > 1 && !(st.t_c + fma((double)(j + n - 1), dt, last) < until)) n--;
+        }
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            const double sb = INTEG == INTEG_EULER ? 0.0 : tb < until ? sa[c] : ch[c].at(f, c, tb);
+            ga[c] = fma(st.c0, sa[c], st.c1 * sb);
+            gb[c] = INTEG == INTEG_HEUN ? st.c0 * sb : fma(st.c1, sa[c], st.c0 * sb);
+        }
+        su2_apply_power64(p, element(ga, gb, n), n);
+    }
+    return true;
 }
 
 // Steps j .. j1 - 1 of a spin-one interval whose quadratic shift is non-zero: full 3 x 3 exponentials
@@ -144,8 +193,8 @@ __device__ __noinline__ Mat<3> spin_one_quadratic_steps64(const MethodConfig& m,
         spin_one_step64(m, u, g.a);
         if constexpr (INTEG != INTEG_EULER) spin_one_step64(m, u, g.b);
         if (++j >= j1) return u;
-        st.template restart<1, INTEG>(j, j0);
-        step_generators<FIELD, 4, 1, INTEG>(f, st, g.a, g.b);
+        st.template restart<INTEG>(j, j0);
+        step_generators<FIELD, 4, INTEG>(f, st, g.a, g.b);
     }
 }
 
@@ -159,13 +208,12 @@ SS_D Mat<3> interval_lt8(const MethodConfig& m, const FieldDesc& f, double t_c, 
     TableCursor cur[L];  // per-channel table cursors for the increasing sample times of the steps
 #pragma unroll
     for (int c = 0; c < L; c++) cur[c] = TableCursor{};
-    Steps<L> st;
-    set_integrator<INTEG>(st, dt);
-    st.j = (double)j0;
+    const StepRule st = step_rule<INTEG>(t_c, dt);
+    double step = (double)j0;
     auto sample = [&](double* s, double off) {
 #pragma unroll
         for (int k = 0; k < L; k++) s[k] = 0.0;
-        const double tau = st.tau(off);
+        const double tau = fma(step, dt, off);
         c64 w = c64{1.0, 0.0};
         if (m.rotating) sincos(rw * tau, &w.im, &w.re);
         sample_field<FIELD, L>(f, t_c + tau, s, cur);
@@ -183,103 +231,188 @@ SS_D Mat<3> interval_lt8(const MethodConfig& m, const FieldDesc& f, double t_c, 
             for (int k = 0; k < L; k++) g[k] = INTEG == INTEG_CF4 ? st.c1 * s0[k] + st.c0 * s1[k] : st.c0 * s1[k];
             u = matmul(expo_lt8_one(g, m.hypercubes, m.precision), u);
         }
-        st.j += 1.0;
+        step += 1.0;
     }
     return u;
+}
+
+// Leave the rotating frame (I:839-852): the operator of an SU(2) pair, or a d x d operator.
+template <int D>
+SS_D void leave_frame(Su2p& v, double rw, double dt_out) {
+    c64 w;  // spin one, whose representation doubles the phase: half of it
+    sincos(rw * dt_out * (D == 2 ? 1.0 : 0.5), &w.im, &w.re);
+    v.a = v.a * conj(w);
+    v.b = v.b * w;
+}
+
+template <int D>
+SS_D void leave_frame(Mat<D>& u, double rw, double dt_out) {
+    c64 w;
+    sincos(rw * dt_out, &w.im, &w.re);
+    const c64 wc = conj(w);
+#pragma unroll
+    for (int k = 0; k < D; k++) {
+        u.a[0][k] = u.a[0][k] * wc;
+        u.a[D - 1][k] = u.a[D - 1][k] * w;
+    }
+}
+
+SS_D void identity_of(Su2p& v) { v = su2p_identity(); }
+template <int D>
+SS_D void identity_of(Mat<D>& u) {
+    set_identity(u);
+}
+template <int D>
+SS_D Mat<D> operator_of(const Su2p& v) {
+    return su2p_to_mat<D>(v);
+}
+template <int D>
+SS_D Mat<D> operator_of(const Mat<D>& u) {
+    return u;
+}
+SS_D Su2p shfl_down_operator(const Su2p& v, int s) { return shfl_down_su2p(v, s); }
+template <int D>
+SS_D Mat<D> shfl_down_operator(const Mat<D>& u, int s) {
+    return shfl_down_mat(u, s);
+}
+SS_D Su2p later_times(const Su2p& later, const Su2p& v) { return su2p_mul(later, v); }
+template <int D>
+SS_D Mat<D> later_times(const Mat<D>& later, const Mat<D>& u) {
+    return matmul(later, u);
+}
+
+// An interval's outputs, from its rotating-frame operator v: an SU(2) pair, or a d x d operator.  With
+// product_out (a warp's 32 intervals are then one tile of the state scan) also the product of the warp's
+// operators, in five shuffle rounds, which saves the scan a pass over U: 56 + 63 us of a launch of 400
+// pulse trains (4.1e6 output steps).
+template <int D, typename V>
+SS_D void finish_interval(const MethodConfig& m, V v, double rw, double dt_out, bool writes, double t_c, int64_t index,
+                          double* time_out, double* u_out, double* product_out) {
+    if (!writes) identity_of(v);
+    else if (m.rotating && rw != 0.0) leave_frame<D>(v, rw, dt_out);
+    if (writes) {
+        const Mat<D> u = operator_of<D>(v);
+        time_out[index] = t_c;
+        double2* dst = reinterpret_cast<double2*>(u_out) + index * (D * D);
+#pragma unroll
+        for (int i = 0; i < D; i++)
+#pragma unroll
+            for (int k = 0; k < D; k++) dst[i * D + k] = make_double2(u.a[i][k].re, u.a[i][k].im);
+    }
+    if (product_out == nullptr) return;
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+        const V later = shfl_down_operator(v, s);
+        if ((lane & (2 * s - 1)) == 0) v = later_times(later, v);
+    }
+    if (lane == 0) {
+        const Mat<D> u = operator_of<D>(v);
+        double2* dst = reinterpret_cast<double2*>(product_out);
+#pragma unroll
+        for (int i = 0; i < D; i++)
+#pragma unroll
+            for (int k = 0; k < D; k++) dst[i * D + k] = make_double2(u.a[i][k].re, u.a[i][k].im);
+    }
+}
+
+// Combine the lanes' partial products in step order: later steps multiply from the left.
+template <typename V>
+SS_D void combine_lanes(V& v, int lanes, int lane_in_group) {
+    for (int s = 1; s < lanes; s <<= 1) {
+        const V later = shfl_down_operator(v, s);
+        if ((lane_in_group & (2 * s - 1)) == 0) v = later_times(later, v);
+    }
+}
+
+// The end of an interval whose lanes hold SU(2) products p, or, where a step with a quadratic shift was met
+// (spin one), 3 x 3 products u.  Every lane of the warp calls this.
+template <int DIMS>
+SS_D void finish_steps(const MethodConfig& m, int dim, const Su2d& p, Mat<3>& u, bool quadratic, int lanes,
+                       int lane_in_group, double rw, double dt_out, bool writes, double t_c, int64_t index,
+                       double* time_out, double* u_out, double* product_out) {
+    Su2p pair = Su2p{c64{1.0 + p.am1.re, p.am1.im}, p.beta};
+    if (DIMS != 2 && __any_sync(0xffffffffu, quadratic)) {
+        if (!quadratic) u = su2p_to_mat<3>(pair);
+        combine_lanes(u, lanes, lane_in_group);
+        finish_interval<3>(m, u, rw, dt_out, writes, t_c, index, time_out, u_out, product_out);
+        return;
+    }
+    combine_lanes(pair, lanes, lane_in_group);
+    if (DIMS != 3 && dim == 2)
+        finish_interval<2>(m, pair, rw, dt_out, writes, t_c, index, time_out, u_out, product_out);
+    else if (DIMS != 2)
+        finish_interval<3>(m, pair, rw, dt_out, writes, t_c, index, time_out, u_out, product_out);
 }
 
 // Evolve one output interval.  Every lane of the warp must call this (shuffles use the full mask);
 // lanes with `active == false` do no steps and write nothing.
 //
-// Bound by the FP64 pipe.  The step's exponentials are SU(2) elements for both spins (su2_step64; spin one
+// Bound by the FP64 pipe.  The step's exponentials are SU(2) elements for both spins (su2_step_element64; spin one
 // with a quadratic shift: spin_one_step64), its frame phasors come from a recurrence, and the fine
 // steps' product is kept in SU(2) residual form: about 120 FP64 operations a step besides the field
 // (600 with a quadratic shift), where the 3 x 3 squarings took over 5000.  Measured against that form,
 // a launch of each: spin-one Rabi sweep of 6.4e6 steps 3157 -> 185 us, 4001 x 50 steps with a
 // quadratic shift 149 -> 35 us, spin-half pulse ensemble of 2.05e8 steps 3832 -> 2880 us.
-template <int D, int INTEG, int EXPO, int FIELD>
+//
+// DIMS 0: a mixed-spin batch.  The spin enters only the frame winding, the exponentiator and the stored
+// operator, so both spins run one copy of the step loop.
+template <int DIMS, int INTEG, int EXPO_H, int EXPO_O, int FIELD>
 SS_D void interval64(const MethodConfig& m, const Instance& inst, const FieldDesc& f, int64_t index, bool active,
-                     int lane_in_group, double* time_out, double* u_out) {
-    constexpr int L = LieDim<D, EXPO>::value;
-    constexpr int P = (D == 2) ? 2 : 1;  // power of the frame winding in the xy transform (I:599-613)
+                     int lane_in_group, double* time_out, double* u_out, double* product_out) {
+    constexpr int L = LieDim<DIMS, EXPO_O>::value;
+    const int dim = DIMS != 0 ? DIMS : inst.dim;
     const int lanes = m.lanes;
     const double dt = inst.dt_int, dt_out = inst.dt_out;
     // I:818, rounded as the reference rounds it (no fused multiply-add), so time[] is bit-exact
     const double t_c = __dadd_rn(inst.t0, __dmul_rn(dt_out, (double)(inst.interval0 + index)));
-    double rw = 0.0;
-    if (active && m.rotating) {  // I:823-829
-        double s[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) s[k] = 0.0;
-        sample_field<FIELD, L>(f, t_c + dt_out / 2, s);
-        rw = s[2];
-        if (D == 2) rw /= 2;
-    }
+    double prw = 0.0;  // Bz at the middle of the interval (I:823-829): P rw for either spin
+    if (active && m.rotating) prw = sample_z<FIELD, L>(f, t_c + dt_out / 2);
+    const double rw = dim == 2 ? prw / 2 : prw;
     const int K = active ? inst.n_fine : 0;
     const int j0 = (int)(((int64_t)K * lane_in_group) / lanes);
     const int j1 = (int)(((int64_t)K * (lane_in_group + 1)) / lanes);
+    const bool writes = active && lane_in_group == 0;
 
-    Mat<D> u;
-    if constexpr (EXPO == EXPO_LIE_TROTTER_8) {
-        u = interval_lt8<INTEG, FIELD>(m, f, t_c, dt, rw, j0, j1);
-        for (int s = 1; s < lanes; s <<= 1) {  // later steps multiply from the left
-            const Mat<D> later = shfl_down_mat(u, s);
-            if ((lane_in_group & (2 * s - 1)) == 0) u = matmul(later, u);
-        }
+    if constexpr (DIMS == 3 && EXPO_O == EXPO_LIE_TROTTER_8) {
+        Mat<3> u = interval_lt8<INTEG, FIELD>(m, f, t_c, dt, rw, j0, j1);
+        combine_lanes(u, lanes, lane_in_group);
+        finish_interval<3>(m, u, rw, dt_out, writes, t_c, index, time_out, u_out, product_out);
     } else {
-        Steps<L> st;
-        set_integrator<INTEG>(st, dt);
-        st.template begin<P, INTEG>(m, rw, t_c, j0, K);
+        const bool lie_trotter = dim == 3 || EXPO_H == EXPO_LIE_TROTTER;
+        const StepRule rule = step_rule<INTEG>(t_c, dt);
         Su2d p = Su2d{c64{0.0, 0.0}, c64{0.0, 0.0}};
+        Mat<3> u;
         bool quadratic = false;  // a step with a quadratic shift was met: the product is in u
-        for (int j = j0; j < j1; j++) {
+        bool held = false;
+        if constexpr (FIELD == FIELD_TABLE) {
+            auto element = [&](const double* ga, const double* gb, int) {
+                Su2d e = su2_step_element64(m, lie_trotter, ga);
+                if constexpr (INTEG != INTEG_EULER) su2_apply64(e, su2_step_element64(m, lie_trotter, gb));
+                return e;
+            };
+            held = hold_steps<INTEG>(f, dim, m.rotating && prw != 0.0, rule, j0, j1, dt_out, p, element);
+        }
+        Steps<L> st(rule);
+        if (!held) st.template begin<INTEG>(m, prw, j0, K);
+        for (int j = j0; !held && j < j1; j++) {
             Generators4 g;
-            if (j != j0) st.template restart<P, INTEG>(j, j0);
-            step_generators<FIELD, L, P, INTEG>(f, st, g.a, g.b);
-            if constexpr (D == 3) {
-                if (g.a[3] != 0.0 || (INTEG != INTEG_EULER && g.b[3] != 0.0)) {
+            if (j != j0) st.template restart<INTEG>(j, j0);
+            step_generators<FIELD, L, INTEG>(f, st, g.a, g.b);
+            if constexpr (DIMS != 2) {
+                if (dim == 3 && (g.a[3] != 0.0 || (INTEG != INTEG_EULER && g.b[3] != 0.0))) {
                     quadratic = true;
                     u = spin_one_quadratic_steps64<INTEG, FIELD>(
                         m, f, st, su2_to_spin_one(c64{1.0 + p.am1.re, p.am1.im}, p.beta), g, j0, j, j1);
                     break;
                 }
             }
-            su2_step64<EXPO>(m, p, g.a);
-            if constexpr (INTEG != INTEG_EULER) su2_step64<EXPO>(m, p, g.b);
+            su2_apply64(p, su2_step_element64(m, lie_trotter, g.a));
+            if constexpr (INTEG != INTEG_EULER) su2_apply64(p, su2_step_element64(m, lie_trotter, g.b));
         }
-        // Combine the lanes' partial products in step order: later steps multiply from the left.
-        if (D == 2 || !__any_sync(0xffffffffu, quadratic)) {
-            for (int s = 1; s < lanes; s <<= 1) {
-                const Su2d later = shfl_down_su2(p, s);
-                if ((lane_in_group & (2 * s - 1)) == 0) su2_apply64(p, later);
-            }
-            u = su2p_to_mat<D>(Su2p{c64{1.0 + p.am1.re, p.am1.im}, p.beta});
-        } else {
-            if (!quadratic) u = su2p_to_mat<D>(Su2p{c64{1.0 + p.am1.re, p.am1.im}, p.beta});
-            for (int s = 1; s < lanes; s <<= 1) {
-                const Mat<D> later = shfl_down_mat(u, s);
-                if ((lane_in_group & (2 * s - 1)) == 0) u = matmul(later, u);
-            }
-        }
+        finish_steps<DIMS>(m, dim, p, u, quadratic, lanes, lane_in_group, rw, dt_out, writes, t_c, index, time_out, u_out,
+                           product_out);
     }
-    if (!active || lane_in_group != 0) return;
-
-    if (m.rotating) {  // leave the rotating frame, I:839-852
-        c64 wo;
-        sincos(rw * dt_out, &wo.im, &wo.re);
-        const c64 woc = conj(wo);
-#pragma unroll
-        for (int k = 0; k < D; k++) {
-            u.a[0][k] = u.a[0][k] * woc;
-            u.a[D - 1][k] = u.a[D - 1][k] * wo;
-        }
-    }
-    time_out[index] = t_c;
-    double2* dst = reinterpret_cast<double2*>(u_out) + index * (D * D);
-#pragma unroll
-    for (int i = 0; i < D; i++)
-#pragma unroll
-        for (int k = 0; k < D; k++) dst[i * D + k] = make_double2(u.a[i][k].re, u.a[i][k].im);
 }
 
 }  // namespace spinsim

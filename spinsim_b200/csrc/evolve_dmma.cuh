@@ -34,7 +34,7 @@
 // against the field, theta = h (|B|max + w_max) <= kMagnusTheta, and CF4 otherwise.  The frame
 // transform, the sum and difference of the samples and the exponential's linear part stay in FP64;
 // the commutator and the exponential's O(|g|^2) remainder are FP32, the interval product FP64
-// (su2_apply_split).  On the benchmark's longest instances (theta = 0.07) the two compositions agree
+// (su2_split).  On the benchmark's longest instances (theta = 0.07) the two compositions agree
 // to 1e-11 in the final state.  Instances with more than kBulkTones
 // tones on a channel, or spin one with a quadratic shift, take the per-interval path (interval32,
 // CF4) inside the same kernel.
@@ -376,7 +376,7 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
                     rest.beta.re = fmaf(0.5f, cy, rest.beta.re);
                     rest.beta.im = fmaf(-0.5f, cx, rest.beta.im);
                     nsq = fmaf(gl[0], gl[0], fmaf(gl[1], gl[1], fmaf(gl[2], gl[2], nsq)));
-                    su2_apply_split(acc, gl64[0], gl64[1], gl64[2], rest);
+                    su2_apply64(acc, su2_split(gl64[0], gl64[1], gl64[2], rest));
                 } else {  // the reference's CF4 (I:655-686): two exponentials
                     double ga[3], gb[3];
 #pragma unroll
@@ -384,7 +384,7 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
                         ga[c] = fma(kW0, sa[c], kW1 * sb[c]);
                         gb[c] = fma(kW1, sa[c], kW0 * sb[c]);
                     }
-                    su2_cf4_step(acc, ga, gb, &nsq);
+                    su2_apply64(acc, su2_cf4_element(ga, gb, &nsq));
                 }
             }
             // the next step's samples, issued after this step's arithmetic (all lanes: mma.sync is
@@ -443,12 +443,9 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
 // registers do not weigh on the tensor path's step loop).
 template <int DIMS>
 __device__ __noinline__ void dmma_tile_fallback(const MethodConfig& m, const Instance& inst, const FieldDesc& f,
-                                                int64_t interval, int dim, double* time_out, double* u_out,
+                                                int64_t interval, bool active, double* time_out, double* u_out,
                                                 float* norms_out) {
-    if (DIMS != 3 && dim == 2)
-        interval32<2, INTEG_CF4, EXPO_ANALYTIC, FIELD_TONES>(m, inst, f, interval, true, 0, time_out, u_out, norms_out);
-    else if (DIMS != 2)
-        interval32<3, INTEG_CF4, EXPO_LIE_TROTTER, FIELD_TONES>(m, inst, f, interval, true, 0, time_out, u_out, norms_out);
+    interval32<DIMS, INTEG_CF4, FIELD_TONES>(m, inst, f, interval, active, 0, time_out, u_out, norms_out, nullptr);
 }
 
 // Persistent launch: CTAs pull tiles of kDmmaTile intervals from the queue (or, without a queue, CTA
@@ -497,8 +494,9 @@ SS_D void evolve_dmma_body(const EvolveArgs& a, DmmaShared& sh) {
             const DmmaConsts* cst = a.dmma_consts != nullptr ? a.dmma_consts + tile.instance : nullptr;
             double* rows_out = a.rows != nullptr ? a.rows + 4 * inst.out_offset : nullptr;
             tile_dmma<DIMS>(a.m, inst, f, tile, sh, time_out, u_out, norms_out, partial_out, cst, rows_out);
-        } else if (threadIdx.x < tile.count) {
-            dmma_tile_fallback<DIMS>(a.m, inst, f, tile.first + threadIdx.x, dim, time_out, u_out, norms_out);
+        } else if (threadIdx.x < kDmmaTile) {  // one warp
+            const bool active = (int)threadIdx.x < tile.count;
+            dmma_tile_fallback<DIMS>(a.m, inst, f, tile.first + (active ? threadIdx.x : 0), active, time_out, u_out, norms_out);
         }
         __syncthreads();  // shared memory and the tile slot are reused by the next tile
         if (a.tile_counter == nullptr) return;

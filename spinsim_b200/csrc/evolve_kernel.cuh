@@ -41,12 +41,17 @@ SS_D void evolve_body(const EvolveArgs& a) {
         }
     }
     const int64_t warp_global = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     int64_t tile_id = warp_global;
+    int reserved = -1;  // lane 0: the warp's next tile
     for (;;) {
         if (a.tile_counter != nullptr) {
             int t = 0;
-            if (lane == 0) t = atomicAdd(a.tile_counter, 1);
+            if (lane == 0) t = reserved >= 0 ? reserved : atomicAdd(a.tile_counter, 1);
             tile_id = __shfl_sync(0xffffffffu, t, 0);
+            // Away from the end of the queue the next tile is taken now: its atomic's latency passes during
+            // this tile.
+            if (lane == 0) reserved = tile_id + 2 * warps < a.n_tiles ? atomicAdd(a.tile_counter, 1) : -1;
         }
         if (tile_id >= a.n_tiles) return;
         Tile tile;
@@ -72,7 +77,7 @@ SS_D void evolve_body(const EvolveArgs& a) {
                 for (int i = 0; i < kSynthIntervals; i++) {
                     const bool act = lane + 32 * i < tile.count;
                     const int64_t idx = tile.first + (act ? lane + 32 * i : 0);
-                    interval32<3, INTEG, EXPO_O, FIELD>(a.m, inst, f, idx, act, 0, time_out, u_out, norms_out);
+                    interval32<3, INTEG, FIELD>(a.m, inst, f, idx, act, 0, time_out, u_out, norms_out, nullptr);
                 }
             } else if (DIMS != 3 && dim == 2) {
                 intervals32_synth<2, EXPO_H>(a.m, inst, f, tile, time_out, u_out, norms_out);
@@ -80,19 +85,19 @@ SS_D void evolve_body(const EvolveArgs& a) {
                 intervals32_synth<3, EXPO_O>(a.m, inst, f, tile, time_out, u_out, norms_out);
             }
         } else {
+            // one lane per interval: the warp's tile is a tile of the state scan, whose product it writes
+            double* product_out = nullptr;
+            if (a.tile_products != nullptr)
+                product_out = a.tile_products + ((a.scan_begin != nullptr ? a.scan_begin[tile.instance] : 0) +
+                                                 tile.first / kScanTile) * kScanMat;
             const bool active = group < tile.count;
             const int64_t index = tile.first + (active ? group : 0);
-            if (DIMS != 3 && dim == 2) {
-                if constexpr (PREC == PREC_FP64)
-                    interval64<2, INTEG, EXPO_H, FIELD>(a.m, inst, f, index, active, lane_in_group, time_out, u_out);
-                else
-                    interval32<2, INTEG, EXPO_H, FIELD>(a.m, inst, f, index, active, lane_in_group, time_out, u_out, norms_out);
-            } else if (DIMS != 2) {
-                if constexpr (PREC == PREC_FP64)
-                    interval64<3, INTEG, EXPO_O, FIELD>(a.m, inst, f, index, active, lane_in_group, time_out, u_out);
-                else
-                    interval32<3, INTEG, EXPO_O, FIELD>(a.m, inst, f, index, active, lane_in_group, time_out, u_out, norms_out);
-            }
+            if constexpr (PREC == PREC_FP64)
+                interval64<DIMS, INTEG, EXPO_H, EXPO_O, FIELD>(a.m, inst, f, index, active, lane_in_group, time_out,
+                                                               u_out, product_out);
+            else
+                interval32<DIMS, INTEG, FIELD>(a.m, inst, f, index, active, lane_in_group, time_out, u_out, norms_out,
+                                               product_out);
         }
         if (a.tile_counter == nullptr) return;
     }

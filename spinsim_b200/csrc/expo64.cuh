@@ -80,7 +80,7 @@ SS_D Su2d su2_exp_m1(double x, double y, double z, double r2) {
 // N-th power, N = 4^h, of e^{-i z Jz / 2N} e^{-i (x Jx + y Jy) / N} e^{-i z Jz / 2N}, minus one.  The
 // factor is an SU(2) rotation by 2 theta, cos theta = cos A cos Z and sin theta (axis) =
 // (sin A, cos A sin Z) with A = a / 2N, Z = z / 2N, so its N-th power is the rotation by 2 N theta.
-// Out of line: the steps that need it are those too large for their N (su2_step64).
+// Out of line: the steps that need it are those too large for their N (su2_step_element64).
 inline __device__ __noinline__ Su2d su2_lie_trotter_m1(double x, double y, double z, double n) {
     const double a = sqrt(x * x + y * y);
     c64 ep = c64{1.0, 0.0};
@@ -130,17 +130,25 @@ SS_D Su2d shfl_down_su2(const Su2d& v, int delta) {
     return o;
 }
 
-// One exponential of a step's generator, applied to the interval's product.  A Lie-Trotter
+// p <- (1 + e)^n p by binary powers.
+SS_D void su2_apply_power64(Su2d& p, Su2d e, int n) {
+    for (;;) {
+        if (n & 1) su2_apply64(p, e);
+        n >>= 1;
+        if (n == 0) return;
+        const Su2d once = e;
+        su2_apply64(e, once);
+    }
+}
+
+// One exponential of a step's generator, minus one.  A Lie-Trotter
 // exponential of N = 4^h factors differs from the exponential by less than |g|^3 / (8 N^2) (symmetric
 // splitting), so for |g|^2 <= lt_norm2_max (|g|^3 <= 2^-53 N^2, |g| = 0.31 at the default 24
 // squarings) the exponential itself is taken, and the N-th power's closed form beyond.
-template <int EXPO>
-SS_D void su2_step64(const MethodConfig& m, Su2d& p, const double* g) {
+SS_D Su2d su2_step_element64(const MethodConfig& m, bool lie_trotter, const double* g) {
     const double r2 = fma(g[0], g[0], fma(g[1], g[1], g[2] * g[2]));
-    Su2d e;
-    if (EXPO == EXPO_ANALYTIC || r2 <= m.lt_norm2_max) e = su2_exp_m1(g[0], g[1], g[2], r2);
-    else e = su2_lie_trotter_m1(g[0], g[1], g[2], m.precision);
-    su2_apply64(p, e);
+    if (!lie_trotter || r2 <= m.lt_norm2_max) return su2_exp_m1(g[0], g[1], g[2], r2);
+    return su2_lie_trotter_m1(g[0], g[1], g[2], m.precision);
 }
 
 // ------------------------------------------------------------------ spin one
@@ -290,7 +298,7 @@ inline __device__ __noinline__ Mat<3> spin_one_squarings_step64(Mat<3> u, double
 }
 
 // One exponential of a spin-one step with a quadratic shift (I:1768-1808), applied to the interval's
-// product u.  As in su2_step64, the exponential itself where the Lie-Trotter product agrees with it to
+// product u.  As in su2_step_element64, the exponential itself where the Lie-Trotter product agrees with it to
 // rounding (|g|^2 <= lt_norm2_max; the reversed sign of the shift in the factor's [0][2] phase is
 // of the same order as the splitting's error, a^2 q / (6 N^2)), else the reference's squarings.
 SS_D void spin_one_step64(const MethodConfig& m, Mat<3>& u, const double* g) {
