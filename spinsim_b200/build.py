@@ -86,8 +86,9 @@ MINB = (2, 3, 4)
 # Tighter budgets (96 and 80 registers) for the FP32-bulk tabulated-field kernels, the serving path,
 # whose latency-bound table lookups gain from residency more than they lose to spills.
 MINB_TIGHT = (5, 6)
-# Register budgets of the tensor-path tone kernels (128-thread CTAs): 5 -> 102, 4 -> 128, 3 -> 168 registers.
-DMMA_MINB = (3, 4, 5, 6)
+# Register budgets of the tensor-path tone kernels (128-thread CTAs) by precision: 6 -> 80, 5 -> 96, 4 -> 128,
+# 3 -> 168 registers.
+DMMA_MINB = {1: (3, 4, 5, 6), 0: (3, 4, 5)}
 
 
 def user_minb(v):
@@ -127,21 +128,20 @@ def gen_sources():
         reg_decl.append(f'extern "C" const unsigned char spinsim_blob_{name}_begin[], spinsim_blob_{name}_end[];')
         user_rows.append(f"    {{{v[0]}, {v[1]}, {v[2]}, {v[3]}, {v[4]}, spinsim_blob_{name}_begin, "
                          f"spinsim_blob_{name}_end}},")
-    # FP32-bulk tone kernels with the field samples on the FP64 tensor path (one per spin mix and
+    # Magnus CF4 tone kernels with the field samples on the FP64 tensor path (one per spin mix, precision and
     # register budget; the exponentiators do not enter them).
     dmma_rows = []
-    for dims in (0, 2, 3):
-        for minb in DMMA_MINB:
-            name = f"dmma_d{dims}_b{minb}"
-            src = os.path.join(GEN, f"k_{name}.cu")
-            body = (f'#include "evolve_dmma.cuh"\n'
-                    f"namespace spinsim {{\ntemplate __global__ void evolve_dmma_kernel<{dims}, {minb}>(EvolveArgs);\n}}\n"
-                    f'extern "C" const void* spinsim_kget_{name}(void) {{\n'
-                    f"    return (const void*)&spinsim::evolve_dmma_kernel<{dims}, {minb}>;\n}}\n")
-            write_if_changed(src, body)
-            units.append(("sass", name, src))
-            reg_decl.append(f'extern "C" const void* spinsim_kget_{name}(void);')
-            dmma_rows.append(f"    {{{dims}, {minb}, spinsim_kget_{name}}},")
+    for dims, prec, minb in ((d, p, b) for d in (0, 2, 3) for p in (1, 0) for b in DMMA_MINB[p]):
+        name = f"dmma_d{dims}_{PREC[prec]}_b{minb}"
+        src = os.path.join(GEN, f"k_{name}.cu")
+        body = (f'#include "evolve_dmma.cuh"\n'
+                f"namespace spinsim {{\ntemplate __global__ void evolve_dmma_kernel<{dims}, {prec}, {minb}>(EvolveArgs);\n}}\n"
+                f'extern "C" const void* spinsim_kget_{name}(void) {{\n'
+                f"    return (const void*)&spinsim::evolve_dmma_kernel<{dims}, {prec}, {minb}>;\n}}\n")
+        write_if_changed(src, body)
+        units.append(("sass", name, src))
+        reg_decl.append(f'extern "C" const void* spinsim_kget_{name}(void);')
+        dmma_rows.append(f"    {{{dims}, {prec}, {minb}, spinsim_kget_{name}}},")
     # the tensor path's per-instance constants (one small launch before the time evolution)
     src = os.path.join(GEN, "k_dmma_consts.cu")
     write_if_changed(src, '#define SPINSIM_DMMA_CONSTS_KERNEL 1\n#include "evolve_dmma.cuh"\n'

@@ -64,7 +64,7 @@ struct UserEntry {
     const unsigned char* end;
 };
 struct DmmaEntry {
-    int dims, minb;
+    int dims, prec, minb;
     kernel_getter get;
 };
 // Generated by the build: declares the getters/blobs and defines kBuiltin[], kUser[].
@@ -175,6 +175,7 @@ struct spinsim_plan {
     bool lockstep = false;  // kernel needs one lane per output interval (tone synthesis)
     int intervals_per_lane = 1;
     bool cta_tiles = false;  // a tile is a CTA's unit of work (the tensor-path tone kernel), not a warp's
+    spinsim_plan* tensor = nullptr;  // FP64 Magnus CF4 tone plans: the tensor-path form, for the fields it takes
 };
 
 // Output intervals in one tile of the plan's time-evolution kernel.
@@ -182,10 +183,10 @@ static int tile_intervals(const spinsim_plan* p, int lanes) {
     return p->cta_tiles ? kDmmaTile : 32 * p->intervals_per_lane / lanes;
 }
 
-// The plan's warps take 32 consecutive output intervals, one per lane: a tile of the state scan, whose product
-// they write.
-static bool warps_write_products(const spinsim_plan* p, int lanes) {
-    return !p->cta_tiles && !p->lockstep && lanes == 1;
+// The plan's warps (one lane per output interval) or CTAs (FP64 tensor path) take 32 consecutive output
+// intervals: a tile of the state scan, whose product they write.
+static bool writes_products(const spinsim_plan* p, int lanes) {
+    return p->cta_tiles ? p->desc.precision == SPINSIM_PRECISION_FP64 : !p->lockstep && lanes == 1;
 }
 
 extern "C" const char* spinsim_version(void) { return "spinsim_b200 0.1.0 (sm_100a)"; }
@@ -217,6 +218,46 @@ extern "C" int spinsim_normalise_steps(double t0, double t1, double dt_int, doub
 static bool valid_expo(int dim, int e) {
     if (dim == 2) return e == EXPO_ANALYTIC || e == EXPO_LIE_TROTTER;
     return e == EXPO_LIE_TROTTER || e == EXPO_LIE_TROTTER_8;
+}
+
+// Make p a tensor-path tone plan (Magnus CF4).  Register budgets: 128 registers (4 CTAs per SM) by default;
+// budgets of at most 85 registers take the 6-CTA build (80 registers), at most 102 the 5-CTA build (96), above
+// 128 the 168-register build.
+static void take_tensor_path(spinsim_plan* p) {
+    const int mr = p->desc.max_registers;
+    const int want_minb = (mr > 0 && mr <= 85) ? 6 : (mr > 0 && mr <= 102) ? 5 : (mr == 0 || mr <= 128) ? 4 : 3;
+    p->func = nullptr;
+    for (int minb = want_minb; minb >= 3 && !p->func; minb--)
+        for (const DmmaEntry& k : kDmma)
+            if (k.dims == p->desc.spin_dim && k.prec == p->desc.precision && k.minb == minb) {
+                p->func = k.get();
+                break;
+            }
+    p->block = kDmmaThreads;
+    p->cta_tiles = true;
+    p->lockstep = true;
+    p->m.lanes = 1;
+}
+
+// The kernel's attributes and resident CTAs.
+static cudaError_t query_kernel(spinsim_plan* p) {
+    cudaFuncAttributes attr;
+    cudaError_t e = cudaFuncGetAttributes(&attr, p->func);
+    if (e == cudaSuccess && p->smem_per_warp) {
+        e = cudaFuncSetAttribute(p->func, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kEvolveThreadsMax / 32 * p->smem_per_warp);
+        // prefer the largest shared-memory carve-out so that shared memory does not cap residency
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(p->func, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                     (int)cudaSharedmemCarveoutMaxShared);
+    }
+    if (e != cudaSuccess) return e;
+    p->regs = attr.numRegs;
+    if (p->block > attr.maxThreadsPerBlock) p->block = attr.maxThreadsPerBlock / 32 * 32;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p->blocks_per_sm, p->func, p->block,
+                                                      (size_t)(p->block / 32) * p->smem_per_warp);
+    if (p->blocks_per_sm < 1) p->blocks_per_sm = 1;
+    return e;
 }
 
 extern "C" int spinsim_plan_create(const spinsim_plan_desc* desc, const void* field_ltoir, size_t field_ltoir_size,
@@ -271,21 +312,7 @@ extern "C" int spinsim_plan_create(const spinsim_plan_desc* desc, const void* fi
     const bool dmma = d.field_kind == SPINSIM_FIELD_TONES && d.precision == SPINSIM_PRECISION_FP32_BULK &&
                       d.integration == SPINSIM_INTEGRATION_MAGNUS_CF4 && d.variant == SPINSIM_VARIANT_TENSOR;
     if (dmma) {
-        // Tensor-path tone kernel: 128 registers (4 CTAs per SM) by default; budgets of at most 85
-        // registers take the 6-CTA build (80 registers), at most 102 the 5-CTA build (96), above 128
-        // the 168-register build.
-        const int mr = d.max_registers;
-        const int want_minb = (mr > 0 && mr <= 85) ? 6 : (mr > 0 && mr <= 102) ? 5 : (mr == 0 || mr <= 128) ? 4 : 3;
-        for (int minb = want_minb; minb >= 3 && !p->func; minb--)
-            for (const DmmaEntry& k : kDmma)
-                if (k.dims == d.spin_dim && k.minb == minb) {
-                    p->func = k.get();
-                    break;
-                }
-        p->block = kDmmaThreads;
-        p->cta_tiles = true;
-        p->lockstep = true;
-        p->m.lanes = 1;
+        take_tensor_path(p);
     } else if (d.field_kind != SPINSIM_FIELD_USER) {
         // Register budget: the kernel built for MINB resident 128-thread CTAs per SM whose cap is the
         // largest that fits max_registers: 6 -> 80, 5 -> 96, 4 -> 128, 3 -> 168 registers, 2 uncapped.
@@ -341,28 +368,19 @@ extern "C" int spinsim_plan_create(const spinsim_plan_desc* desc, const void* fi
         p->intervals_per_lane = kSynthIntervals;
         p->m.lanes = 1;
     }
-    cudaFuncAttributes attr;
-    e = cudaFuncGetAttributes(&attr, p->func);
-    if (e == cudaSuccess && p->smem_per_warp) {
-        e = cudaFuncSetAttribute(p->func, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kEvolveThreadsMax / 32 * p->smem_per_warp);
-        // prefer the largest shared-memory carve-out so that shared memory does not cap residency
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(p->func, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     (int)cudaSharedmemCarveoutMaxShared);
-    }
-    if (e == cudaSuccess) {
-        p->regs = attr.numRegs;
-        if (p->block > attr.maxThreadsPerBlock) p->block = attr.maxThreadsPerBlock / 32 * 32;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p->blocks_per_sm, p->func, p->block,
-                                                          (size_t)(p->block / 32) * p->smem_per_warp);
+    e = query_kernel(p);
+    if (e == cudaSuccess && d.field_kind == SPINSIM_FIELD_TONES && d.precision == SPINSIM_PRECISION_FP64 &&
+        d.integration == SPINSIM_INTEGRATION_MAGNUS_CF4 && eo != EXPO_LIE_TROTTER_8) {
+        p->tensor = new spinsim_plan(*p);
+        take_tensor_path(p->tensor);
+        e = query_kernel(p->tensor);
     }
     if (e != cudaSuccess) {
         if (p->lib) cudaLibraryUnload(p->lib);
+        delete p->tensor;
         delete p;
         return fail(SPINSIM_ERR_CUDA, "querying the kernel failed: %s", cudaGetErrorString(e));
     }
-    if (p->blocks_per_sm < 1) p->blocks_per_sm = 1;
     *out = p;
     return SPINSIM_OK;
 }
@@ -370,12 +388,14 @@ extern "C" int spinsim_plan_create(const spinsim_plan_desc* desc, const void* fi
 extern "C" int spinsim_plan_destroy(spinsim_plan* plan) {
     if (!plan) return SPINSIM_OK;
     if (plan->lib) cudaLibraryUnload(plan->lib);
+    delete plan->tensor;
     delete plan;
     return SPINSIM_OK;
 }
 
 extern "C" int spinsim_plan_get_info(const spinsim_plan* plan, spinsim_plan_info* info) {
     if (!plan || !info) return fail(SPINSIM_ERR_INVALID, "null argument");
+    if (plan->tensor) plan = plan->tensor;  // the kernel of nearly every tone field
     info->registers_per_thread = plan->regs;
     info->threads_per_block = plan->block;
     info->blocks_per_sm = plan->blocks_per_sm;
@@ -795,7 +815,8 @@ static size_t single_workspace(int64_t n_out, bool with_scan, bool with_rows = f
 
 extern "C" size_t spinsim_evaluate_workspace_size(const spinsim_plan* plan, int64_t n_out) {
     if (!plan || n_out < 0 || plan->desc.spin_dim == 0) return 0;
-    return single_workspace(n_out, true, plan->cta_tiles, plan->cta_tiles);  // the tensor path's SU(2) rows for the scan
+    // the tensor path's SU(2) rows for the scan (FP32-bulk), its descriptors and constants
+    return single_workspace(n_out, true, plan->cta_tiles, plan->cta_tiles || plan->tensor);
 }
 
 static int evaluate_impl(const spinsim_plan* p, const spinsim_field* field, double t0, double dt_int, double dt_out,
@@ -808,11 +829,13 @@ static int evaluate_impl(const spinsim_plan* p, const spinsim_field* field, doub
     Instance inst;
     rc = make_instance(p, t0, dt_int, dt_out, n_out, psi0, &inst);
     if (rc) return rc;
+    if (p->tensor && tones_on_tensor_path(*reinterpret_cast<const FieldDesc*>(field), inst.dim)) p = p->tensor;
     if (n_out == 0) return SPINSIM_OK;
     if (!time || !u || (with_scan && !state)) return fail(SPINSIM_ERR_INVALID, "output pointer is null");
     if (with_scan && !psi0) return fail(SPINSIM_ERR_INVALID, "psi0 is null");
     if (!ws || ((uintptr_t)ws & 255)) return fail(SPINSIM_ERR_WORKSPACE, "workspace must be non-null and 256-byte aligned");
-    const bool with_rows = with_scan && p->cta_tiles;
+    const bool bulk = p->desc.precision == SPINSIM_PRECISION_FP32_BULK;
+    const bool with_rows = with_scan && p->cta_tiles && bulk;
     const size_t need = single_workspace(n_out, with_scan, with_rows, p->cta_tiles);
     if (ws_bytes < need) return fail(SPINSIM_ERR_WORKSPACE, "workspace of %zu bytes is below the %zu needed", ws_bytes, need);
 
@@ -837,14 +860,14 @@ static int evaluate_impl(const spinsim_plan* p, const spinsim_field* field, doub
     a.tile_counter = nullptr;
     a.time = time;
     a.u = u;
-    a.step_norms = p->desc.precision == SPINSIM_PRECISION_FP32_BULK ? norms : nullptr;
+    a.step_norms = bulk ? norms : nullptr;
     // the tensor path writes the scan's tile partials as it goes (its CTA tiles are the scan tiles)
-    const bool partials = with_scan && p->cta_tiles && n_out > kScanShort &&
+    const bool partials = with_scan && p->cta_tiles && bulk && n_out > kScanShort &&
                           tones_on_tensor_path(*reinterpret_cast<const FieldDesc*>(field), inst.dim);
     a.tile_partials = partials ? b.tile_product : nullptr;
     a.scan_begin = nullptr;
     a.rows = partials ? rows : nullptr;
-    const bool products = with_scan && warps_write_products(p, a.m.lanes) && n_out > kScanShort;
+    const bool products = with_scan && writes_products(p, a.m.lanes) && n_out > kScanShort;
     a.tile_products = products ? b.tile_product : nullptr;
     if (p->cta_tiles) {
         Instance* inst_dev = c.take<Instance>(1);
@@ -1013,7 +1036,9 @@ struct spinsim_batch {
     FieldDesc* fields_dev;
     Tile* tiles_dev;
     int64_t n_tiles;
-    int32_t* counter;
+    Tile* tensor_tiles_dev = nullptr;  // FP64 tones: the tiles of the instances whose field the tensor path takes
+    int64_t n_tensor_tiles = 0;        // (a launch of its own; an instance's route depends on its field alone)
+    int32_t* counter;                  // [2]: the two queues
     int lanes;
     float* step_norms = nullptr;  // FP32-bulk: per output step, the sum of |g|^2 over its fine steps
     ScanBuffers scan;  // every instance's scan tiles (both spins)
@@ -1025,7 +1050,9 @@ struct spinsim_batch {
 // The time evolution's tiles, ordered longest-first so that the long instances start early.  An
 // instance's full tiles share one cost, so the (stable) order is found by sorting runs: each
 // instance's full tiles as one run, its partial last tile as another.
-static void fill_evolve_tiles(const spinsim_plan* p, const Instance* inst, int32_t n, int per_warp, Tile* out) {
+// Only instances with tensor[i] == on (null: all).  Returns the number of tiles.
+static int64_t fill_evolve_tiles(const spinsim_plan* p, const Instance* inst, int32_t n, int per_warp,
+                                 const std::vector<char>* tensor, char on, Tile* out) {
     struct Run {
         double cost;
         int32_t instance;
@@ -1036,6 +1063,7 @@ static void fill_evolve_tiles(const spinsim_plan* p, const Instance* inst, int32
     std::vector<Run> runs;
     runs.reserve(2 * (size_t)n);
     for (int i = 0; i < n; i++) {
+        if (tensor && (*tensor)[i] != on) continue;
         // a spin-one step costs about a spin-half one (SU(2) elements), more with a quadratic shift, and
         // its squarings with the eight-generator exponential
         const double step_cost =
@@ -1054,6 +1082,7 @@ static void fill_evolve_tiles(const spinsim_plan* p, const Instance* inst, int32
             t.count = r.count;
         }
     }
+    return at;
 }
 
 // Sizes and carves a batch's workspace (ws null: sizes only).  The tiles are written by
@@ -1075,7 +1104,11 @@ static int batch_layout(const spinsim_plan* p, const spinsim_instance* instances
     const int lanes = pick_lanes(p, total, max_fine);
     const int per_warp = tile_intervals(p, lanes);
     int64_t n_tiles = 0;
-    for (int i = 0; i < n; i++) n_tiles += (inst[i].n_out + per_warp - 1) / per_warp;
+    int64_t n_tensor_tiles = 0;
+    for (int i = 0; i < n; i++) {
+        n_tiles += (inst[i].n_out + per_warp - 1) / per_warp;
+        if (p->tensor) n_tensor_tiles += (inst[i].n_out + kDmmaTile - 1) / kDmmaTile;
+    }
     count_scan_plan(inst, n, sp);
 
     // Workspace: every descriptor first (one block that a staged prepare uploads with one copy),
@@ -1084,15 +1117,17 @@ static int batch_layout(const spinsim_plan* p, const spinsim_instance* instances
     b->inst_dev = c.take<Instance>(std::max(1, n));
     b->fields_dev = c.take<FieldDesc>(std::max(1, n_fields));
     b->tiles_dev = c.take<Tile>(std::max<int64_t>(1, n_tiles));
+    if (p->tensor) b->tensor_tiles_dev = c.take<Tile>(std::max<int64_t>(1, n_tensor_tiles));
     carve_scan_desc(c, *sp, &b->scan);
     if (desc_bytes) *desc_bytes = c.used;
-    b->counter = c.take<int32_t>(1);
+    b->counter = c.take<int32_t>(2);
     carve_scan_scratch(c, b->scan.n_tiles, &b->scan);
+    if (p->cta_tiles || p->tensor) b->consts = c.take<DmmaConsts>(std::max(1, n));
     if (p->cta_tiles) {
-        b->consts = c.take<DmmaConsts>(std::max(1, n));
         b->rows = c.take<double>(4 * (size_t)std::max<int64_t>(1, total));
     }
     b->n_tiles = n_tiles;
+    b->n_tensor_tiles = n_tensor_tiles;
     b->plan = p;
     b->lanes = lanes;
     *used = c.used + 256;
@@ -1282,31 +1317,44 @@ static int batch_prepare(const spinsim_plan* plan, const spinsim_instance* insta
         // The tile lists: written in place in the staging image, else built here and uploaded.
         const Instance* inst = reinterpret_cast<const Instance*>(instances);
         const int per_warp = tile_intervals(plan, b->lanes);
-        std::vector<Tile> evolve_tiles, scan_tiles;
+        std::vector<char> on_path;  // FP64 tones: which instances the tensor path takes
+        if (plan->tensor)
+            for (int i = 0; i < n_instances; i++)
+                on_path.push_back(tones_on_tensor_path(reinterpret_cast<const FieldDesc*>(fields)[inst[i].field], inst[i].dim));
+        std::vector<Tile> evolve_tiles, tensor_tiles, scan_tiles;
         std::vector<int32_t> begin, end;
-        Tile *et, *stl;
+        Tile *et, *tt, *stl;
         int32_t *bg, *en;
         if (st) {
             et = reinterpret_cast<Tile*>(st + ((char*)b->tiles_dev - (char*)ws));
+            tt = plan->tensor ? reinterpret_cast<Tile*>(st + ((char*)b->tensor_tiles_dev - (char*)ws)) : nullptr;
             stl = reinterpret_cast<Tile*>(st + ((char*)b->scan.tiles - (char*)ws));
             bg = reinterpret_cast<int32_t*>(st + ((char*)b->scan.begin - (char*)ws));
             en = reinterpret_cast<int32_t*>(st + ((char*)b->scan.end - (char*)ws));
         } else {
             evolve_tiles.resize((size_t)b->n_tiles);
+            tensor_tiles.resize((size_t)b->n_tensor_tiles);
             scan_tiles.resize((size_t)sp.n_tiles);
             begin.resize((size_t)n_instances);
             end.resize((size_t)n_instances);
             et = evolve_tiles.data();
+            tt = tensor_tiles.data();
             stl = scan_tiles.data();
             bg = begin.data();
             en = end.data();
         }
-        fill_evolve_tiles(plan, inst, n_instances, per_warp, et);
+        if (plan->tensor) {
+            b->n_tensor_tiles = fill_evolve_tiles(plan->tensor, inst, n_instances, kDmmaTile, &on_path, 1, tt);
+            b->n_tiles = fill_evolve_tiles(plan, inst, n_instances, per_warp, &on_path, 0, et);
+        } else {
+            fill_evolve_tiles(plan, inst, n_instances, per_warp, nullptr, 0, et);
+        }
         fill_scan_plan(inst, n_instances, stl, bg, en);
         if (st) {
             rc = upload(ws, st, desc, s);
         } else {
             rc = upload(b->tiles_dev, et, sizeof(Tile) * (size_t)b->n_tiles, s);
+            if (!rc) rc = upload(b->tensor_tiles_dev, tt, sizeof(Tile) * (size_t)b->n_tensor_tiles, s);
             if (!rc) rc = upload(b->scan.tiles, stl, sizeof(Tile) * (size_t)sp.n_tiles, s);
             if (!rc) rc = upload(b->scan.begin, bg, sizeof(int32_t) * (size_t)n_instances, s);
             if (!rc) rc = upload(b->scan.end, en, sizeof(int32_t) * (size_t)n_instances, s);
@@ -1347,33 +1395,40 @@ extern "C" int spinsim_batch_prepare_staged(const spinsim_plan* plan, const spin
 extern "C" int spinsim_batch_launch(const spinsim_batch* b, double* time_dev, double* u_dev, double* state_dev,
                                     double* spin_dev, void* stream) {
     if (!b) return fail(SPINSIM_ERR_INVALID, "batch is null");
-    if (b->n_tiles == 0) return SPINSIM_OK;
+    if (b->n_tiles + b->n_tensor_tiles == 0) return SPINSIM_OK;
     if (!time_dev || !u_dev) return fail(SPINSIM_ERR_INVALID, "output pointer is null");
     cudaStream_t s = (cudaStream_t)stream;
     const spinsim_plan* p = b->plan;
-    CUDA_TRY(cudaMemsetAsync(b->counter, 0, sizeof(int32_t), s));
+    CUDA_TRY(cudaMemsetAsync(b->counter, 0, 2 * sizeof(int32_t), s));
     EvolveArgs a;
     memset(&a, 0, sizeof(a));
-    a.m = p->m;
-    a.m.lanes = b->lanes;
     a.instances = b->inst_dev;
     a.fields = b->fields_dev;
-    a.tiles = b->tiles_dev;
-    a.n_tiles = b->n_tiles;
-    a.tile_counter = b->counter;
     a.time = time_dev;
     a.u = u_dev;
     a.step_norms = p->desc.precision == SPINSIM_PRECISION_FP32_BULK ? b->step_norms : nullptr;
     a.tile_partials = b->partials ? b->scan.tile_product : nullptr;  // the same kernel work with or without the scan
     a.rows = b->partials ? b->rows : nullptr;
-    const bool products = warps_write_products(p, b->lanes);
+    // the scan's tile products, when every launch of the time evolution writes its own
+    const bool products = (b->n_tensor_tiles == 0 || writes_products(p->tensor, 1)) &&
+                          (b->n_tiles == 0 || writes_products(p, b->lanes));
     a.tile_products = products ? b->scan.tile_product : nullptr;
     a.scan_begin = b->scan.begin;
-    if (b->consts != nullptr && b->scan.n_instances > 0) {  // the tensor path's per-instance constants first
+    if (b->consts != nullptr && b->scan.n_instances > 0 && (p->cta_tiles || b->n_tensor_tiles > 0)) {
         int rc = launch_dmma_consts(&a, b->consts, b->scan.n_instances, nullptr, nullptr, s);
         if (rc) return rc;
     }
-    int rc = launch_evolve(p, a, b->n_tiles, s, a.dmma_consts != nullptr);
+    auto evolve = [&](const spinsim_plan* q, int lanes, const Tile* tiles, int64_t n_tiles, int32_t* counter) {
+        if (n_tiles == 0) return (int)SPINSIM_OK;
+        a.m = q->m;
+        a.m.lanes = lanes;
+        a.tiles = tiles;
+        a.n_tiles = n_tiles;
+        a.tile_counter = counter;
+        return launch_evolve(q, a, n_tiles, s, q->cta_tiles);  // early behind the tensor path's constants
+    };
+    int rc = evolve(p->tensor, 1, b->tensor_tiles_dev, b->n_tensor_tiles, b->counter + 1);
+    if (!rc) rc = evolve(p, b->lanes, b->tiles_dev, b->n_tiles, b->counter);
     if (rc || !state_dev) return rc;
     rc = launch_scan(b->inst_dev, nullptr, b->scan, u_dev, state_dev, spin_dev, s, SCAN_ALL, nullptr, b->partials, a.rows,
                      products);
@@ -1388,10 +1443,11 @@ extern "C" int spinsim_batch_set_step_norms(spinsim_batch* b, float* step_norms_
 
 extern "C" int spinsim_batch_get_info(const spinsim_batch* b, spinsim_batch_info* info) {
     if (!b || !info) return fail(SPINSIM_ERR_INVALID, "null argument");
-    info->tiles = b->n_tiles;
+    info->tiles = b->n_tiles + b->n_tensor_tiles;
     info->scan_tiles = b->scan.n_tiles;
-    info->lanes = b->lanes;
-    info->tile_intervals = tile_intervals(b->plan, b->lanes);
+    const bool tensor_only = b->n_tiles == 0 && b->n_tensor_tiles > 0;
+    info->lanes = tensor_only ? 1 : b->lanes;
+    info->tile_intervals = tensor_only ? kDmmaTile : tile_intervals(b->plan, b->lanes);
     info->scan_partials = b->partials ? 1 : 0;
     info->reserved = 0;
     return SPINSIM_OK;

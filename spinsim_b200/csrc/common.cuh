@@ -133,14 +133,15 @@ constexpr int kBulkTones = 8;               // tones per channel (x, y, z) synth
 constexpr int kToneSlots = 3 * kBulkTones;  // slot = channel * kBulkTones + tone
 
 // Per-instance constants of the tensor-path kernel (evolve_dmma.cuh), the same for all of an
-// instance's tiles: the phasor table's start values exp(i w tau) of every (channel, tone, time
-// segment, Gauss point), each tone's step rotation exp(i w dt) and half-interval phasor
-// exp(i w dt_out / 2), and the choice of step (1: Magnus).
+// instance's tiles: the phasor table's start values exp(i w delta) of every (channel, tone, time
+// segment, Gauss point), each tone's step rotation exp(i w dt), half-interval phasor
+// exp(i w dt_out / 2) and phasor of the middle step's samples, and the choice of step (1: Magnus).
 constexpr int kDmmaRecurrences = 3 * kBulkTones * 4 * 2;
 struct __align__(16) DmmaConsts {
     double2 z[kDmmaRecurrences];
     double2 rot[kToneSlots];
     double2 half_step[kToneSlots];
+    double2 middle[kToneSlots];
     int32_t magnus;
     int32_t pad[3];
 };

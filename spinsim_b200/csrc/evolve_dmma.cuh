@@ -1,33 +1,36 @@
-// FP32-bulk time evolution of tone fields with the field samples formed on the FP64 tensor path.
+// Time evolution of tone fields (Magnus CF4) with the field samples formed on the FP64 tensor path, in FP32-bulk
+// and in FP64.
 //
 // The reference samples its field once per Gauss point of every fine step of every output interval
-// (get_field_integration_magnus_cf4, spinsim/__init__.py:624-652).  For a tone field
-//     B_c(t_c + tau) = bias_c + sum_k A_k sin(w_k (t_c + tau) + phi_k)
-//                    = bias_c + sum_k [Re L_ck sin(w_k tau) + Im L_ck cos(w_k tau)],  L_ck = A_k exp(i (w_k t_c + phi_k)),
-// so the samples of a block of output intervals (rows, through L) at a block of sample offsets tau
-// (columns, through sin / cos) are a matrix product with inner dimension 2 x (tones per channel).
-// That product runs as mma.sync.m8n8k4.f64 (FP64 in, FP64 accumulate: the samples are exact to FP64
-// rounding), which takes eight multiply-adds per lane per instruction instead of one.
+// (get_field_integration_magnus_cf4, spinsim/__init__.py:624-652).  For a tone field, at distances +-delta from
+// the middle t_m of an interval,
+//     B_c(t_m +- delta) = bias_c + sum_k Im(L_ck) cos(w_k delta) +- sum_k Re(L_ck) sin(w_k delta),
+//     L_ck = A_k exp(i (w_k t_m + phi_k)),
+// and the Gauss points of the steps lie symmetrically about the middle, so the even and the odd sum at one
+// distance give two samples.  The sums of a block of output intervals (rows, through L) at a block of
+// distances (columns, through cos and sin) are matrix products with inner dimension (tones per channel) each.
+// They run as mma.sync.m8n8k4.f64 (FP64 in, FP64 accumulate: the samples are exact to FP64 rounding), which
+// takes eight multiply-adds per lane per instruction.  (Sampling each time by itself takes twice the
+// products: inner dimension 2 x tones for one sample.)
 //
 // Mapping.  A CTA takes a tile of kDmmaTile consecutive output intervals of one instance; warp w
-// takes intervals 8 w .. 8 w + 7 (the eight rows of the m8n8k4 product).  Each interval's K fine
-// steps are split into kDmmaSegments consecutive segments, one per lane of a quad: in the
-// accumulator layout lane 4 g + q holds row g, columns 2 q and 2 q + 1, which are made to be the
-// two Gauss points of one step of segment q.  So every lane receives exactly the two field
-// samples of its own step, runs the step's exponentials and keeps the FP64 product of its
-// segment; the four segment products are combined once per interval with quad shuffles (later
-// segments multiply from the left, as append_exponentiation does, I:561-580).
+// takes intervals 8 w .. 8 w + 7 (the eight rows of the m8n8k4 product).  The K / 2 steps after the middle
+// are split into kDmmaSegments consecutive segments, one per lane of a quad: in the accumulator layout lane
+// 4 g + q holds row g, columns 2 q and 2 q + 1, which are made to be the distances of the two Gauss points
+// of one step of segment q.  So every lane receives the samples of its own step and of that step's mirror
+// image before the middle; it multiplies the first to its product of later steps from the left and the second
+// to its product of earlier steps from the right, two independent chains.  The quad's products are combined
+// once per interval with shuffles.  For odd K the middle step, its own mirror image, takes one column of one
+// more product.
 //
-// Operands.  A (8 x 4 per k-step): lane 4 g + q holds L of interval g for tone 2 s + q / 2, real
-// part for even q and imaginary part for odd q, computed once per tile with FP64 sincos.  B (4 x 8):
-// lane 4 g + q needs sin / cos (w tau) for that tone at the step of segment g / 2, Gauss point
-// g % 2.  These depend on the instance only, not on the interval, so the CTA builds them in shared
-// memory: 192 phasor recurrences exp(i w tau) (channel, tone, segment, Gauss point) advanced by
-// exp(i w dt) per step in FP64, written in lane order so that every B load is one conflict-free
-// 8-byte load per lane.  The table is double-buffered in phases of kDmmaPhase steps (one CTA barrier
-// per phase).  The accumulator starts at the channel bias.
+// Operands.  A (8 x 4 per k-step): lane 4 g + q holds Im L (even sums) or Re L (odd sums) of interval g for tone
+// 4 s + q, computed once per tile with FP64 sincos.  B (4 x 8): lane 4 g + q needs cos or sin (w delta) of that
+// tone at column g.  These depend on the instance only, not on the interval, so the CTA builds them in shared
+// memory: 192 phasor recurrences exp(i w delta) (channel, tone, column) advanced by exp(i w dt) per pair of steps
+// in FP64, written in lane order so that every B load and store is conflict-free.  The table is double-buffered
+// in phases of kDmmaPhase pairs (one CTA barrier per phase).  The even sums start at the channel bias.
 //
-// Step.  The reference's Magnus CF4 (I:655-686) composes two exponentials per step; its order-four
+// Step, FP32-bulk.  The reference's Magnus CF4 (I:655-686) composes two exponentials per step; its order-four
 // Magnus expansion at the same Gauss points, exp(g), g = (h/2)(b1 + b2) + (sqrt3 h^2 / 12) b2 x b1
 // (the commutator [A2, A1] of A = -i b.J is -i (b2 x b1).J; Blanes, Casas and Ros, BIT 40 (2000)),
 // is the same map to O(h^5): one SU(2) exponential per step.  A tile takes it when the step is small
@@ -38,6 +41,9 @@
 // to 1e-11 in the final state.  Instances with more than kBulkTones
 // tones on a channel, or spin one with a quadratic shift, take the per-interval path (interval32,
 // CF4) inside the same kernel.
+//
+// Step, FP64.  CF4 with the two FP64 exponentials of evolve64.cuh.  Instances the products do not take run in
+// that file's kernel instead (the host splits the batch's tiles).
 //
 // Scan partials.  A CTA tile is one state scan tile (scan.cuh).  Each interval's lab-frame operator is
 // an SU(2) pair (spin one: its representation), so each warp also multiplies its eight rows' pairs
@@ -61,16 +67,23 @@ constexpr int kDmmaPhase = SPINSIM_DMMA_PHASE;
 // and 1e-11 over 10^6 steps at theta = 0.07, i.e. about 3e-10 theta^5 per step, so at theta <= 0.1
 // below 4e-15 per step, 4e-9 over 10^6 steps.
 constexpr double kMagnusTheta = 0.1;
-constexpr int kDmmaChunkDoubles = 3 * 4 * 32;                // B operands of one step: [channel][k-step][lane]
+constexpr int kDmmaChunkDoubles = 3 * 4 * 32;  // B operands of one pair: [channel][even, odd][k-step][lane]
 static_assert(kDmmaRecurrences == 3 * kBulkTones * kDmmaSegments * 2, "(channel, tone, segment, Gauss point)");
+static_assert(kBulkTones == 8 && kDmmaSegments == 4, "two k-steps of four tones, eight columns");
+// CF4 generators from samples in units of h / 2: h (w0 b1 + w1 b2) = 2 w0 sa + 2 w1 sb
+constexpr double kDmmaW0 = (1.5 + kSqrt3) / 3.0, kDmmaW1 = (1.5 - kSqrt3) / 3.0;
+
+// First pair of segment seg: pair i is the i-th step after the middle of the K and its mirror image.
+SS_D int dmma_segment(int K, int seg) { return (int)(((int64_t)(K / 2) * seg) / kDmmaSegments); }
 
 struct __align__(16) DmmaShared {
     double table[2][kDmmaPhase][kDmmaChunkDoubles];
-    double2 z[kDmmaRecurrences];  // exp(i w tau) of each recurrence at its next step
-    double2 rot[3 * kBulkTones];  // exp(i w dt)
-    double2 half_step[3 * kBulkTones];  // exp(i w dt_out / 2)
+    double2 z[kDmmaRecurrences];   // exp(i w delta) of each recurrence at its next pair
+    double2 rot[kToneSlots];       // exp(i w dt)
+    double2 middle[kToneSlots];    // exp(i w delta) at the middle step's samples
+    Su2p warp_product[kDmmaWarps];
     int32_t tile;
-    int32_t magnus;                     // 1: the tile takes the one-exponential Magnus step
+    int32_t magnus;                // 1: the tile takes the one-exponential Magnus step
 };
 
 // d[0..1] += a b over the 8 x 8 x 4 product of the warp (FP64 tensor path).
@@ -80,20 +93,10 @@ SS_D void dmma_m8n8k4(double& d0, double& d1, double a, double b) {
         : "d"(a), "d"(b));
 }
 
-// b a in FP64 residual form (b later): alpha - 1 = a.am1 + b.am1 + b.am1 a.am1 - conj(b.beta) a.beta,
-// beta = b.beta + a.beta + b.beta a.am1 + conj(b.am1) a.beta.
-SS_D Su2d su2d_mul(const Su2d& b, const Su2d& a) {
-    Su2d o;
-    o.am1 = cfma(b.am1, a.am1, a.am1 + b.am1) - conj(b.beta) * a.beta;
-    o.beta = cfma(b.beta, a.am1, b.beta + a.beta) + conj(b.am1) * a.beta;
-    return o;
-}
-
 static_assert(kDmmaTile == kScanTile, "a CTA tile is one state scan tile (its warps' row products are its partials)");
 
-// Recurrence r = ((channel * kBulkTones + tone) * kDmmaSegments + segment) * 2 + Gauss point of an
-// instance with K fine steps of dt: its start phasor exp(i w tau), tau = (segment start) dt + a_lo or
-// a_hi (the reference's sample offsets, I:644-647), and its tone's step rotation exp(i w dt).
+// Pair recurrence r = slot * 8 + column (column = 2 * segment + Gauss point): the phasor exp(i w delta) of its tone
+// at the column's first distance from the middle of the interval, and the tone's step rotation exp(i w dt).
 SS_D void dmma_recurrence(const FieldDesc& f, int K, double dt, int r, double2* z, double2* rot) {
     const int gauss = r & 1, seg = (r >> 1) & (kDmmaSegments - 1), slot = r >> 3;
     const int c = slot / kBulkTones, tone = slot % kBulkTones;
@@ -102,21 +105,21 @@ SS_D void dmma_recurrence(const FieldDesc& f, int K, double dt, int r, double2* 
     if (tone < f.tone_count[c]) {
         const double a = 0.5 * dt * (gauss ? 1.0 + 1.0 / kSqrt3 : 1.0 - 1.0 / kSqrt3);
         const double w = __ldg(f.tones + 3 * (f.tone_start[c] + tone));
-        const int start = (int)(((int64_t)K * seg) / kDmmaSegments);
+        const double start = (double)dmma_segment(K, seg) + (K & 1 ? 0.5 : 0.0);
         double sn, cs;
-        sincos(w * fma((double)start, dt, a), &sn, &cs);
+        sincos(w * fma(start, dt, a), &sn, &cs);
         *z = make_double2(cs, sn);
         sincos(w * dt, &sn, &cs);
         *rot = make_double2(cs, sn);
     }
 }
 
-// exp(i w dt_out / 2) of tone slot (1 for an absent tone).
-SS_D double2 dmma_half_step(const FieldDesc& f, int slot, double dt_out) {
+// exp(i w tau) of tone slot (1 for an absent tone).
+SS_D double2 dmma_phasor(const FieldDesc& f, int slot, double tau) {
     const int c = slot / kBulkTones, tone = slot % kBulkTones;
     if (tone >= f.tone_count[c]) return make_double2(1.0, 0.0);
     double sn, cs;
-    sincos(0.5 * __ldg(f.tones + 3 * (f.tone_start[c] + tone)) * dt_out, &sn, &cs);
+    sincos(__ldg(f.tones + 3 * (f.tone_start[c] + tone)) * tau, &sn, &cs);
     return make_double2(cs, sn);
 }
 
@@ -160,7 +163,10 @@ __global__ void __launch_bounds__(kDmmaRecurrences) dmma_consts_kernel(const __g
     dmma_recurrence(f, inst.n_fine, inst.dt_int, r, &z, &rot);
     c.z[r] = z;
     if ((r & 7) == 0) c.rot[r >> 3] = rot;
-    if (r < kToneSlots) c.half_step[r] = dmma_half_step(f, r, inst.dt_out);
+    if (r < kToneSlots) {
+        c.half_step[r] = dmma_phasor(f, r, 0.5 * inst.dt_out);
+        c.middle[r] = dmma_phasor(f, r, inst.dt_int * (0.5 / kSqrt3));
+    }
     if (r == 0) c.magnus = dmma_magnus(f, inst.dt_int);
 }
 #endif
@@ -177,17 +183,75 @@ SS_D void store_interval_operator(const Su2p& v, double* u_out, int64_t idx) {
         for (int k = 0; k < D; k++) dst[r * D + k] = make_double2(u.a[r][k].re, u.a[r][k].im);
 }
 
+// How far an output step's start, rounded as the reference rounds it (I:818), lies from t0 + dt_out i.
+SS_D double time_rounding(double t0, double dt_out, double i) {
+    const double p = __dmul_rn(dt_out, i), ep = __fma_rn(dt_out, i, -p);
+    const double s = __dadd_rn(t0, p), b = __dsub_rn(s, t0);
+    return -(__dadd_rn(__dsub_rn(t0, __dsub_rn(s, b)), __dsub_rn(p, b)) + ep);
+}
+
+// One step's element from its samples in units of h / 2, FP32-bulk: the Magnus step or the reference's CF4
+// (I:655-686).
+SS_D Su2d dmma_step32(const double* sa, const double* sb, bool magnus, float* nsq) {
+    if (magnus) {
+        // g = (h / 2)(b1 + b2) + (sqrt3 h^2 / 12) b2 x b1, with (h / 2) b in sa, sb: the linear part
+        // g_lin = sa + sb stays FP64; the commutator (sqrt3 / 6) d x g_lin, d = (h / 2)(b2 - b1), and
+        // the exponential's remainder are FP32.
+        double gl64[3];
+        float gl[3], dd[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            gl64[c] = sa[c] + sb[c];
+            gl[c] = __double2float_rn(gl64[c]);
+            dd[c] = __double2float_rn(sb[c] - sa[c]);
+        }
+        constexpr float kComm = 0.28867513459481287f;  // sqrt3 / 6
+        const float cx = kComm * fmaf(dd[1], gl[2], -dd[2] * gl[1]);
+        const float cy = kComm * fmaf(dd[2], gl[0], -dd[0] * gl[2]);
+        const float cz = kComm * fmaf(dd[0], gl[1], -dd[1] * gl[0]);
+        Su2f rest = su2_exp_rest(gl[0] + cx, gl[1] + cy, gl[2] + cz);
+        rest.am1.im = fmaf(-0.5f, cz, rest.am1.im);  // the commutator's linear part
+        rest.beta.re = fmaf(0.5f, cy, rest.beta.re);
+        rest.beta.im = fmaf(-0.5f, cx, rest.beta.im);
+        *nsq = fmaf(gl[0], gl[0], fmaf(gl[1], gl[1], fmaf(gl[2], gl[2], *nsq)));
+        return su2_split(gl64[0], gl64[1], gl64[2], rest);
+    }
+    double ga[3], gb[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        ga[c] = fma(kDmmaW0, sa[c], kDmmaW1 * sb[c]);
+        gb[c] = fma(kDmmaW1, sa[c], kDmmaW0 * sb[c]);
+    }
+    return su2_cf4_element(ga, gb, nsq);
+}
+
+// The quad's four lanes hold products of consecutive pair segments; lane 0 of the quad gets the whole product:
+// of steps after the middle (later segments from the left) and of mirrored steps before it (from the right).
+template <bool MIRRORED>
+SS_D void combine_segments(Su2d& p, int q) {
+#pragma unroll
+    for (int s = 1; s < kDmmaSegments; s <<= 1) {
+        Su2d other = shfl_down_su2(p, s);
+        if ((q & (2 * s - 1)) != 0) continue;
+        if (MIRRORED) {
+            su2_apply64(other, p);
+            p = other;
+        } else {
+            su2_apply64(p, other);
+        }
+    }
+}
+
 // partial_out (may be null): the tile's scan partials, where this warp writes the lab-frame SU(2) pair of
-// its rows' product (later rows from the left; rows past the tile's end are the identity).  cst (may be
-// null): the instance's constants from dmma_consts_kernel; without them the tile computes them.  The
-// spin dimension enters only the frame winding and the stored operator, so a mixed-spin launch
-// (DIMS 0) runs one copy of the step loop for both spins.
-template <int DIMS>
+// its rows' product (later rows from the left; rows past the tile's end are the identity); product_out (may be
+// null): the tile's product as a d x d operator instead.  The spin dimension enters only the frame winding, the
+// exponentiator and the stored operator, so a mixed-spin launch (DIMS 0) runs one copy of the step loop for
+// both spins.
+template <int DIMS, int PREC>
 SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc& f, const Tile& tile, DmmaShared& sh,
-                    double* time_out, double* u_out, float* norms_out, double* partial_out, const DmmaConsts* cst,
-                    double* rows_out) {
+                    double* time_out, double* u_out, float* norms_out, double* partial_out, double* product_out,
+                    const DmmaConsts* cst, double* rows_out) {
     const int D = DIMS != 0 ? DIMS : inst.dim;
-    const int P = (D == 2) ? 2 : 1;  // power of the frame winding in the xy transform (I:599-613)
     const int lane = threadIdx.x & 31;
     const int g = lane >> 2, q = lane & 3;
     const int row = (threadIdx.x >> 5) * kDmmaRows + g;
@@ -195,225 +259,257 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
     const int64_t idx = tile.first + (active ? row : 0);
     const double dt = inst.dt_int, dt_out = inst.dt_out;
     const int K = inst.n_fine;
-    const int seg_start = (int)(((int64_t)K * q) / kDmmaSegments);
-    const int seg_len = (int)(((int64_t)K * (q + 1)) / kDmmaSegments) - seg_start;
-    const int n_steps = (K + kDmmaSegments - 1) / kDmmaSegments;  // steps of the longest segment
+    const int seg_start = dmma_segment(K, q);
+    const int seg_len = dmma_segment(K, q + 1) - seg_start;
+    const int n_steps = (K / 2 + kDmmaSegments - 1) / kDmmaSegments;  // pairs of the longest segment
     const double a_lo = 0.5 * dt * (1.0 - 1.0 / kSqrt3);
     const double a_hi = 0.5 * dt * (1.0 + 1.0 / kSqrt3);
     const double half_dt = 0.5 * dt;
     const double t_c = __dadd_rn(inst.t0, __dmul_rn(dt_out, (double)(inst.interval0 + idx)));  // I:818, unfused
 
-    // Producer recurrences (dmma_recurrence), their rotations and the step choice: the instance's
-    // constants, or computed here.
-    if (cst != nullptr) {
-        grid_dependency_wait();  // the constants' kernel may still be running (it lets this launch start early)
-        for (int r = threadIdx.x; r < kDmmaRecurrences; r += kDmmaThreads) sh.z[r] = cst->z[r];
-        if (threadIdx.x < kToneSlots) sh.rot[threadIdx.x] = cst->rot[threadIdx.x];
-        if (threadIdx.x == 0) sh.magnus = cst->magnus;
-    } else {
-        for (int r = threadIdx.x; r < kDmmaRecurrences; r += kDmmaThreads) {
-            double2 z, rot;
-            dmma_recurrence(f, K, dt, r, &z, &rot);
-            sh.z[r] = z;
-            if ((r & 7) == 0) sh.rot[r >> 3] = rot;
-        }
-        if (threadIdx.x == 0) sh.magnus = dmma_magnus(f, dt);
+    // The instance's constants (dmma_consts_kernel, which may still be running: it lets this launch start early).
+    grid_dependency_wait();
+    for (int r = threadIdx.x; r < kDmmaRecurrences; r += kDmmaThreads) sh.z[r] = cst->z[r];
+    if (threadIdx.x < kToneSlots) {
+        sh.rot[threadIdx.x] = cst->rot[threadIdx.x];
+        sh.middle[threadIdx.x] = cst->middle[threadIdx.x];
     }
+    if (threadIdx.x == 0) sh.magnus = cst->magnus;
 
-    // L of every tone and interval of the tile (buffer 1 of the table holds it until the first refill):
-    // thread 4 slot + quarter evaluates interval 8 quarter once and steps to the next seven intervals
-    // with exp(i w dt_out); h = exp(i w dt_out / 2) per tone is kept for the frame's mid-interval sample.
+    // L of every tone at the middle of every interval of the tile (buffer 1 of the table holds it until the first
+    // refill): thread 4 slot + quarter evaluates interval 8 quarter once and steps to the next seven intervals
+    // with exp(i w dt_out), corrected for the rounding of each interval's start (a phase of w times it, below
+    // 1e-10, so to first order).
     double2* lval = reinterpret_cast<double2*>(&sh.table[1][0][0]);  // [slot][interval of the tile]
     static_assert(sizeof(sh.table[1]) >= sizeof(double2) * kToneSlots * kDmmaTile, "L table fits one buffer");
     if (threadIdx.x < 4 * kToneSlots) {
         const int slot = threadIdx.x >> 2, quarter = threadIdx.x & 3;
         const int c = slot / kBulkTones, tone = slot % kBulkTones;
-        c64 l = c64{0.0, 0.0}, gstep = c64{1.0, 0.0}, h = c64{1.0, 0.0};
+        const int64_t i0 = inst.interval0 + tile.first + kDmmaRows * quarter;
+        c64 l = c64{0.0, 0.0}, gstep = c64{1.0, 0.0};
+        double w = 0.0;
         if (tone < f.tone_count[c]) {
             const double* tn = f.tones + 3 * (f.tone_start[c] + tone);
-            const double w = __ldg(tn), amp = f.gain[c] * __ldg(tn + 1);
-            const int64_t i0 = inst.interval0 + tile.first + kDmmaRows * quarter;
+            const double amp = f.gain[c] * __ldg(tn + 1);
+            w = __ldg(tn);
             const double tq = __dadd_rn(inst.t0, __dmul_rn(dt_out, (double)i0));  // as the intervals' own t_c
             double sn, cs;
             sincos(fma(w, tq, __ldg(tn + 2)), &sn, &cs);
-            l = c64{half_dt * amp * cs, half_dt * amp * sn};
-            const double2 hs = cst != nullptr ? cst->half_step[slot] : dmma_half_step(f, slot, dt_out);
-            h = c64{hs.x, hs.y};
+            const double2 hs = cst->half_step[slot];
+            const c64 h = c64{hs.x, hs.y};
+            l = c64{half_dt * amp * cs, half_dt * amp * sn} * h;
             gstep = h * h;
         }
-        if (quarter == 0) sh.half_step[slot] = make_double2(h.re, h.im);
+        const double first = time_rounding(inst.t0, dt_out, (double)i0);
 #pragma unroll
         for (int r = 0; r < kDmmaRows; r++) {
-            lval[slot * kDmmaTile + kDmmaRows * quarter + r] = make_double2(l.re, l.im);
+            const double turn = w * (time_rounding(inst.t0, dt_out, (double)(i0 + r)) - first);
+            lval[slot * kDmmaTile + kDmmaRows * quarter + r] = make_double2(fma(-turn, l.im, l.re), fma(turn, l.re, l.im));
             l = l * gstep;
         }
     }
     __syncthreads();  // producer phasors, rotations, step choice and L in place
 
-    // A operands: L of this lane's interval for tone 2 s + q / 2 (Re L for even q, Im L for odd q)
-    double afr[3][4];
+    // A operands: L of this lane's interval for tone 4 s + q, its imaginary part for the even sums, real for the odd
+    double even_a[3][2], odd_a[3][2];
 #pragma unroll
     for (int c = 0; c < 3; c++)
 #pragma unroll
-        for (int s = 0; s < 4; s++) {
-            const double* lv = reinterpret_cast<const double*>(&lval[(c * kBulkTones + 2 * s + (q >> 1)) * kDmmaTile + row]);
-            afr[c][s] = active ? lv[q & 1] : 0.0;
+        for (int s = 0; s < 2; s++) {
+            const double2 lv = lval[(c * kBulkTones + 4 * s + q) * kDmmaTile + row];
+            even_a[c][s] = active ? lv.y : 0.0;
+            odd_a[c][s] = active ? lv.x : 0.0;
         }
-    // Rotating frame (I:823-829): Bz at the middle of the interval, sum_k Im(L_zk h_k) + bias;
-    // lane q sums tones 2 q, 2 q + 1 and the quad adds the four parts.
-    double rw = 0.0;
+    // Rotating frame (I:823-829): Bz at the middle of the interval, sum_k Im L_zk + bias; lane q sums tones
+    // 2 q, 2 q + 1 and the quad adds the four parts.  prw: P times the frame's rate (for either spin).
+    double prw = 0.0;
     if (m.rotating) {
         double part = 0.0;
 #pragma unroll
-        for (int k = 2 * q; k < 2 * q + 2; k++) {
-            const double2 lz = lval[(2 * kBulkTones + k) * kDmmaTile + row];
-            const double2 hk = sh.half_step[2 * kBulkTones + k];
-            part += fma(lz.x, hk.y, lz.y * hk.x);
-        }
+        for (int k = 2 * q; k < 2 * q + 2; k++) part += lval[(2 * kBulkTones + k) * kDmmaTile + row].y;
         part += __shfl_xor_sync(0xffffffffu, part, 1);
         part += __shfl_xor_sync(0xffffffffu, part, 2);
-        rw = f.bias[2] + part / half_dt;
-        if (D == 2) rw /= 2;
+        prw = f.bias[2] + part / half_dt;
     }
-    const double prw = (double)P * rw;
-    const double hprw = half_dt * prw;
-    // (h / 2) bias, the starting value of the samples' accumulation; in the rotating frame z also
-    // carries the frame's -P rw (I:582-618), added once here instead of to every sample
+    // (h / 2) bias, the starting value of the even sums; in the rotating frame z also carries the frame's
+    // -P rw (I:582-618), added once here instead of to every sample
     double bias[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) bias[c] = half_dt * f.bias[c];
-    bias[2] -= hprw;
-    // Frame phasors at the Gauss points of this segment's steps: exp(-i P rw (tau - 0)), tau as above
+    bias[2] -= half_dt * prw;
+    // Frame phasors at the Gauss points of this segment's steps after the middle: exp(-i P rw delta); those of
+    // the mirrored steps before it are their conjugates
+    const double start = (double)seg_start + (K & 1 ? 0.5 : 0.0);
     c64 wa = c64{1.0, 0.0}, wb = c64{1.0, 0.0}, wrot = c64{1.0, 0.0};
     if (m.rotating) {
         sincos_small(-prw * dt, &wrot.im, &wrot.re);
-        sincos_small(-prw * fma((double)seg_start, dt, a_lo), &wa.im, &wa.re);
-        sincos_small(-prw * fma((double)seg_start, dt, a_hi), &wb.im, &wb.re);
+        sincos_small(-prw * fma(start, dt, a_lo), &wa.im, &wa.re);
+        sincos_small(-prw * fma(start, dt, a_hi), &wb.im, &wb.re);
     }
 
-    // Fill table buffer (ph & 1) with the B operands of steps [ph kDmmaPhase, ...) of every segment.
+    // Fill table buffer (ph & 1) with the B operands of pairs [ph kDmmaPhase, ...) of every segment.
     auto fill = [&](int ph) {
         const int m0 = ph * kDmmaPhase;
         const int mc = min(kDmmaPhase, n_steps - m0);
         for (int r = threadIdx.x; r < kDmmaRecurrences; r += kDmmaThreads) {
-            const int gauss = r & 1, seg = (r >> 1) & (kDmmaSegments - 1), slot = r >> 3;
+            const int col = r & 7, slot = r >> 3;
             const int c = slot / kBulkTones, tone = slot % kBulkTones;
-            // consumer lane 4 g' + q' with g' = 2 segment + Gauss point, q' = 2 (tone & 1) + (0 sin, 1 cos)
-            double* dst = &sh.table[ph & 1][0][(c * 4 + (tone >> 1)) * 32 + 4 * (2 * seg + gauss) + 2 * (tone & 1)];
+            // consumer lane 4 col + tone % 4 of k-step tone / 4: cosines (even sums), then sines
+            double* dst = &sh.table[ph & 1][0][(c * 4 + (tone >> 2)) * 32 + 4 * col + (tone & 3)];
             double2 z = sh.z[r];
             const double2 rt = sh.rot[slot];
             for (int mm = 0; mm < mc; mm++) {
-                *reinterpret_cast<double2*>(dst + mm * kDmmaChunkDoubles) = make_double2(z.y, z.x);
+                dst[mm * kDmmaChunkDoubles] = z.x;
+                dst[mm * kDmmaChunkDoubles + 64] = z.y;
                 z = make_double2(fma(z.x, rt.x, -z.y * rt.y), fma(z.x, rt.y, z.y * rt.x));
             }
             sh.z[r] = z;
         }
     };
 
-    fill(0);  // buffer 0; buffer 1 (the L table) is first refilled after the barrier below
-    __syncthreads();
-    const bool magnus = sh.magnus != 0;
-    // CF4 generators from samples in units of h / 2: h (w0 b1 + w1 b2) = 2 w0 sa + 2 w1 sb
-    constexpr double kW0 = (1.5 + kSqrt3) / 3.0, kW1 = (1.5 - kSqrt3) / 3.0;
-    Su2d acc = Su2d{c64{0.0, 0.0}, c64{0.0, 0.0}};
+    Su2d after = Su2d{c64{0.0, 0.0}, c64{0.0, 0.0}};   // this lane's steps after the middle
+    Su2d before = Su2d{c64{0.0, 0.0}, c64{0.0, 0.0}};  // and their mirrored steps before it
     float nsq = 0.0f;  // sum of |g|^2 over this lane's steps (the error statement's scale)
+    const bool magnus = sh.magnus != 0;
+    const bool lie_trotter = D == 3 || m.expo_half == EXPO_LIE_TROTTER;
+    // An xy sample in the rotating frame (I:582-618; z: in the bias)
+    auto rotate = [&](double* s, c64 w) {
+        const c64 x = c64{s[0], s[1]} * w;
+        s[0] = x.re;
+        s[1] = x.im;
+    };
+    // p <- step p (a step after p's), or p step (a mirrored step, before p's)
+    auto apply = [&](Su2d& p, double* sa, double* sb, bool mirrored) {
+        Su2d e;
+        if constexpr (PREC == PREC_FP32_BULK) {
+            e = dmma_step32(sa, sb, magnus, &nsq);
+        } else {  // the reference's CF4 (I:655-686) with FP64 exponentials
+            double ga[3], gb[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                ga[c] = fma(kDmmaW0, sa[c], kDmmaW1 * sb[c]);
+                gb[c] = fma(kDmmaW1, sa[c], kDmmaW0 * sb[c]);
+            }
+            e = su2_step_element64(m, lie_trotter, ga);
+            const Su2d eb = su2_step_element64(m, lie_trotter, gb);
+            if (!mirrored) {
+                su2_apply64(p, e);
+                e = eb;
+            } else {
+                su2_apply64(e, eb);
+            }
+        }
+        if (mirrored) {
+            su2_apply64(e, p);
+            p = e;
+        } else {
+            su2_apply64(p, e);
+        }
+    };
+
+    fill(0);  // buffer 0; buffer 1 (the L table) is first refilled after the barrier below
+    if (K & 1) {  // the middle step, whose two samples mirror each other: column 0 of one more product
+        double ev[3], od[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            double e0 = bias[c], e1 = 0.0, o0 = 0.0, o1 = 0.0;
+#pragma unroll
+            for (int s = 0; s < 2; s++) {
+                const double2 z = sh.middle[c * kBulkTones + 4 * s + q];
+                dmma_m8n8k4(e0, e1, even_a[c][s], g == 0 ? z.x : 0.0);
+                dmma_m8n8k4(o0, o1, odd_a[c][s], g == 0 ? z.y : 0.0);
+            }
+            ev[c] = e0;
+            od[c] = o0;
+        }
+        if (active && q == 0) {
+            double sa[3], sb[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                sa[c] = ev[c] - od[c];
+                sb[c] = ev[c] + od[c];
+            }
+            if (m.rotating) {
+                c64 w;
+                sincos_small(-prw * (dt * (0.5 / kSqrt3)), &w.im, &w.re);
+                rotate(sa, conj(w));
+                rotate(sb, w);
+            }
+            apply(after, sa, sb, false);
+        }
+    }
+    __syncthreads();
     const int n_phases = (n_steps + kDmmaPhase - 1) / kDmmaPhase;
     for (int ph = 0; ph < n_phases; ph++) {
         if (ph + 1 < n_phases) fill(ph + 1);
         const int m0 = ph * kDmmaPhase;
         const int mc = min(kDmmaPhase, n_steps - m0);
         const double* tb = &sh.table[ph & 1][0][lane];
-        // The samples of step mm + 1 (tensor path) are issued at the end of step mm, so they are in flight
-        // while the next step begins.
-        double na[3], nb[3];
-        auto samples = [&](int mm, double* xa, double* xb) {
+        // Even and odd sums at the two distances of pair mm (tensor path), issued at the end of pair mm - 1, so
+        // they are in flight while the next pair begins.
+        double e0[3], e1[3], o0[3], o1[3];
+        auto sums = [&](int mm) {
 #pragma unroll
             for (int c = 0; c < 3; c++) {
-                double d0 = bias[c], d1 = bias[c];
+                e0[c] = e1[c] = bias[c];
+                o0[c] = o1[c] = 0.0;
+                const double* t = tb + mm * kDmmaChunkDoubles + c * 128;
 #pragma unroll
-                for (int s = 0; s < 4; s++) dmma_m8n8k4(d0, d1, afr[c][s], tb[mm * kDmmaChunkDoubles + (c * 4 + s) * 32]);
-                xa[c] = d0;
-                xb[c] = d1;
+                for (int s = 0; s < 2; s++) {
+                    dmma_m8n8k4(e0[c], e1[c], even_a[c][s], t[32 * s]);
+                    dmma_m8n8k4(o0[c], o1[c], odd_a[c][s], t[64 + 32 * s]);
+                }
             }
         };
-        samples(0, na, nb);
+        sums(0);
         for (int mm = 0; mm < mc; mm++) {
-            double sa[3], sb[3];
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                sa[c] = na[c];
-                sb[c] = nb[c];
-            }
             if (active && m0 + mm < seg_len) {
-                if (m.rotating) {  // xy times exp(-i P rw tau) (I:582-618), in units of h / 2 (z: in the bias)
-                    const c64 xa = c64{sa[0], sa[1]} * wa;
-                    const c64 xb = c64{sb[0], sb[1]} * wb;
-                    sa[0] = xa.re;
-                    sa[1] = xa.im;
-                    sb[0] = xb.re;
-                    sb[1] = xb.im;
+                double sa[3], sb[3], ma[3], mb[3];  // the step after the middle, and its mirror image
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    sa[c] = e0[c] + o0[c];
+                    sb[c] = e1[c] + o1[c];
+                    ma[c] = e1[c] - o1[c];
+                    mb[c] = e0[c] - o0[c];
+                }
+                if (m.rotating) {
+                    rotate(sa, wa);
+                    rotate(sb, wb);
+                    rotate(ma, conj(wb));
+                    rotate(mb, conj(wa));
                     wa = wa * wrot;
                     wb = wb * wrot;
                 }
-                if (magnus) {
-                    // g = (h / 2)(b1 + b2) + (sqrt3 h^2 / 12) b2 x b1, with (h / 2) b in sa, sb: the
-                    // linear part g_lin = sa + sb stays FP64; the commutator (sqrt3 / 6) d x g_lin,
-                    // d = (h / 2)(b2 - b1), and the exponential's remainder are FP32.
-                    double gl64[3];
-                    float gl[3], dd[3];
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        gl64[c] = sa[c] + sb[c];
-                        gl[c] = __double2float_rn(gl64[c]);
-                        dd[c] = __double2float_rn(sb[c] - sa[c]);
-                    }
-                    constexpr float kComm = 0.28867513459481287f;  // sqrt3 / 6
-                    const float cx = kComm * fmaf(dd[1], gl[2], -dd[2] * gl[1]);
-                    const float cy = kComm * fmaf(dd[2], gl[0], -dd[0] * gl[2]);
-                    const float cz = kComm * fmaf(dd[0], gl[1], -dd[1] * gl[0]);
-                    Su2f rest = su2_exp_rest(gl[0] + cx, gl[1] + cy, gl[2] + cz);
-                    rest.am1.im = fmaf(-0.5f, cz, rest.am1.im);  // the commutator's linear part
-                    rest.beta.re = fmaf(0.5f, cy, rest.beta.re);
-                    rest.beta.im = fmaf(-0.5f, cx, rest.beta.im);
-                    nsq = fmaf(gl[0], gl[0], fmaf(gl[1], gl[1], fmaf(gl[2], gl[2], nsq)));
-                    su2_apply64(acc, su2_split(gl64[0], gl64[1], gl64[2], rest));
-                } else {  // the reference's CF4 (I:655-686): two exponentials
-                    double ga[3], gb[3];
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        ga[c] = fma(kW0, sa[c], kW1 * sb[c]);
-                        gb[c] = fma(kW1, sa[c], kW0 * sb[c]);
-                    }
-                    su2_apply64(acc, su2_cf4_element(ga, gb, &nsq));
-                }
+                apply(after, sa, sb, false);
+                apply(before, ma, mb, true);
             }
-            // the next step's samples, issued after this step's arithmetic (all lanes: mma.sync is
+            // the next pair's sums, issued after this pair's arithmetic (all lanes: mma.sync is
             // warp-collective); measured 0.7% faster than issuing them before it
-            if (mm + 1 < mc) samples(mm + 1, na, nb);
+            if (mm + 1 < mc) sums(mm + 1);
         }
         __syncthreads();  // buffer (ph & 1) is refilled in phase ph + 1
     }
 
-    // The interval's product: segment 3 ... segment 0 (later segments from the left)
+    // The interval's product, in lane 0 of the quad
+    combine_segments<false>(after, q);
+    combine_segments<true>(before, q);
+    su2_apply64(before, after);
+    if constexpr (PREC == PREC_FP32_BULK) {
 #pragma unroll
-    for (int sft = 1; sft < kDmmaSegments; sft <<= 1) {
-        const Su2d later = shfl_down_su2(acc, sft);
-        nsq += __shfl_down_sync(0xffffffffu, nsq, sft);
-        if ((q & (2 * sft - 1)) == 0) acc = su2d_mul(later, acc);
+        for (int s = 1; s < kDmmaSegments; s <<= 1) nsq += __shfl_down_sync(0xffffffffu, nsq, s);
     }
-    // The interval's lab-frame operator as an SU(2) pair: leaving the frame (I:839-852) multiplies by
-    // the SU(2) element diag(exp(-i phi), exp(i phi)), phi = rw dt_out (spin half, rw halved above) or
-    // rw dt_out / 2 (spin one, whose representation doubles the phase).  Rows past the tile's end and
-    // the other lanes of a quad hold the identity.
+    // The interval's lab-frame operator as an SU(2) pair.  With the frame's phases counted from the middle of the
+    // interval, entering and leaving the frame (I:839-852) multiply alpha by exp(-i P rw dt_out / 2) and leave
+    // beta (spin one: the same element's representation).  Rows past the tile's end and the other lanes of a quad
+    // hold the identity.
     Su2p v = su2p_identity();
     if (active && q == 0) {
-        v.a = c64{1.0 + acc.am1.re, acc.am1.im};
-        v.b = acc.beta;
+        v.a = c64{1.0 + before.am1.re, before.am1.im};
+        v.b = before.beta;
         if (m.rotating) {
-            c64 wh;
-            sincos_small(rw * dt_out * (D == 2 ? 1.0 : 0.5), &wh.im, &wh.re);
-            v.a = v.a * conj(wh);
-            v.b = v.b * wh;
+            c64 w;
+            sincos_small(0.5 * prw * dt_out, &w.im, &w.re);
+            v.a = v.a * conj(w);
         }
         time_out[idx] = t_c;
         if (norms_out != nullptr) norms_out[idx] = nsq;
@@ -425,16 +521,24 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
             r[1] = make_double2(v.b.re, v.b.im);
         }
     }
-    if (partial_out != nullptr) {  // the warp's product of its rows (lanes 4 g), later rows from the left
+    if (partial_out == nullptr && product_out == nullptr) return;
 #pragma unroll
-        for (int sft = kDmmaSegments; sft < 32; sft <<= 1) {
-            const Su2p later = shfl_down_su2p(v, sft);
-            if ((lane & (2 * sft - 1)) == 0) v = su2p_mul(later, v);
-        }
-        if (lane == 0) {
-            double2* dst = reinterpret_cast<double2*>(partial_out) + 2 * (threadIdx.x >> 5);
-            dst[0] = make_double2(v.a.re, v.a.im);
-            dst[1] = make_double2(v.b.re, v.b.im);
+    for (int sft = kDmmaSegments; sft < 32; sft <<= 1) {  // the warp's product of its rows (lanes 4 g), later rows from the left
+        const Su2p later = shfl_down_su2p(v, sft);
+        if ((lane & (2 * sft - 1)) == 0) v = su2p_mul(later, v);
+    }
+    if (partial_out != nullptr && lane == 0) {
+        double2* dst = reinterpret_cast<double2*>(partial_out) + 2 * (threadIdx.x >> 5);
+        dst[0] = make_double2(v.a.re, v.a.im);
+        dst[1] = make_double2(v.b.re, v.b.im);
+    }
+    if (product_out != nullptr) {
+        if (lane == 0) sh.warp_product[threadIdx.x >> 5] = v;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < kDmmaWarps; w++) v = su2p_mul(sh.warp_product[w], v);
+            if (D == 2) store_interval_operator<2>(v, product_out, 0);
+            else store_interval_operator<3>(v, product_out, 0);
         }
     }
 }
@@ -450,7 +554,7 @@ __device__ __noinline__ void dmma_tile_fallback(const MethodConfig& m, const Ins
 
 // Persistent launch: CTAs pull tiles of kDmmaTile intervals from the queue (or, without a queue, CTA
 // b takes tile b of a single instance).
-template <int DIMS>
+template <int DIMS, int PREC>
 SS_D void evolve_dmma_body(const EvolveArgs& a, DmmaShared& sh) {
     int64_t tile_id = blockIdx.x;
     if (a.tiles == nullptr) grid_dependency_wait();  // a single call: its descriptors come from dmma_consts_kernel
@@ -485,18 +589,19 @@ SS_D void evolve_dmma_body(const EvolveArgs& a, DmmaShared& sh) {
         double* u_out = a.u + inst.u_offset;
         float* norms_out = a.step_norms != nullptr ? a.step_norms + inst.out_offset : nullptr;
         const int dim = (DIMS == 0) ? inst.dim : DIMS;
-        if (tones_on_tensor_path(f, dim)) {
-            double* partial_out = nullptr;
-            if (a.tile_partials != nullptr) {
-                const int64_t k = (a.scan_begin != nullptr ? a.scan_begin[tile.instance] : 0) + tile.first / kScanTile;
-                partial_out = a.tile_partials + k * kScanMat;
-            }
-            const DmmaConsts* cst = a.dmma_consts != nullptr ? a.dmma_consts + tile.instance : nullptr;
+        if (PREC == PREC_FP64 || tones_on_tensor_path(f, dim)) {
+            const int64_t k = (a.scan_begin != nullptr ? a.scan_begin[tile.instance] : 0) + tile.first / kScanTile;
+            double* partial_out = a.tile_partials != nullptr ? a.tile_partials + k * kScanMat : nullptr;
+            double* product_out = a.tile_products != nullptr ? a.tile_products + k * kScanMat : nullptr;
             double* rows_out = a.rows != nullptr ? a.rows + 4 * inst.out_offset : nullptr;
-            tile_dmma<DIMS>(a.m, inst, f, tile, sh, time_out, u_out, norms_out, partial_out, cst, rows_out);
-        } else if (threadIdx.x < kDmmaTile) {  // one warp
-            const bool active = (int)threadIdx.x < tile.count;
-            dmma_tile_fallback<DIMS>(a.m, inst, f, tile.first + (active ? threadIdx.x : 0), active, time_out, u_out, norms_out);
+            tile_dmma<DIMS, PREC>(a.m, inst, f, tile, sh, time_out, u_out, norms_out, partial_out, product_out,
+                                  a.dmma_consts + tile.instance, rows_out);
+        } else if constexpr (PREC == PREC_FP32_BULK) {
+            if (threadIdx.x < kDmmaTile) {  // one warp
+                const bool active = (int)threadIdx.x < tile.count;
+                dmma_tile_fallback<DIMS>(a.m, inst, f, tile.first + (active ? threadIdx.x : 0), active, time_out, u_out,
+                                         norms_out);
+            }
         }
         __syncthreads();  // shared memory and the tile slot are reused by the next tile
         if (a.tile_counter == nullptr) return;
@@ -504,10 +609,10 @@ SS_D void evolve_dmma_body(const EvolveArgs& a, DmmaShared& sh) {
 }
 
 // MINB: minimum resident CTAs per SM for the register allocation (6: 80 registers, 5: 96, 4: 128, 3: 168).
-template <int DIMS, int MINB>
+template <int DIMS, int PREC, int MINB>
 __global__ void __launch_bounds__(kDmmaThreads, MINB) evolve_dmma_kernel(EvolveArgs a) {
     __shared__ DmmaShared sh;
-    evolve_dmma_body<DIMS>(a, sh);
+    evolve_dmma_body<DIMS, PREC>(a, sh);
 }
 
 }  // namespace spinsim
