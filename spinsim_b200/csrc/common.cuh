@@ -175,7 +175,15 @@ struct c64 {
 SS_HD c64 mk(double r, double i) { return c64{r, i}; }
 SS_HD c64 operator+(c64 a, c64 b) { return c64{a.re + b.re, a.im + b.im}; }
 SS_HD c64 operator-(c64 a, c64 b) { return c64{a.re - b.re, a.im - b.im}; }
-SS_HD c64 operator*(c64 a, c64 b) { return c64{a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re}; }
+// On the device one product is rounded and the other fused, always the same one: left to the compiler, the
+// choice would depend on the surrounding code, and results would differ between kernels of one computation.
+SS_HD c64 operator*(c64 a, c64 b) {
+#ifdef __CUDA_ARCH__
+    return c64{__fma_rn(a.re, b.re, -__dmul_rn(a.im, b.im)), __fma_rn(a.re, b.im, __dmul_rn(a.im, b.re))};
+#else
+    return c64{a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re};
+#endif
+}
 SS_HD c64 operator*(double s, c64 a) { return c64{s * a.re, s * a.im}; }
 SS_HD c64 conj(c64 a) { return c64{a.re, -a.im}; }
 // a * b + c

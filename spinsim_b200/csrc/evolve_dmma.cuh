@@ -81,6 +81,7 @@ struct __align__(16) DmmaShared {
     double2 z[kDmmaRecurrences];   // exp(i w delta) of each recurrence at its next pair
     double2 rot[kToneSlots];       // exp(i w dt)
     double2 middle[kToneSlots];    // exp(i w delta) at the middle step's samples
+    double w[kToneSlots];          // the tones' frequencies
     Su2p warp_product[kDmmaWarps];
     int32_t tile;
     int32_t magnus;                // 1: the tile takes the one-exponential Magnus step
@@ -190,10 +191,16 @@ SS_D double time_rounding(double t0, double dt_out, double i) {
     return -(__dadd_rn(__dsub_rn(t0, __dsub_rn(s, b)), __dsub_rn(p, b)) + ep);
 }
 
+template <bool B>
+struct Flag {
+    static constexpr bool value = B;
+};
+
 // One step's element from its samples in units of h / 2, FP32-bulk: the Magnus step or the reference's CF4
 // (I:655-686).
-SS_D Su2d dmma_step32(const double* sa, const double* sb, bool magnus, float* nsq) {
-    if (magnus) {
+template <bool MAGNUS>
+SS_D Su2d dmma_step32(const double* sa, const double* sb, float* nsq) {
+    if constexpr (MAGNUS) {
         // g = (h / 2)(b1 + b2) + (sqrt3 h^2 / 12) b2 x b1, with (h / 2) b in sa, sb: the linear part
         // g_lin = sa + sb stays FP64; the commutator (sqrt3 / 6) d x g_lin, d = (h / 2)(b2 - b1), and
         // the exponential's remainder are FP32.
@@ -215,14 +222,15 @@ SS_D Su2d dmma_step32(const double* sa, const double* sb, bool magnus, float* ns
         rest.beta.im = fmaf(-0.5f, cx, rest.beta.im);
         *nsq = fmaf(gl[0], gl[0], fmaf(gl[1], gl[1], fmaf(gl[2], gl[2], *nsq)));
         return su2_split(gl64[0], gl64[1], gl64[2], rest);
-    }
-    double ga[3], gb[3];
+    } else {
+        double ga[3], gb[3];
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-        ga[c] = fma(kDmmaW0, sa[c], kDmmaW1 * sb[c]);
-        gb[c] = fma(kDmmaW1, sa[c], kDmmaW0 * sb[c]);
+        for (int c = 0; c < 3; c++) {
+            ga[c] = fma(kDmmaW0, sa[c], kDmmaW1 * sb[c]);
+            gb[c] = fma(kDmmaW1, sa[c], kDmmaW0 * sb[c]);
+        }
+        return su2_cf4_element(ga, gb, nsq);
     }
-    return su2_cf4_element(ga, gb, nsq);
 }
 
 // The quad's four lanes hold products of consecutive pair segments; lane 0 of the quad gets the whole product:
@@ -278,8 +286,7 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
 
     // L of every tone at the middle of every interval of the tile (buffer 1 of the table holds it until the first
     // refill): thread 4 slot + quarter evaluates interval 8 quarter once and steps to the next seven intervals
-    // with exp(i w dt_out), corrected for the rounding of each interval's start (a phase of w times it, below
-    // 1e-10, so to first order).
+    // with exp(i w dt_out).
     double2* lval = reinterpret_cast<double2*>(&sh.table[1][0][0]);  // [slot][interval of the tile]
     static_assert(sizeof(sh.table[1]) >= sizeof(double2) * kToneSlots * kDmmaTile, "L table fits one buffer");
     if (threadIdx.x < 4 * kToneSlots) {
@@ -300,33 +307,35 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
             l = c64{half_dt * amp * cs, half_dt * amp * sn} * h;
             gstep = h * h;
         }
-        const double first = time_rounding(inst.t0, dt_out, (double)i0);
+        if (quarter == 0) sh.w[slot] = w;
 #pragma unroll
         for (int r = 0; r < kDmmaRows; r++) {
-            const double turn = w * (time_rounding(inst.t0, dt_out, (double)(i0 + r)) - first);
-            lval[slot * kDmmaTile + kDmmaRows * quarter + r] = make_double2(fma(-turn, l.im, l.re), fma(turn, l.re, l.im));
+            lval[slot * kDmmaTile + kDmmaRows * quarter + r] = make_double2(l.re, l.im);
             l = l * gstep;
         }
     }
     __syncthreads();  // producer phasors, rotations, step choice and L in place
 
-    // A operands: L of this lane's interval for tone 4 s + q, its imaginary part for the even sums, real for the odd
+    // A operands: L of this lane's interval for tone 4 s + q, its imaginary part for the even sums, real for the
+    // odd; corrected (a phase below 1e-10, so to first order) for how the interval's start is rounded, relative to
+    // the warp's first interval, whose phase was taken at its rounded start
+    const int64_t first_index = inst.interval0 + tile.first + kDmmaRows * (threadIdx.x >> 5);
+    const double late = time_rounding(inst.t0, dt_out, (double)(first_index + g)) - time_rounding(inst.t0, dt_out, (double)first_index);
     double even_a[3][2], odd_a[3][2];
 #pragma unroll
     for (int c = 0; c < 3; c++)
 #pragma unroll
         for (int s = 0; s < 2; s++) {
             const double2 lv = lval[(c * kBulkTones + 4 * s + q) * kDmmaTile + row];
-            even_a[c][s] = active ? lv.y : 0.0;
-            odd_a[c][s] = active ? lv.x : 0.0;
+            const double turn = late * sh.w[c * kBulkTones + 4 * s + q];
+            even_a[c][s] = active ? fma(turn, lv.x, lv.y) : 0.0;
+            odd_a[c][s] = active ? fma(-turn, lv.y, lv.x) : 0.0;
         }
-    // Rotating frame (I:823-829): Bz at the middle of the interval, sum_k Im L_zk + bias; lane q sums tones
-    // 2 q, 2 q + 1 and the quad adds the four parts.  prw: P times the frame's rate (for either spin).
+    // Rotating frame (I:823-829): Bz at the middle of the interval, sum_k Im L_zk + bias, over the quad's
+    // tones.  prw: P times the frame's rate (for either spin).
     double prw = 0.0;
     if (m.rotating) {
-        double part = 0.0;
-#pragma unroll
-        for (int k = 2 * q; k < 2 * q + 2; k++) part += lval[(2 * kBulkTones + k) * kDmmaTile + row].y;
+        double part = even_a[2][0] + even_a[2][1];
         part += __shfl_xor_sync(0xffffffffu, part, 1);
         part += __shfl_xor_sync(0xffffffffu, part, 2);
         prw = f.bias[2] + part / half_dt;
@@ -335,8 +344,8 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
     // -P rw (I:582-618), added once here instead of to every sample
     double bias[3];
 #pragma unroll
-    for (int c = 0; c < 3; c++) bias[c] = half_dt * f.bias[c];
-    bias[2] -= half_dt * prw;
+    for (int c = 0; c < 3; c++) bias[c] = __dmul_rn(half_dt, f.bias[c]);
+    bias[2] = __fma_rn(-half_dt, prw, bias[2]);
     // Frame phasors at the Gauss points of this segment's steps after the middle: exp(-i P rw delta); those of
     // the mirrored steps before it are their conjugates
     const double start = (double)seg_start + (K & 1 ? 0.5 : 0.0);
@@ -370,7 +379,6 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
     Su2d after = Su2d{c64{0.0, 0.0}, c64{0.0, 0.0}};   // this lane's steps after the middle
     Su2d before = Su2d{c64{0.0, 0.0}, c64{0.0, 0.0}};  // and their mirrored steps before it
     float nsq = 0.0f;  // sum of |g|^2 over this lane's steps (the error statement's scale)
-    const bool magnus = sh.magnus != 0;
     const bool lie_trotter = D == 3 || m.expo_half == EXPO_LIE_TROTTER;
     // An xy sample in the rotating frame (I:582-618; z: in the bias)
     auto rotate = [&](double* s, c64 w) {
@@ -379,10 +387,10 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
         s[1] = x.im;
     };
     // p <- step p (a step after p's), or p step (a mirrored step, before p's)
-    auto apply = [&](Su2d& p, double* sa, double* sb, bool mirrored) {
+    auto apply = [&](auto magnus, Su2d& p, double* sa, double* sb, bool mirrored) {
         Su2d e;
         if constexpr (PREC == PREC_FP32_BULK) {
-            e = dmma_step32(sa, sb, magnus, &nsq);
+            e = dmma_step32<decltype(magnus)::value>(sa, sb, &nsq);
         } else {  // the reference's CF4 (I:655-686) with FP64 exponentials
             double ga[3], gb[3];
 #pragma unroll
@@ -435,60 +443,66 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
                 rotate(sa, conj(w));
                 rotate(sb, w);
             }
-            apply(after, sa, sb, false);
+            if (PREC == PREC_FP32_BULK && sh.magnus != 0) apply(Flag<true>(), after, sa, sb, false);
+            else apply(Flag<false>(), after, sa, sb, false);
         }
     }
     __syncthreads();
     const int n_phases = (n_steps + kDmmaPhase - 1) / kDmmaPhase;
-    for (int ph = 0; ph < n_phases; ph++) {
-        if (ph + 1 < n_phases) fill(ph + 1);
-        const int m0 = ph * kDmmaPhase;
-        const int mc = min(kDmmaPhase, n_steps - m0);
-        const double* tb = &sh.table[ph & 1][0][lane];
-        // Even and odd sums at the two distances of pair mm (tensor path), issued at the end of pair mm - 1, so
-        // they are in flight while the next pair begins.
-        double e0[3], e1[3], o0[3], o1[3];
-        auto sums = [&](int mm) {
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                e0[c] = e1[c] = bias[c];
-                o0[c] = o1[c] = 0.0;
-                const double* t = tb + mm * kDmmaChunkDoubles + c * 128;
-#pragma unroll
-                for (int s = 0; s < 2; s++) {
-                    dmma_m8n8k4(e0[c], e1[c], even_a[c][s], t[32 * s]);
-                    dmma_m8n8k4(o0[c], o1[c], odd_a[c][s], t[64 + 32 * s]);
-                }
-            }
-        };
-        sums(0);
-        for (int mm = 0; mm < mc; mm++) {
-            if (active && m0 + mm < seg_len) {
-                double sa[3], sb[3], ma[3], mb[3];  // the step after the middle, and its mirror image
-#pragma unroll
+    // The step loop, one copy for each kind of step (both inside one loop do not fit the instruction cache).
+    auto steps = [&](auto magnus) {
+        for (int ph = 0; ph < n_phases; ph++) {
+            if (ph + 1 < n_phases) fill(ph + 1);
+            const int m0 = ph * kDmmaPhase;
+            const int mc = min(kDmmaPhase, n_steps - m0);
+            const double* tb = &sh.table[ph & 1][0][lane];
+            // Even and odd sums at the two distances of pair mm (tensor path), issued at the end of pair mm - 1, so
+            // they are in flight while the next pair begins.
+            double e0[3], e1[3], o0[3], o1[3];
+            auto sums = [&](int mm) {
+    #pragma unroll
                 for (int c = 0; c < 3; c++) {
-                    sa[c] = e0[c] + o0[c];
-                    sb[c] = e1[c] + o1[c];
-                    ma[c] = e1[c] - o1[c];
-                    mb[c] = e0[c] - o0[c];
+                    e0[c] = e1[c] = bias[c];
+                    o0[c] = o1[c] = 0.0;
+                    const double* t = tb + mm * kDmmaChunkDoubles + c * 128;
+    #pragma unroll
+                    for (int s = 0; s < 2; s++) {
+                        dmma_m8n8k4(e0[c], e1[c], even_a[c][s], t[32 * s]);
+                        dmma_m8n8k4(o0[c], o1[c], odd_a[c][s], t[64 + 32 * s]);
+                    }
                 }
-                if (m.rotating) {
-                    rotate(sa, wa);
-                    rotate(sb, wb);
-                    rotate(ma, conj(wb));
-                    rotate(mb, conj(wa));
-                    wa = wa * wrot;
-                    wb = wb * wrot;
+            };
+            sums(0);
+            for (int mm = 0; mm < mc; mm++) {
+                if (active && m0 + mm < seg_len) {
+                    double sa[3], sb[3], ma[3], mb[3];  // the step after the middle, and its mirror image
+    #pragma unroll
+                    for (int c = 0; c < 3; c++) {
+                        sa[c] = e0[c] + o0[c];
+                        sb[c] = e1[c] + o1[c];
+                        ma[c] = e1[c] - o1[c];
+                        mb[c] = e0[c] - o0[c];
+                    }
+                    if (m.rotating) {
+                        rotate(sa, wa);
+                        rotate(sb, wb);
+                        rotate(ma, conj(wb));
+                        rotate(mb, conj(wa));
+                        wa = wa * wrot;
+                        wb = wb * wrot;
+                    }
+                    apply(magnus, after, sa, sb, false);
+                    apply(magnus, before, ma, mb, true);
                 }
-                apply(after, sa, sb, false);
-                apply(before, ma, mb, true);
+                // the next pair's sums, issued after this pair's arithmetic (all lanes: mma.sync is
+                // warp-collective); measured 0.7% faster than issuing them before it
+                if (mm + 1 < mc) sums(mm + 1);
             }
-            // the next pair's sums, issued after this pair's arithmetic (all lanes: mma.sync is
-            // warp-collective); measured 0.7% faster than issuing them before it
-            if (mm + 1 < mc) sums(mm + 1);
+            __syncthreads();  // buffer (ph & 1) is refilled in phase ph + 1
         }
-        __syncthreads();  // buffer (ph & 1) is refilled in phase ph + 1
-    }
+    };
+    if (PREC == PREC_FP32_BULK && sh.magnus != 0) steps(Flag<true>());
+    else steps(Flag<false>());
 
     // The interval's product, in lane 0 of the quad
     combine_segments<false>(after, q);
