@@ -187,6 +187,19 @@ class Results:
         self.__dict__["_keep"] = keep
         self.__dict__["_error"] = error
 
+    @classmethod
+    def _from_block(cls, block, spin_calculator, keep, error):
+        """Results in one device block (``_Block``); its tensor views are made on first use."""
+        self = cls.__new__(cls)
+        self.__dict__.update(_dev=None, _block=block, spin_calculator=spin_calculator, _keep=keep, _error=error)
+        return self
+
+    def _device(self):
+        dev = self.__dict__["_dev"]
+        if dev is None:
+            dev = self.__dict__["_dev"] = self.__dict__["_block"].tensors()
+        return dev
+
     @property
     def error_estimate(self):
         """Stated error of ``state`` against the FP64 form (max over entries and output steps of the
@@ -202,11 +215,15 @@ class Results:
     @property
     def device_arrays(self):
         """The torch device tensors behind the results (no copy)."""
-        return dict(self.__dict__["_dev"])
+        return dict(self._device())
 
     def __getattr__(self, name):
-        dev = self.__dict__["_dev"]
         if name in Results._ARRAYS:
+            if self.__dict__["_dev"] is None:
+                # no tensor of it has been handed out: one copy brings all four arrays
+                self.__dict__.update(self.__dict__["_block"].host_arrays())
+                return self.__dict__[name]
+            dev = self._device()
             if name in dev:
                 value = _to_numpy(dev[name])
             elif name == "spin":
@@ -219,6 +236,55 @@ class Results:
             self.__dict__[name] = value
             return value
         raise AttributeError("{} has no attribute called {}.".format(self, name))
+
+
+class _Block:
+    """One device allocation for a small call's outputs (time, U, state, spin), step norms and workspace, as
+    16-byte words: its layout, addresses and views.  Pieces start at multiples of 256 bytes, the outputs first.
+    Reading any of the arrays on the host copies all of them: at these sizes a copy is its latency (four reads
+    of a call of 100 output steps 72 -> 20 us)."""
+
+    SMALL = 1 << 20  # output bytes
+
+    __slots__ = ("words", "n", "d", "offsets", "norms_at", "ws_at")
+
+    def __init__(self, n, d, with_norms, ws_bytes, device):
+        import torch
+        self.n, self.d = n, d
+        at, offsets = 0, []
+        for nbytes in (8 * n, 16 * n * d * d, 16 * n * d, 24 * n):
+            offsets.append(at)
+            at += (nbytes + 255) // 256 * 16
+        self.offsets = offsets + [at]
+        self.norms_at = at if with_norms else None
+        if with_norms:
+            at += (4 * n + 255) // 256 * 16
+        self.ws_at = at
+        self.words = torch.empty(at + (ws_bytes + 15) // 16, dtype=torch.complex128, device=device)
+
+    def pointers(self):
+        base, (t, u, st, sp, _) = self.words.data_ptr(), self.offsets
+        return (base + 16 * t, base + 16 * u, base + 16 * st, base + 16 * sp,
+                None if self.norms_at is None else base + 16 * self.norms_at, base + 16 * self.ws_at)
+
+    def tensors(self):
+        import torch
+        n, d, (t, u, st, sp, _) = self.n, self.d, self.offsets
+        real = self.words.view(torch.float64)
+        return {"time": real.as_strided((n,), (1,), 2 * t),
+                "time_evolution": self.words.as_strided((n, d, d), (d * d, d, 1), u),
+                "state": self.words.as_strided((n, d), (d, 1), st), "spin": real.as_strided((n, 3), (3, 1), 2 * sp)}
+
+    def norms(self):
+        import torch
+        return self.words.view(torch.float32).as_strided((self.n,), (1,), 4 * self.norms_at)
+
+    def host_arrays(self):
+        n, d, (t, u, st, sp, end) = self.n, self.d, self.offsets
+        host = self.words[:end].cpu().numpy()
+        real = host.view(np.float64)
+        return {"time": real[2 * t:2 * t + n], "time_evolution": host[u:u + n * d * d].reshape(n, d, d),
+                "state": host[st:st + n * d].reshape(n, d), "spin": real[2 * sp:2 * sp + 3 * n].reshape(n, 3)}
 
 
 def _to_numpy(x):
@@ -234,6 +300,12 @@ def _to_numpy(x):
 
 
 # -------------------------------------------------------------------------------------- Simulator
+def _current_stream(device):
+    """The raw handle of torch's current stream on the device."""
+    import torch
+    return torch._C._cuda_getCurrentRawStream(device.index)
+
+
 def _cuda_device():
     import torch
     if not torch.cuda.is_available():
@@ -407,31 +479,40 @@ class Simulator:
             params = np.zeros(1)
         by_value = self._builtin is None and params.size <= _lib.MAX_CALL_PARAMS
         sweep = None if by_value or self._builtin is not None else torch.as_tensor(params, device=dev)
-        time = torch.empty(n, dtype=torch.float64, device=dev)
-        u = torch.empty((n, d, d), dtype=torch.complex128, device=dev)
-        state = torch.empty((n, d), dtype=torch.complex128, device=dev)
-        spin = torch.empty((n, 3), dtype=torch.float64, device=dev)
-        ws_bytes = self._lib.spinsim_evaluate_workspace_size(self._plan, n)
-        ws = torch.empty(max(ws_bytes, 256), dtype=torch.uint8, device=dev)
-        stream = torch.cuda.current_stream(dev).cuda_stream
         bulk = self.precision == Precision.FP32_BULK
-        norms = torch.zeros(max(n, 1), dtype=torch.float32, device=dev) if bulk else None
-        call = (float(time_start), float(dt_int), float(time_step_output), n, psi0.ctypes.data, time.data_ptr(),
-                u.data_ptr(), state.data_ptr(), spin.data_ptr(), norms.data_ptr() if bulk else None, ws.data_ptr(),
-                ws.numel(), stream)
+        ws_bytes = max(self._lib.spinsim_evaluate_workspace_size(self._plan, n), 256)
+        block = None
+        if n * (32 + 16 * d * (d + 1)) <= _Block.SMALL:
+            block = _Block(n, d, bulk, ws_bytes, dev)
+            pointers = block.pointers()
+        else:  # tensors of their own, so that a caller who keeps one of them keeps no more
+            time = torch.empty(n, dtype=torch.float64, device=dev)
+            u = torch.empty((n, d, d), dtype=torch.complex128, device=dev)
+            state = torch.empty((n, d), dtype=torch.complex128, device=dev)
+            spin = torch.empty((n, 3), dtype=torch.float64, device=dev)
+            norms = torch.empty(n, dtype=torch.float32, device=dev) if bulk else None
+            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
+            pointers = (time.data_ptr(), u.data_ptr(), state.data_ptr(), spin.data_ptr(),
+                        norms.data_ptr() if bulk else None, ws.data_ptr())
+        call = (float(time_start), dt_int, float(time_step_output), n, psi0.ctypes.data, *pointers, ws_bytes,
+                _current_stream(dev))
         if by_value:
             _lib.check(self._lib.spinsim_evaluate_params(self._plan, params.ctypes.data, params.size, *call))
         else:
             _lib.check(self._lib.spinsim_evaluate_with_norms(self._plan, ctypes.byref(self._field_struct(sweep)), *call))
         error = 0.0
         if bulk:
-            steps = n * int(math.floor(float(time_step_output) / float(dt_int) + 0.5))
-            bound = magnus_method_bound(self.get_field, dt_int, steps)
-            lt = self._lie_trotter_hypercubes()
+            field, lt = self.get_field, self._lie_trotter_hypercubes()
+            steps = n * int(math.floor(float(time_step_output) / dt_int + 0.5))
 
             def error():
-                return bulk_error_estimate(norms[:n].double().sum().item(), d, bound, steps, lt)
-        return Results(time, u, state, self.spin_calculator, spin=spin, keep=(sweep, ws, self._builtin), error=error)
+                sums = block.norms() if block is not None else norms
+                bound = magnus_method_bound(field, dt_int, steps)
+                return bulk_error_estimate(sums.double().sum().item(), d, bound, steps, lt)
+        keep = (sweep, self._builtin)
+        if block is not None:
+            return Results._from_block(block, self.spin_calculator, keep, error)
+        return Results(time, u, state, self.spin_calculator, spin=spin, keep=(*keep, ws), error=error)
 
     def spin_calculator(self, state):
         """get_spin / spin_calculator (I:899-988): Bloch vector of a state series, on the device."""

@@ -4,6 +4,7 @@ The library is built in-tree by ``spinsim_b200.build``.  There is no CPU fallbac
 is missing or fails to load, every entry point raises.
 """
 import ctypes
+import math
 import os
 import threading
 
@@ -153,7 +154,16 @@ def check(rc):
 
 
 def normalise_steps(t0, t1, dt_int, dt_out):
-    """(dt_int', N, K, warned) of Simulator.evaluate's step normalisation (spinsim/__init__.py:1025-1034)."""
+    """(dt_int', N, K, warned) of Simulator.evaluate's step normalisation (spinsim/__init__.py:1025-1034), as
+    ``spinsim_normalise_steps`` computes it (Python's round is round-half-to-even too)."""
+    t0, t1, dt_int, dt_out = float(t0), float(t1), float(dt_int), float(dt_out)
+    if dt_int > 0.0 and dt_out > 0.0:
+        ratio = dt_out / dt_int
+        n = (t1 - t0) / dt_out
+        if ratio < 1e9 and n < 1e18:  # finite, within the integers' range
+            steps = round(ratio)
+            dti = dt_out / (steps if ratio > 1.0 else 1)
+            return dti, int(n) if n > 0.0 else 0, math.floor(dt_out / dti + 0.5), abs(ratio - steps) > 1e-6
     d = c_dbl()
     n = c_i64()
     k = c_i32()
