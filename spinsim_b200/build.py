@@ -92,10 +92,11 @@ DMMA_MINB = {1: (3, 4, 5, 6), 0: (3, 4, 5)}
 
 
 def user_minb(v):
-    """Resident CTAs a user-field kernel's register allocation must allow: four (128 registers; the
-    spin-one Rabi sweep's time evolution 179 -> 131 us against 208 registers and two CTAs), except for
-    the eight-generator exponential, whose 3 x 3 temporaries would spill in its inner loop."""
-    return 2 if v[3] == 2 else 4
+    """Resident CTAs a user-field kernel's register allocation must allow: five for spin half (96 registers; the
+    pulse ensemble's time evolution 2709 -> 2637 us against four CTAs), four with spin one (128; the
+    spin-one Rabi sweep's 179 -> 131 us against 208 registers and two CTAs), except for the
+    eight-generator exponential, whose 3 x 3 temporaries would spill in its inner loop."""
+    return 2 if v[3] == 2 else 5 if v[0] == 2 else 4
 
 
 def gen_sources():

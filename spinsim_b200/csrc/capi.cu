@@ -427,13 +427,14 @@ struct Carver {
 
 // Lanes per output interval.  A lane's chain is its start-up (frame sample and phasors), its share of the
 // fine steps and one product per level of the lanes' combination; the launch takes that chain's latency
-// while the FP64 pipes have room (up to about four warps per scheduler at a chain's own parallelism) and
+// while the FP64 pipes have room (up to about two warps per scheduler at a chain's own parallelism) and
 // its throughput beyond.  The lane count with the least of that is taken, in units of FP64 operations.
-// Measured: 4001 x 50 steps with a quadratic shift 35 us at 16 lanes and 62 at 32; 100,000 x 10 steps 35 us at 1.
+// Measured (whole calls): 4001 x 50 steps with a quadratic shift 36 / 33 / 39 / 48 us at 4 / 8 / 16 / 32 lanes,
+// 5003 x 37 of a cubic waveform 49 / 33 / 40 / 44, 100,000 x 10 of a drive 59 / 64 us at 1 / 2.
 int pick_lanes(const spinsim_plan* p, int64_t intervals, int max_fine) {
     if (p->lockstep) return 1;
     if (p->m.lanes) return p->m.lanes;
-    const double start = 300.0, step = 200.0, level = 60.0, saturated = 4.0;
+    const double start = 300.0, step = 200.0, level = 60.0, saturated = 2.0;
     double best = 0.0;
     int lanes = 1;
     for (int l = 1, levels = 0; l <= 32 && l <= std::max(1, max_fine); l *= 2, levels++) {

@@ -39,40 +39,54 @@ struct Su2d {
     c64 am1, beta;
 };
 
-// cos(r/2) - 1 and sin(r/2) / r from r^2: even Taylor series for r <= 1/2 (the first omitted terms
-// are below 2^-56 of the leading ones; no square root, division or argument reduction), else sincos.
-SS_D void su2_exp_factors(double r2, double* c, double* s) {
+// Series coefficients of the step loops, in constant memory: a multiply-add then takes its coefficient as an
+// operand, where a literal costs two moves into registers every time (the loops have no registers to
+// keep them in).  Half the pulse ensemble's instructions were not FP64 ones.
+static __constant__ double kCosHalf[6] = {-0.125, 1.0 / 384.0, -1.0 / 46080.0, 1.0 / 10321920.0, -1.0 / 3715891200.0,
+                                          1.0 / 1961990553600.0};  // (-1)^k / ((2k)! 4^k), k = 1 ...
+static __constant__ double kSinHalf[6] = {0.5, -1.0 / 48.0, 1.0 / 3840.0, -1.0 / 645120.0, 1.0 / 185794560.0,
+                                          -1.0 / 81749606400.0};   // (-1)^k / (2 (2k+1)! 4^k), k = 0 ...
+static __constant__ double kInvFact[16] = {1.0,
+                                           1.0,
+                                           1.0 / 2.0,
+                                           1.0 / 6.0,
+                                           1.0 / 24.0,
+                                           1.0 / 120.0,
+                                           1.0 / 720.0,
+                                           1.0 / 5040.0,
+                                           1.0 / 40320.0,
+                                           1.0 / 362880.0,
+                                           1.0 / 3628800.0,
+                                           1.0 / 39916800.0,
+                                           1.0 / 479001600.0,
+                                           1.0 / 6227020800.0,
+                                           1.0 / 87178291200.0,
+                                           1.0 / 1307674368000.0};
+
+// matrix_exponential_analytic (I:1618-1642): exp of -i(x Jx + y Jy + z Jz), minus one, with r2 = |(x, y, z)|^2:
+// alpha - 1 = cos(r/2) - 1 - i z s, beta = (y - i x) s, s = sin(r/2) / r.  Even Taylor series for r <= 1/2 (the first
+// omitted terms are below 2^-56 of the leading ones; no square root, division or argument reduction), else
+// sincos.  Not a number: the identity, as the reference's "r > 0" test gives (I:1626).
+SS_D Su2d su2_exp_m1(double x, double y, double z, double r2) {
+    double c, s;
     if (r2 <= 0.25) {
-        double a = 1.0 / 1961990553600.0;               //  1 / (12! 4^6)
-        a = fma(a, r2, -1.0 / 3715891200.0);            // -1 / (10! 4^5)
-        a = fma(a, r2, 1.0 / 10321920.0);               //  1 / (8! 4^4)
-        a = fma(a, r2, -1.0 / 46080.0);                 // -1 / (6! 4^3)
-        a = fma(a, r2, 1.0 / 384.0);                    //  1 / (4! 4^2)
-        a = fma(a, r2, -0.125);                         // -1 / (2! 4)
-        *c = a * r2;
-        double b = -1.0 / 81749606400.0;                // -1 / (2 11! 4^5)
-        b = fma(b, r2, 1.0 / 185794560.0);              //  1 / (2 9! 4^4)
-        b = fma(b, r2, -1.0 / 645120.0);                // -1 / (2 7! 4^3)
-        b = fma(b, r2, 1.0 / 3840.0);                   //  1 / (2 5! 4^2)
-        b = fma(b, r2, -1.0 / 48.0);                    // -1 / (2 3! 4)
-        *s = fma(b, r2, 0.5);
+        c = kCosHalf[5];
+        s = kSinHalf[5];
+#pragma unroll
+        for (int k = 4; k >= 0; k--) {
+            c = fma(c, r2, kCosHalf[k]);
+            s = fma(s, r2, kSinHalf[k]);
+        }
+        c *= r2;
     } else if (r2 > 0.0) {
         const double r = sqrt(r2);
         double s4, c4;
         sincos(0.25 * r, &s4, &c4);
-        *c = -2.0 * (s4 * s4);
-        *s = 2.0 * s4 * c4 / r;
-    } else {  // not a number: the identity, as the reference's "r > 0" test gives (I:1626)
-        *c = 0.0;
-        *s = 0.0;
+        c = -2.0 * (s4 * s4);
+        s = 2.0 * s4 * c4 / r;
+    } else {
+        return Su2d{c64{0.0, 0.0}, c64{0.0, 0.0}};
     }
-}
-
-// matrix_exponential_analytic (I:1618-1642): exp of -i(x Jx + y Jy + z Jz), minus one.
-SS_D Su2d su2_exp_m1(double x, double y, double z, double r2) {
-    double c, s;
-    su2_exp_factors(r2, &c, &s);
-    if (!(r2 > 0.0)) return Su2d{c64{0.0, 0.0}, c64{0.0, 0.0}};
     return Su2d{c64{c, -z * s}, c64{y * s, -x * s}};
 }
 
@@ -216,22 +230,6 @@ SS_D Mat<3> spin_one_exp_m1_64(double x, double y, double z, double q) {
     }
     const double d = (2.0 / 3.0) * q * (fma(z, z, -0.5 * a2) - q * q * (1.0 / 9.0));
     // (-i)^n / n! times the coefficients (al, be, ga) of H^n, summed into f0, f1, f2
-    constexpr double inv_fact[16] = {1.0,
-                                     1.0,
-                                     1.0 / 2.0,
-                                     1.0 / 6.0,
-                                     1.0 / 24.0,
-                                     1.0 / 120.0,
-                                     1.0 / 720.0,
-                                     1.0 / 5040.0,
-                                     1.0 / 40320.0,
-                                     1.0 / 362880.0,
-                                     1.0 / 3628800.0,
-                                     1.0 / 39916800.0,
-                                     1.0 / 479001600.0,
-                                     1.0 / 6227020800.0,
-                                     1.0 / 87178291200.0,
-                                     1.0 / 1307674368000.0};
     c64 f0 = c64{0.0, 0.0}, f1 = c64{0.0, -1.0}, f2 = c64{-0.5, 0.0};  // n = 1 and n = 2
     double al = 0.0, be = 0.0, ga = 1.0;                                 // of H^2
     auto term = [&](int n) {                                             // H^n = H H^(n-1)
@@ -239,15 +237,16 @@ SS_D Mat<3> spin_one_exp_m1_64(double x, double y, double z, double q) {
         al = na;
         be = nb;
         ga = ng;
-        const double c = ((n & 3) == 0 || (n & 3) == 3) ? inv_fact[n] : -inv_fact[n];
+        const double c = kInvFact[n];
+        const bool plus = (n & 3) == 0 || (n & 3) == 3;
         if (n & 1) {  // (-i)^3 = i, (-i)^5 = -i
-            f0.im = fma(c, al, f0.im);
-            f1.im = fma(c, be, f1.im);
-            f2.im = fma(c, ga, f2.im);
+            f0.im = plus ? fma(c, al, f0.im) : fma(-c, al, f0.im);
+            f1.im = plus ? fma(c, be, f1.im) : fma(-c, be, f1.im);
+            f2.im = plus ? fma(c, ga, f2.im) : fma(-c, ga, f2.im);
         } else {
-            f0.re = fma(c, al, f0.re);
-            f1.re = fma(c, be, f1.re);
-            f2.re = fma(c, ga, f2.re);
+            f0.re = plus ? fma(c, al, f0.re) : fma(-c, al, f0.re);
+            f1.re = plus ? fma(c, be, f1.re) : fma(-c, be, f1.re);
+            f2.re = plus ? fma(c, ga, f2.re) : fma(-c, ga, f2.re);
         }
     };
 #pragma unroll
