@@ -522,7 +522,7 @@ class Batch:
 class Evaluator:
     """Evaluate lists of instances into host memory with the stages overlapped.
 
-    The list is split into ``chunks`` contiguous groups of about equal output bytes.  Group k's host set-up
+    The list is split into up to ``chunks`` contiguous groups of about equal output bytes.  Group k's host set-up
     (descriptors, field packing into pinned staging), uploads and kernels run while group k-1's
     outputs are copied to pinned host memory, one copy per group; uploads, kernels and copies have
     a stream each.  The copies are usually the longest stage (every output crosses PCIe), so the
@@ -533,6 +533,10 @@ class Evaluator:
     list, otherwise a group may pick other lanes or a single-spin kernel and the results agree to
     rounding.
     """
+
+    # A group's set-up and launches (about 0.2 ms) hide the copy of about this many bytes of the group before;
+    # smaller groups only add launches (a dozen instances, 9 MB: eight groups 2.0 ms, one 0.6 ms).
+    GROUP_BYTES = 12 << 20
 
     def __init__(self, chunks=8, **batch_kwargs):
         import torch
@@ -554,7 +558,7 @@ class Evaluator:
     def groups(self, instances):
         """Contiguous (first, end) groups of about equal output bytes, since the device-to-host copies
         are the longest stage: about (t1 - t0) / dt_out output steps, spin one weighted 224 / 128 (the
-        bytes of time, U, state and spin per output step)."""
+        bytes of time, U, state and spin per output step).  At most ``chunks``, of at least GROUP_BYTES each."""
         n = len(instances)
         if not n:
             return []
@@ -567,9 +571,10 @@ class Evaluator:
         one = np.fromiter(map(spin_one.__contains__, ids), np.bool_, n)
         work = np.maximum((t1 - t0) / dt_out, 1.0) * np.where(one, 224.0 / 128.0, 1.0)
         cum = np.cumsum(work)
+        chunks = min(self.chunks, max(1, int(128.0 * cum[-1] / self.GROUP_BYTES)))
         cuts = [0]
-        for g in range(1, self.chunks):
-            k = int(np.searchsorted(cum, cum[-1] * g / self.chunks))
+        for g in range(1, chunks):
+            k = int(np.searchsorted(cum, cum[-1] * g / chunks))
             if k > cuts[-1]:
                 cuts.append(k)
         cuts.append(n)
