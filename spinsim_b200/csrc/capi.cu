@@ -603,13 +603,13 @@ int launch_scan_short(const ScanArgs& a, int32_t dim, cudaStream_t s) {
 }
 
 // The tile prefixes: a warp per instance, or, where some instance has many tiles, a cluster per instance
-// with about four tiles per thread of the longest (fewer CTAs where that would be many of them).  A warp
+// with about two tiles per thread of the longest (fewer CTAs where that would be many of them).  A warp
 // takes 1.1 us for each 32 tiles of the longest instance from SU(2) partials, and 1.7 or 3 us from 2 x 2 or
 // 3 x 3 products; a cluster kernel takes about 6 us and 0.5 us for each tile of its longest thread, in waves
 // of three CTAs per SM (one of 6250 tiles 165 -> 10 us).  The shorter of the two is launched.
 int launch_prefix(const ScanArgs& a, const ScanBuffers& b, const bool* has_dim, int sm, cudaStream_t s) {
     unsigned c = 1;
-    while (c < (unsigned)kClusterMax && (int64_t)c * 4 * kClusterThreads < b.max_tiles &&
+    while (c < (unsigned)kClusterMax && (int64_t)c * 2 * kClusterThreads < b.max_tiles &&
            (int64_t)2 * c * b.n_instances <= 16 * (int64_t)sm)
         c *= 2;
     const double per_chunk = a.partials ? 1.1 : has_dim[1] ? 3.0 : 1.7;

@@ -316,7 +316,7 @@ static __constant__ double kCosSmall[8] = {-0.5,           1.0 / 24.0,          
 
 // sin x and cos x: for |x| <= 1/2 by their Taylor series (terms to x^15 and x^16, coefficients 1/n!;
 // the first omitted terms are below 2e-17 there, and the results agree with sin and cos to one
-// rounding), else by sincos.  For the small per-interval frame phases of the tensor path.
+// rounding), else by sincos.  For the frame's phases within an interval, which are mostly small.
 SS_D void sincos_small(double x, double* s, double* c) {
     if (fabs(x) <= 0.5) {
         const double y = x * x;

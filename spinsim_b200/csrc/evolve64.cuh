@@ -38,6 +38,19 @@ SS_D void transform_frame_lt8(double* s, double rw, c64 w) {
 // (about one rounding a step) stays far below the phase's own argument rounding.
 constexpr int kPhasorSteps = 64;
 
+struct PhasorPair {
+    c64 a, b;
+};
+
+// exp(i x) and exp(i y).  Out of line: the step loops restart their phasors so rarely that its code and registers
+// should not be theirs.
+__attribute__((const)) inline __device__ __noinline__ PhasorPair phasor_pair(double x, double y) {
+    PhasorPair p;
+    sincos_small(x, &p.a.im, &p.a.re);
+    sincos_small(y, &p.b.im, &p.b.re);
+    return p;
+}
+
 // Where an interval's steps sample the field and how they weight the samples: the interval's start, the
 // reference's sample offsets and weights of an integrator for steps of dt (I:624-686 Magnus CF4 at the two
 // Gauss points, I:693-752 Heun at the step's ends, I:759-791 Euler at its middle).  A sample's time is t_c + tau
@@ -78,8 +91,9 @@ struct Steps : StepRule {
 
     template <int INTEG>
     SS_D void start_phasors() {
-        sincos(-prw * tau(off_a), &wa.im, &wa.re);
-        if (INTEG != INTEG_EULER) sincos(-prw * tau(off_b), &wb.im, &wb.re);
+        const PhasorPair p = phasor_pair(-prw * tau(off_a), INTEG != INTEG_EULER ? -prw * tau(off_b) : 0.0);
+        wa = p.a;
+        wb = p.b;
     }
     // Steps from number `first` of an interval that starts at t (steps: how many it has; 0: none).
     template <int INTEG>
@@ -89,7 +103,7 @@ struct Steps : StepRule {
         rotating = m.rotating;
         wa = wb = wrot = c64{1.0, 0.0};
         if (m.rotating && steps > 0 && prw != 0.0) {
-            sincos(-prw * dt, &wrot.im, &wrot.re);
+            sincos_small(-prw * dt, &wrot.im, &wrot.re);
             start_phasors<INTEG>();
         }
 #pragma unroll
@@ -240,7 +254,7 @@ SS_D Mat<3> interval_lt8(const MethodConfig& m, const FieldDesc& f, double t_c, 
 template <int D>
 SS_D void leave_frame(Su2p& v, double rw, double dt_out) {
     c64 w;  // spin one, whose representation doubles the phase: half of it
-    sincos(rw * dt_out * (D == 2 ? 1.0 : 0.5), &w.im, &w.re);
+    sincos_small(rw * dt_out * (D == 2 ? 1.0 : 0.5), &w.im, &w.re);
     v.a = v.a * conj(w);
     v.b = v.b * w;
 }

@@ -95,7 +95,7 @@ SS_D Su2d su2_exp_m1(double x, double y, double z, double r2) {
 // factor is an SU(2) rotation by 2 theta, cos theta = cos A cos Z and sin theta (axis) =
 // (sin A, cos A sin Z) with A = a / 2N, Z = z / 2N, so its N-th power is the rotation by 2 N theta.
 // Out of line: the steps that need it are those too large for their N (su2_step_element64).
-inline __device__ __noinline__ Su2d su2_lie_trotter_m1(double x, double y, double z, double n) {
+__attribute__((const)) inline __device__ __noinline__ Su2d su2_lie_trotter_m1(double x, double y, double z, double n) {
     const double a = sqrt(x * x + y * y);
     c64 ep = c64{1.0, 0.0};
     if (a > 0) {

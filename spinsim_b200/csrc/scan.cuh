@@ -426,9 +426,11 @@ __global__ void __launch_bounds__(kClusterThreads) scan_prefix_cluster_kernel(co
         if (a.partials) return su2p_to_mat<D>(tile_product_of(load_partials(a, k, true)));
         return load_mat<D>(a.tile_product + k * kScanMat);
     };
-    Mat<D> m;
-    set_identity(m);
-    for (int64_t k = k0; k < k1; k++) m = matmul(tile_of(k), m);
+    Mat<D> m, first;  // the thread's first tile is kept for the second pass
+    set_identity(first);
+    if (k0 < k1) first = tile_of(k0);
+    m = first;
+    for (int64_t k = k0 + 1; k < k1; k++) m = matmul(tile_of(k), m);
     m = warp_scan<D>(m, lane);
     if (lane == 31) sh.warp_total[w] = m;
     m = shfl_up_mat(m, 1);
@@ -446,7 +448,7 @@ __global__ void __launch_bounds__(kClusterThreads) scan_prefix_cluster_kernel(co
     m = matmul(m, sh.warp_enter[w]);
     for (int64_t k = k0; k < k1; k++) {
         store_mat<D>(a.tile_prefix + k * kScanMat, m);
-        m = matmul(tile_of(k), m);
+        if (k + 1 < k1 || a.total != nullptr) m = matmul(k == k0 ? first : tile_of(k), m);
     }
     if (a.total != nullptr && k0 < k1 && k1 == e) store_mat<D>(a.total + (int64_t)i * 2 * D * D, m);
     cluster_wait();
