@@ -318,11 +318,10 @@ extern "C" int spinsim_plan_create(const spinsim_plan_desc* desc, const void* fi
         // largest that fits max_registers: 6 -> 80, 5 -> 96, 4 -> 128, 3 -> 168 registers, 2 uncapped.
         // Budgets of 80 and 96 exist only for some kernels; without one the next larger budget is taken.
         // By default 128, except for the eight-generator exponential, whose 3 x 3 temporaries would
-        // spill, and 96 for FP32-bulk tables, bound by latency: a launch of 400 pulse trains takes 723 us
-        // at 168, 637 at 128, 568 at 96 and 512 at 80, where an interpolated table's steps spill too much.
+        // spill: a launch of 400 pulse trains (FP32-bulk tables) takes 677 us at 168, 564 at 128, 561 at 96
+        // and 519 at 80, where an interpolated table's steps spill too much.
         const int mr = d.max_registers;
-        const bool bulk_table = d.field_kind == SPINSIM_FIELD_TABLE && d.precision == SPINSIM_PRECISION_FP32_BULK;
-        const int want_minb = mr <= 0 ? (eo == EXPO_LIE_TROTTER_8 ? 2 : bulk_table ? 5 : 4) : mr <= 80 ? 6 : mr <= 96 ? 5 : mr <= 128 ? 4 : mr <= 168 ? 3 : 2;
+        const int want_minb = mr <= 0 ? (eo == EXPO_LIE_TROTTER_8 ? 2 : 4) : mr <= 80 ? 6 : mr <= 96 ? 5 : mr <= 128 ? 4 : mr <= 168 ? 3 : 2;
         for (int minb = want_minb; minb >= 2 && !p->func; minb--) {
             for (const BuiltinEntry& b : kBuiltin) {
                 if (b.dims == d.spin_dim && b.integ == d.integration && b.expo_h == eh && b.expo_o == eo &&

@@ -306,7 +306,65 @@ __device__ __noinline__ SpinOneProduct spin_one_quadratic_steps32(const FieldDes
     return SpinOneProduct{u, nsq};
 }
 
-// Every lane of the warp calls this, as interval64 (whose DIMS and step loop these are).
+// Steps j0 .. j1 - 1 of an interval, one after another.  nsq accumulates |g|^2 (the error statement's scale).
+// Phase 1: every step an SU(2) element (spin half always; spin one while the quadratic shift is zero), the product
+// an FP64 SU(2) element; software-pipelined: the next step's field samples (independent FP64 work) are issued
+// next to this step's exponentials and product.  Phase 2 (spin one with a quadratic shift): full 3x3
+// exponentials and an FP64 3x3 product.
+template <int DIMS, int INTEG, int FIELD>
+SS_D StepsResult steps32(const MethodConfig& m, const FieldDesc& f, const StepRule& rule, double prw, int dim, int j0, int j1) {
+    constexpr int L = LieDim<DIMS, EXPO_LIE_TROTTER>::value;
+    Steps<L> st(rule);
+    st.template begin<INTEG>(m, prw, j0, j1 - j0);
+    auto next_generators = [&](double* ga, double* gb) { step_generators<FIELD, L, INTEG>(f, st, ga, gb); };
+    StepsResult r;
+    r.p = Su2d{c64{0.0, 0.0}, c64{0.0, 0.0}};
+    r.nsq = 0.0f;
+    r.quadratic = false;
+    double ga[4] = {0.0, 0.0, 0.0, 0.0}, gb[4] = {0.0, 0.0, 0.0, 0.0};
+    int j = j0;
+    if (j < j1) next_generators(ga, gb);
+    for (; j < j1; j++) {
+        if (DIMS != 2 && dim == 3 && (ga[3] != 0.0 || gb[3] != 0.0)) {
+            r.quadratic = true;
+            break;
+        }
+        double na[4] = {0.0, 0.0, 0.0, 0.0}, nb[4] = {0.0, 0.0, 0.0, 0.0};
+        if (j + 1 < j1) next_generators(na, nb);
+        if constexpr (INTEG == INTEG_EULER) su2_apply64(r.p, su2_euler_element(ga, &r.nsq));
+        else su2_apply64(r.p, su2_cf4_element(ga, gb, &r.nsq));
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            ga[k] = na[k];
+            gb[k] = nb[k];
+        }
+    }
+    if constexpr (DIMS != 2) {
+        if (r.quadratic) {
+            Generators4 g;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                g.a[k] = ga[k];
+                g.b[k] = gb[k];
+            }
+            const SpinOneProduct q = spin_one_quadratic_steps32<INTEG, FIELD>(
+                f, st, su2_to_spin_one(c64{1.0 + r.p.am1.re, r.p.am1.im}, r.p.beta), g, j, j1, r.nsq);
+            r.u = q.u;
+            r.nsq = q.nsq;
+        }
+    }
+    return r;
+}
+
+// For table fields out of line: their cursors' registers would otherwise be the piecewise constant path's too
+// (400 pulse trains 550 -> 603 us when the cursors grew by four doubles a channel).
+template <int DIMS, int INTEG, int FIELD>
+__device__ __noinline__ StepsResult steps32_call(const MethodConfig& m, const FieldDesc& f, StepRule rule, double prw, int dim,
+                                                 int j0, int j1) {
+    return steps32<DIMS, INTEG, FIELD>(m, f, rule, prw, dim, j0, j1);
+}
+
+// Every lane of the warp calls this, as interval64 (whose DIMS these are).
 template <int DIMS, int INTEG, int FIELD>
 SS_D void interval32(const MethodConfig& m, const Instance& inst, const FieldDesc& f, int64_t index, bool active,
                      int lane_in_group, double* time_out, double* u_out, float* norms_out, double* product_out) {
@@ -321,69 +379,27 @@ SS_D void interval32(const MethodConfig& m, const Instance& inst, const FieldDes
     const int K = active ? inst.n_fine : 0;
     const int j0 = (int)(((int64_t)K * lane_in_group) / lanes);
     const int j1 = (int)(((int64_t)K * (lane_in_group + 1)) / lanes);
-
     const StepRule rule = step_rule<INTEG>(t_c, dt);
-    Steps<L> st(rule);
-    auto next_generators = [&](double* ga, double* gb) { step_generators<FIELD, L, INTEG>(f, st, ga, gb); };
-
-    // Phase 1: every step an SU(2) element (spin half always; spin one while the quadratic shift
-    // is zero); the interval product is an FP64 SU(2) element.  Software-pipelined: the next step's
-    // field samples (independent FP64 work) are issued next to this step's exponentials and product.
-    Su2d su2 = Su2d{c64{0.0, 0.0}, c64{0.0, 0.0}};
-    double ga[4] = {0.0, 0.0, 0.0, 0.0}, gb[4] = {0.0, 0.0, 0.0, 0.0};
-    float nsq = 0.0f;  // sum of |g|^2 over this lane's steps (the error statement's scale)
-    int j = j0;
-    bool pending = false;
-    auto quadratic_step = [&]() { return DIMS != 2 && dim == 3 && (ga[3] != 0.0 || gb[3] != 0.0); };
+    StepsResult r;
     if constexpr (FIELD == FIELD_TABLE) {
+        r.p = Su2d{c64{0.0, 0.0}, c64{0.0, 0.0}};
+        r.nsq = 0.0f;
+        r.quadratic = false;
         auto element = [&](const double* a, const double* b, int n) {
             float step = 0.0f;
             const Su2d e = INTEG == INTEG_EULER ? su2_euler_element(a, &step) : su2_cf4_element(a, b, &step);
-            nsq = fmaf((float)n, step, nsq);
+            r.nsq = fmaf((float)n, step, r.nsq);
             return e;
         };
-        if (hold_steps<INTEG>(f, dim, m.rotating && prw != 0.0, rule, j0, j1, dt_out, su2, element)) j = j1;
+        if (!hold_steps<INTEG>(f, dim, m.rotating && prw != 0.0, rule, j0, j1, dt_out, r.p, element))
+            r = steps32_call<DIMS, INTEG, FIELD>(m, f, rule, prw, dim, j0, j1);
+    } else {
+        r = steps32<DIMS, INTEG, FIELD>(m, f, rule, prw, dim, j0, j1);
     }
-    if (j < j1) {
-        st.template begin<INTEG>(m, prw, j0, K);
-        next_generators(ga, gb);
-    }
-    for (; j < j1; j++) {
-        if (quadratic_step()) {
-            pending = true;
-            break;
-        }
-        double na[4] = {0.0, 0.0, 0.0, 0.0}, nb[4] = {0.0, 0.0, 0.0, 0.0};
-        if (j + 1 < j1) next_generators(na, nb);
-        if constexpr (INTEG == INTEG_EULER) su2_apply64(su2, su2_euler_element(ga, &nsq));
-        else su2_apply64(su2, su2_cf4_element(ga, gb, &nsq));
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            ga[k] = na[k];
-            gb[k] = nb[k];
-        }
-    }
-    // Phase 2 (spin one with a quadratic shift): full 3x3 exponentials and an FP64 3x3 product.
-    // The pending step's generators are in ga, gb.
-    Mat<3> u;
-    if constexpr (DIMS != 2) {
-        if (pending) {
-            Generators4 g;
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                g.a[k] = ga[k];
-                g.b[k] = gb[k];
-            }
-            const SpinOneProduct r = spin_one_quadratic_steps32<INTEG, FIELD>(
-                f, st, su2_to_spin_one(c64{1.0 + su2.am1.re, su2.am1.im}, su2.beta), g, j, j1, nsq);
-            u = r.u;
-            nsq = r.nsq;
-        }
-    }
-    for (int s = 1; s < lanes; s <<= 1) nsq += __shfl_down_sync(0xffffffffu, nsq, s);
+    for (int s = 1; s < lanes; s <<= 1) r.nsq += __shfl_down_sync(0xffffffffu, r.nsq, s);
     const bool writes = active && lane_in_group == 0;
-    if (writes && norms_out != nullptr) norms_out[index] = nsq;
-    finish_steps<DIMS>(m, dim, su2, u, pending, lanes, lane_in_group, rw, dt_out, writes, t_c, index, time_out, u_out,
+    if (writes && norms_out != nullptr) norms_out[index] = r.nsq;
+    finish_steps<DIMS>(m, dim, r.p, r.u, r.quadratic, lanes, lane_in_group, rw, dt_out, writes, t_c, index, time_out, u_out,
                        product_out);
 }
 

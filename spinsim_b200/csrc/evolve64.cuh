@@ -160,7 +160,7 @@ struct Generators4 {
 // squarings; a step with a knot between its samples is a run of its own.  element(ga, gb, n) is the element of
 // n steps of these generators.  False, with nothing done, unless every lane of the warp (which all call
 // this) can take this form.  Bound by latency (the knots' search and the runs' divergence).  A launch of 400
-// pulse trains (4.1e6 output steps of 20, FP32-bulk, 96 registers): 1806 -> 568 us.
+// pulse trains (4.1e6 output steps of 20, FP32-bulk, 128 registers): 1704 -> 564 us.
 template <int INTEG, typename Element>
 SS_D bool hold_steps(const FieldDesc& f, int dim, bool turns, const StepRule& st, int j0, int j1, double dt_out, Su2d& p,
                      Element element) {
@@ -359,6 +359,50 @@ SS_D void finish_steps(const MethodConfig& m, int dim, const Su2d& p, Mat<3>& u,
         finish_interval<3>(m, pair, rw, dt_out, writes, t_c, index, time_out, u_out, product_out);
 }
 
+// The product of an interval's steps: an SU(2) element p, or, where a step with a quadratic shift was met (spin
+// one), the 3 x 3 operator u; FP32-bulk: the sum of |g|^2.
+struct StepsResult {
+    Su2d p;
+    Mat<3> u;
+    float nsq;
+    bool quadratic;
+};
+
+// Steps j0 .. j1 - 1 of an interval, one after another.
+template <int DIMS, int INTEG, bool LT_HALF, int FIELD>
+SS_D StepsResult steps64(const MethodConfig& m, const FieldDesc& f, const StepRule& rule, double prw, int dim, int j0, int j1) {
+    constexpr int L = LieDim<DIMS, EXPO_LIE_TROTTER>::value;
+    const bool lie_trotter = dim == 3 || LT_HALF;
+    Steps<L> st(rule);
+    st.template begin<INTEG>(m, prw, j0, j1 - j0);
+    StepsResult r;
+    r.p = Su2d{c64{0.0, 0.0}, c64{0.0, 0.0}};
+    r.quadratic = false;
+    for (int j = j0; j < j1; j++) {
+        Generators4 g;
+        if (j != j0) st.template restart<INTEG>(j, j0);
+        step_generators<FIELD, L, INTEG>(f, st, g.a, g.b);
+        if constexpr (DIMS != 2) {
+            if (dim == 3 && (g.a[3] != 0.0 || (INTEG != INTEG_EULER && g.b[3] != 0.0))) {
+                r.quadratic = true;
+                r.u = spin_one_quadratic_steps64<INTEG, FIELD>(
+                    m, f, st, su2_to_spin_one(c64{1.0 + r.p.am1.re, r.p.am1.im}, r.p.beta), g, j0, j, j1);
+                break;
+            }
+        }
+        su2_apply64(r.p, su2_step_element64(m, lie_trotter, g.a));
+        if constexpr (INTEG != INTEG_EULER) su2_apply64(r.p, su2_step_element64(m, lie_trotter, g.b));
+    }
+    return r;
+}
+
+// For table fields out of line, so that their cursors' registers are not the piecewise constant path's too.
+template <int DIMS, int INTEG, bool LT_HALF, int FIELD>
+__device__ __noinline__ StepsResult steps64_call(const MethodConfig& m, const FieldDesc& f, StepRule rule, double prw, int dim,
+                                                 int j0, int j1) {
+    return steps64<DIMS, INTEG, LT_HALF, FIELD>(m, f, rule, prw, dim, j0, j1);
+}
+
 // Evolve one output interval.  Every lane of the warp must call this (shuffles use the full mask);
 // lanes with `active == false` do no steps and write nothing.
 //
@@ -393,39 +437,25 @@ SS_D void interval64(const MethodConfig& m, const Instance& inst, const FieldDes
         combine_lanes(u, lanes, lane_in_group);
         finish_interval<3>(m, u, rw, dt_out, writes, t_c, index, time_out, u_out, product_out);
     } else {
-        const bool lie_trotter = dim == 3 || EXPO_H == EXPO_LIE_TROTTER;
+        constexpr bool kLieTrotterHalf = EXPO_H == EXPO_LIE_TROTTER;
         const StepRule rule = step_rule<INTEG>(t_c, dt);
-        Su2d p = Su2d{c64{0.0, 0.0}, c64{0.0, 0.0}};
-        Mat<3> u;
-        bool quadratic = false;  // a step with a quadratic shift was met: the product is in u
-        bool held = false;
+        StepsResult r;
         if constexpr (FIELD == FIELD_TABLE) {
+            r.p = Su2d{c64{0.0, 0.0}, c64{0.0, 0.0}};
+            r.quadratic = false;
             auto element = [&](const double* ga, const double* gb, int) {
+                const bool lie_trotter = dim == 3 || kLieTrotterHalf;
                 Su2d e = su2_step_element64(m, lie_trotter, ga);
                 if constexpr (INTEG != INTEG_EULER) su2_apply64(e, su2_step_element64(m, lie_trotter, gb));
                 return e;
             };
-            held = hold_steps<INTEG>(f, dim, m.rotating && prw != 0.0, rule, j0, j1, dt_out, p, element);
+            if (!hold_steps<INTEG>(f, dim, m.rotating && prw != 0.0, rule, j0, j1, dt_out, r.p, element))
+                r = steps64_call<DIMS, INTEG, kLieTrotterHalf, FIELD>(m, f, rule, prw, dim, j0, j1);
+        } else {
+            r = steps64<DIMS, INTEG, kLieTrotterHalf, FIELD>(m, f, rule, prw, dim, j0, j1);
         }
-        Steps<L> st(rule);
-        if (!held) st.template begin<INTEG>(m, prw, j0, K);
-        for (int j = j0; !held && j < j1; j++) {
-            Generators4 g;
-            if (j != j0) st.template restart<INTEG>(j, j0);
-            step_generators<FIELD, L, INTEG>(f, st, g.a, g.b);
-            if constexpr (DIMS != 2) {
-                if (dim == 3 && (g.a[3] != 0.0 || (INTEG != INTEG_EULER && g.b[3] != 0.0))) {
-                    quadratic = true;
-                    u = spin_one_quadratic_steps64<INTEG, FIELD>(
-                        m, f, st, su2_to_spin_one(c64{1.0 + p.am1.re, p.am1.im}, p.beta), g, j0, j, j1);
-                    break;
-                }
-            }
-            su2_apply64(p, su2_step_element64(m, lie_trotter, g.a));
-            if constexpr (INTEG != INTEG_EULER) su2_apply64(p, su2_step_element64(m, lie_trotter, g.b));
-        }
-        finish_steps<DIMS>(m, dim, p, u, quadratic, lanes, lane_in_group, rw, dt_out, writes, t_c, index, time_out, u_out,
-                           product_out);
+        finish_steps<DIMS>(m, dim, r.p, r.u, r.quadratic, lanes, lane_in_group, rw, dt_out, writes, t_c, index, time_out,
+                           u_out, product_out);
     }
 }
 
