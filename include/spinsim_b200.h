@@ -93,7 +93,7 @@ typedef struct {
  * handed to the user's get_field. */
 typedef struct {
     const double* params;
-    int64_t n_params;
+    int64_t n_params;       /* how many; FIELD_TONES: the largest |w| rounded up, or 0 where it is not known */
     const spinsim_table* tables; /* device array [8] */
     const double* tones;         /* device array */
     int32_t tone_start[8];

@@ -829,7 +829,7 @@ static int evaluate_impl(const spinsim_plan* p, const spinsim_field* field, doub
     Instance inst;
     rc = make_instance(p, t0, dt_int, dt_out, n_out, psi0, &inst);
     if (rc) return rc;
-    if (p->tensor && tones_on_tensor_path(*reinterpret_cast<const FieldDesc*>(field), inst.dim)) p = p->tensor;
+    if (p->tensor && tones_on_fp64_tensor_path(*reinterpret_cast<const FieldDesc*>(field), inst)) p = p->tensor;
     if (n_out == 0) return SPINSIM_OK;
     if (!time || !u || (with_scan && !state)) return fail(SPINSIM_ERR_INVALID, "output pointer is null");
     if (with_scan && !psi0) return fail(SPINSIM_ERR_INVALID, "psi0 is null");
@@ -1212,7 +1212,11 @@ extern "C" int64_t spinsim_pack_fields(int32_t n_fields, const int64_t* plan, in
         if (h[0] == 2) {  // tones
             const int64_t n = h[5];
             if (n < 0 || at + n > host_doubles) return fail(SPINSIM_ERR_WORKSPACE, "staging too small for field %d", f);
-            if (n) memcpy(host + at, reinterpret_cast<const double*>(h[4]), (size_t)n * sizeof(double));
+            const double* tones = reinterpret_cast<const double*>(h[4]);
+            if (n) memcpy(host + at, tones, (size_t)n * sizeof(double));
+            double rate = 1.0;
+            for (int64_t k = 0; k + 2 < n; k += 3) rate = std::max(rate, fabs(tones[k]));
+            out.n_params = rate < 1e18 ? (int64_t)ceil(rate) : (int64_t)1e18;
             const int32_t* counts = reinterpret_cast<const int32_t*>(h[6]);
             for (int c = 0; c < 8; c++) {
                 out.tone_start[c] = counts[c];
@@ -1320,7 +1324,7 @@ static int batch_prepare(const spinsim_plan* plan, const spinsim_instance* insta
         std::vector<char> on_path;  // FP64 tones: which instances the tensor path takes
         if (plan->tensor)
             for (int i = 0; i < n_instances; i++)
-                on_path.push_back(tones_on_tensor_path(reinterpret_cast<const FieldDesc*>(fields)[inst[i].field], inst[i].dim));
+                on_path.push_back(tones_on_fp64_tensor_path(reinterpret_cast<const FieldDesc*>(fields)[inst[i].field], inst[i]));
         std::vector<Tile> evolve_tiles, tensor_tiles, scan_tiles;
         std::vector<int32_t> begin, end;
         Tile *et, *tt, *stl;

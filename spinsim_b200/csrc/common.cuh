@@ -46,7 +46,7 @@ struct TableChannel {
 // FIELD_USER ignores everything but params/n_params, which go to the linked get_field().
 struct FieldDesc {
     const double* params;          // sweep parameters for a user get_field (device)
-    int64_t n_params;
+    int64_t n_params;              // how many; FIELD_TONES: the largest |w|, rounded up (0: not given)
     const TableChannel* tables;    // [kMaxChannels] (FIELD_TABLE)
     const double* tones;           // FIELD_TONES: (w, A, phi) triples, channel after channel
     int32_t tone_start[kMaxChannels];
@@ -152,6 +152,19 @@ SS_HD bool tones_on_tensor_path(const FieldDesc& f, int dim) {
     for (int c = 0; c < 3; c++)
         if (f.tone_count[c] > kBulkTones) return false;
     return !(dim == 3 && (f.bias[3] != 0.0 || f.tone_count[3] > 0));
+}
+// In FP64 also none whose phase w t grows beyond kToneMaxPhase: there the rounding of the reference's sample times,
+// which the per-sample form repeats and these products do not, shows in the operators (at 1.7e5 rad, 27 ms of 1 MHz
+// tones, states 4e-10 apart; at 6e4 rad, 1e-11).  A tone field's n_params is its largest |w|, rounded up; 0, not
+// given, counts as kToneDefaultRate.
+constexpr double kToneMaxPhase = 1e5;
+constexpr double kToneDefaultRate = 1e7;
+SS_HD bool tones_on_fp64_tensor_path(const FieldDesc& f, const Instance& inst) {
+    const double rate = f.n_params > 0 ? (double)f.n_params : kToneDefaultRate;
+    const double first = inst.t0 + inst.dt_out * (double)inst.interval0, last = first + inst.dt_out * (double)inst.n_out;
+    const double far = (first < 0 ? -first : first) > (last < 0 ? -last : last) ? (first < 0 ? -first : first)
+                                                                              : (last < 0 ? -last : last);
+    return rate * far <= kToneMaxPhase && tones_on_tensor_path(f, inst.dim);
 }
 constexpr int kSynthIntervals = 2;          // output intervals per lane, 32 intervals apart
 // Slot-fastest layouts: a warp's 16-byte stores and loads of one quantity for all slots are

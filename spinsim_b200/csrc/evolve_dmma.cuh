@@ -42,8 +42,9 @@
 // tones on a channel, or spin one with a quadratic shift, take the per-interval path (interval32,
 // CF4) inside the same kernel.
 //
-// Step, FP64.  CF4 with the two FP64 exponentials of evolve64.cuh.  Instances the products do not take run in
-// that file's kernel instead (the host splits the batch's tiles).
+// Step, FP64.  CF4 with the two FP64 exponentials of evolve64.cuh.  Instances the products do not take, and those
+// whose tones' phases are large (tones_on_fp64_tensor_path), run in that file's kernel instead (the host splits the
+// batch's tiles).
 //
 // Scan partials.  A CTA tile is one state scan tile (scan.cuh).  Each interval's lab-frame operator is
 // an SU(2) pair (spin one: its representation), so each warp also multiplies its eight rows' pairs
@@ -317,19 +318,27 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
     __syncthreads();  // producer phasors, rotations, step choice and L in place
 
     // A operands: L of this lane's interval for tone 4 s + q, its imaginary part for the even sums, real for the
-    // odd; corrected (a phase below 1e-10, so to first order) for how the interval's start is rounded, relative to
-    // the warp's first interval, whose phase was taken at its rounded start
-    const int64_t first_index = inst.interval0 + tile.first + kDmmaRows * (threadIdx.x >> 5);
-    const double late = time_rounding(inst.t0, dt_out, (double)(first_index + g)) - time_rounding(inst.t0, dt_out, (double)first_index);
+    // odd; in FP64 corrected (a phase below 1e-10, so to first order) for how the interval's start is rounded,
+    // relative to the warp's first interval, whose phase was taken at its rounded start
+    double late = 0.0;
+    if constexpr (PREC == PREC_FP64) {
+        const int64_t first_index = inst.interval0 + tile.first + kDmmaRows * (threadIdx.x >> 5);
+        late = time_rounding(inst.t0, dt_out, (double)(first_index + g)) - time_rounding(inst.t0, dt_out, (double)first_index);
+    }
     double even_a[3][2], odd_a[3][2];
 #pragma unroll
     for (int c = 0; c < 3; c++)
 #pragma unroll
         for (int s = 0; s < 2; s++) {
             const double2 lv = lval[(c * kBulkTones + 4 * s + q) * kDmmaTile + row];
-            const double turn = late * sh.w[c * kBulkTones + 4 * s + q];
-            even_a[c][s] = active ? fma(turn, lv.x, lv.y) : 0.0;
-            odd_a[c][s] = active ? fma(-turn, lv.y, lv.x) : 0.0;
+            if constexpr (PREC == PREC_FP64) {
+                const double turn = late * sh.w[c * kBulkTones + 4 * s + q];
+                even_a[c][s] = active ? fma(turn, lv.x, lv.y) : 0.0;
+                odd_a[c][s] = active ? fma(-turn, lv.y, lv.x) : 0.0;
+            } else {
+                even_a[c][s] = active ? lv.y : 0.0;
+                odd_a[c][s] = active ? lv.x : 0.0;
+            }
         }
     // Rotating frame (I:823-829): Bz at the middle of the interval, sum_k Im L_zk + bias, over the quad's
     // tones.  prw: P times the frame's rate (for either spin).
