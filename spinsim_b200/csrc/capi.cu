@@ -12,7 +12,9 @@
 #include <string.h>
 
 #include <algorithm>
+#include <list>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -157,6 +159,48 @@ int jit_link(const void* kernel_fatbin, size_t kernel_size, const void* user_lto
     if (g_jl.cubin(h, cubin->data()) != 0) return log_fail("reading the linked cubin failed");
     g_jl.destroy(&h);
     return SPINSIM_OK;
+}
+
+// The last kernels linked, by everything that goes into a link (the built-in kernel's image, the register cap and
+// the field's whole LTO-IR), most recent first: another plan of the same field, which a program that makes a
+// simulator per call asks for, takes a copy. Even from its disk cache nvJitLink needs milliseconds, more the
+// larger the kernel's image. At most kLinkedKept entries.
+struct Linked {
+    const void* kernel;
+    int max_registers;
+    std::string field;
+    std::vector<char> cubin;
+};
+constexpr size_t kLinkedKept = 8;
+std::mutex g_linked_mutex;
+std::list<Linked> g_linked;
+
+int linked_cubin(const void* kernel_fatbin, size_t kernel_size, const void* user_ltoir, size_t user_size,
+                 int max_registers, std::vector<char>* cubin) {
+    try {
+        const std::string field((const char*)user_ltoir, user_size);
+        auto is_this = [&](const Linked& k) {
+            return k.kernel == kernel_fatbin && k.max_registers == max_registers && k.field == field;
+        };
+        {
+            std::lock_guard<std::mutex> lock(g_linked_mutex);
+            auto at = std::find_if(g_linked.begin(), g_linked.end(), is_this);
+            if (at != g_linked.end()) {
+                g_linked.splice(g_linked.begin(), g_linked, at);
+                *cubin = at->cubin;
+                return SPINSIM_OK;
+            }
+        }
+        const int rc = jit_link(kernel_fatbin, kernel_size, user_ltoir, user_size, max_registers, cubin);
+        if (rc) return rc;
+        std::lock_guard<std::mutex> lock(g_linked_mutex);
+        if (std::none_of(g_linked.begin(), g_linked.end(), is_this))
+            g_linked.push_front(Linked{kernel_fatbin, max_registers, field, *cubin});
+        if (g_linked.size() > kLinkedKept) g_linked.pop_back();
+        return SPINSIM_OK;
+    } catch (const std::bad_alloc&) {
+        return fail(SPINSIM_ERR_LINK, "out of host memory while linking the user field");
+    }
 }
 }  // namespace
 
@@ -338,7 +382,7 @@ extern "C" int spinsim_plan_create(const spinsim_plan_desc* desc, const void* fi
                 u = &x;
         if (u) {
             std::vector<char> cubin;
-            int rc = jit_link(u->begin, (size_t)(u->end - u->begin), field_ltoir, field_ltoir_size, d.max_registers, &cubin);
+            int rc = linked_cubin(u->begin, (size_t)(u->end - u->begin), field_ltoir, field_ltoir_size, d.max_registers, &cubin);
             if (rc) {
                 delete p;
                 return rc;
