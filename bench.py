@@ -73,23 +73,23 @@ def instances(ss, specs):
 
 
 # Algorithmic work per integration step, counted from the kernels' arithmetic (a fused multiply-add
-# is 2 flops; sin, cos, sqrt and division count 1 each).  Plain FP64, spin half: field 192 + 48 sin,
-# windings 8 + 4 sincos, frame 24, generators 24, two analytic exponentials 40 + 8, two 2x2 complex
-# products 128, time 1.  Spin one (Lie-Trotter, 24 squarings): field 192 + 48, windings 8 + 4,
-# frame 14, generators 32, two exponentials 10,920 + 14, two 3x3 products 432, time 1.  FP32-bulk
-# (tensor-path tone kernel, Magnus step): field samples 192 as FP64 tensor-core products (two Gauss
-# points x three channels x 16 multiply-adds) + the phasor table's recurrences 9, frame 24 (the xy
-# rotations and the phasors' steps; z's frame shift is in the samples' starting value), sum and
-# difference of the samples 6, the exponential's linear part and the SU(2) product into the
-# interval's FP64 operator 39; in FP32 the commutator 15 and the exponential's O(|g|^2) remainder 21.
-# Spin one runs as SU(2) (no quadratic shift here).
-FLOPS_FP64_PLAIN = {2: 417 + 60, 3: 11600 + 66}
-FLOPS_BULK = {2: {"fp64": 270, "fp32": 36}, 3: {"fp64": 270, "fp32": 36}}
+# is 2 flops).  Both forms sample the tones on the FP64 tensor path, with each interval's samples as
+# even and odd sums about its middle: 96 (two Gauss points x three channels x 8 multiply-adds, one
+# product for two mirrored samples), their sum and difference 6, the phasor table's recurrences 4,
+# frame 24 (the xy rotations and the phasors' steps; z's frame shift is in the samples' starting
+# value).  Plain FP64 adds two CF4 generators 18, their squared norms 10, two SU(2) exponentials
+# from series 48, and their two products into the interval's operator 72; FP32-bulk the samples' sum
+# and difference 6, the exponential's linear part and the SU(2) product 39, and in FP32 the
+# commutator 15 and the exponential's O(|g|^2) remainder 21.  Spin one runs as SU(2) in both (no
+# quadratic shift here).
+FLOPS_FP64_PLAIN = {2: 278, 3: 278}
+FLOPS_BULK = {2: {"fp64": 175, "fp32": 36}, 3: {"fp64": 175, "fp32": 36}}
 # DRAM bytes (read + write) of one full-size FP32-bulk time-evolution launch of this workload (the
 # tensor-path kernel at 96 registers, writing the scan's tile partials and each output step's SU(2)
 # pair beside U: 46 MB of the writes are that scan scratch, not outputs), from one capture of
 # `ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none -k regex:evolve_dmma -c 1`
 # on `bench.py --workload profile --profile-size full --precision fp32_bulk --max-registers 96 --variant 0`.
+# The capture is of the kernel with 192 sample flops per step; what it reads and writes has not changed since.
 TRAFFIC_BYTES_PER_LAUNCH = 7328000 + 137223936
 
 
@@ -233,9 +233,7 @@ def cpu_sample(specs, seconds_target=8.0, n_threads=0):
 # ------------------------------------------------------------------------------------ our arm
 class PerSpinBatches:
     """The plain FP64 form run as one launch per spin (spin half and spin one, each with its own
-    autotuned register budget and launch shape), on two streams: a mixed-spin FP64 launch carries the
-    register budget and code of the spin-one Lie-Trotter path into the spin-half steps, so splitting by
-    spin is the faster way to run this batch in FP64."""
+    autotuned register budget and launch shape), on two streams."""
 
     def __init__(self, ss, insts, plans, tune):
         import torch
@@ -418,9 +416,8 @@ def bench_ours(args, world, rank):
                        "fp64_tflops": fp64_plain_flops / float(np.mean(t_evolve_plain)) / 1e12,
                        "fp64_frac": fp64_plain_flops / float(np.mean(t_evolve_plain)) / 1e12 / measured_fp64_peak()["tflops"],
                        "per_spin": plain_parts,
-                       "flop_count": "sin, cos, sqrt and division count 1 flop each; a spin-half step's 60 "
-                                     "transcendental calls (48 of them the tone field) keep the FP64 pipe busy far "
-                                     "longer than their flop count"},
+                       "flop_count": "a fused multiply-add is 2 flops; both spins step as SU(2), their samples as "
+                                     "FP64 tensor-path products"},
         "speedup_vs_fp64": t_plain_total / t_bulk_total,
         "state_err": {"max": float(errs.max()), "p50": float(np.median(errs)), "p99": float(np.percentile(errs, 99)),
                       "tolerance": 1e-6, "vs": "plain FP64 form, final state state[N-1] per instance"},
