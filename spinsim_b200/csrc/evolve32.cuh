@@ -288,12 +288,12 @@ struct SpinOneProduct {
 // and an FP64 3x3 product, from the product u of the steps before.  On entry step j's generators are
 // in g and st is at step j + 1.  Out of line (and with its state passed by value), so that the
 // registers of the common SU(2) loop are allocated without this path's.
-template <int INTEG, int FIELD, bool FAR>
+template <int INTEG, int FIELD>
 __device__ __noinline__ SpinOneProduct spin_one_quadratic_steps32(const FieldDesc& f, Steps<4> st, Mat<3> u,
                                                                   Generators4 g, int j, int j1, float nsq) {
     bool first = true;
     for (; j < j1; j++) {
-        if (!first) step_generators<FIELD, 4, INTEG, false, FAR>(f, st, g.a, g.b);
+        if (!first) step_generators<FIELD, 4, INTEG, false>(f, st, g.a, g.b);
         first = false;
         if constexpr (INTEG == INTEG_EULER) spin_one_euler_step(u, g.a, &nsq);
         else spin_one_cf4_step(u, g.a, g.b, &nsq);
@@ -306,12 +306,12 @@ __device__ __noinline__ SpinOneProduct spin_one_quadratic_steps32(const FieldDes
 // an FP64 SU(2) element; software-pipelined: the next step's field samples (independent FP64 work) are issued
 // next to this step's exponentials and product.  Phase 2 (spin one with a quadratic shift): full 3x3
 // exponentials and an FP64 3x3 product.
-template <int DIMS, int INTEG, int FIELD, bool FAR>
+template <int DIMS, int INTEG, int FIELD>
 SS_D StepsResult steps32(const MethodConfig& m, const FieldDesc& f, const StepRule& rule, double prw, int dim, int j0, int j1) {
     constexpr int L = LieDim<DIMS, EXPO_LIE_TROTTER>::value;
     Steps<L> st(rule);
-    st.template begin<INTEG, FAR>(m, prw, j0, j1 - j0);
-    auto next_generators = [&](double* ga, double* gb) { step_generators<FIELD, L, INTEG, false, FAR>(f, st, ga, gb); };
+    st.template begin<INTEG>(m, prw, j0, j1);
+    auto next_generators = [&](double* ga, double* gb) { step_generators<FIELD, L, INTEG, false>(f, st, ga, gb); };
     StepsResult r;
     r.p = Su2d{c64{0.0, 0.0}, c64{0.0, 0.0}};
     r.nsq = 0.0f;
@@ -342,7 +342,7 @@ SS_D StepsResult steps32(const MethodConfig& m, const FieldDesc& f, const StepRu
                 g.a[k] = ga[k];
                 g.b[k] = gb[k];
             }
-            const SpinOneProduct q = spin_one_quadratic_steps32<INTEG, FIELD, FAR>(
+            const SpinOneProduct q = spin_one_quadratic_steps32<INTEG, FIELD>(
                 f, st, su2_to_spin_one(c64{1.0 + r.p.am1.re, r.p.am1.im}, r.p.beta), g, j, j1, r.nsq);
             r.u = q.u;
             r.nsq = q.nsq;
@@ -353,10 +353,10 @@ SS_D StepsResult steps32(const MethodConfig& m, const FieldDesc& f, const StepRu
 
 // For table fields out of line: their cursors' registers would otherwise be the piecewise constant path's too
 // (400 pulse trains 550 -> 603 us when the cursors grew by four doubles a channel).
-template <int DIMS, int INTEG, int FIELD, bool FAR>
+template <int DIMS, int INTEG, int FIELD>
 __device__ __noinline__ StepsResult steps32_call(const MethodConfig& m, const FieldDesc& f, StepRule rule, double prw, int dim,
                                                  int j0, int j1) {
-    return steps32<DIMS, INTEG, FIELD, FAR>(m, f, rule, prw, dim, j0, j1);
+    return steps32<DIMS, INTEG, FIELD>(m, f, rule, prw, dim, j0, j1);
 }
 
 // Every lane of the warp calls this, as interval64 (whose DIMS these are).
@@ -386,16 +386,10 @@ SS_D void interval32(const MethodConfig& m, const Instance& inst, const FieldDes
             r.nsq = fmaf((float)n, step, r.nsq);
             return e;
         };
-        if (hold_steps<INTEG>(f, dim, m.rotating && prw != 0.0, rule, j0, j1, dt_out, r.p, element)) {
-        } else if (far_from_zero(rule)) {
-            r = steps32_call<DIMS, INTEG, FIELD, true>(m, f, rule, prw, dim, j0, j1);
-        } else {
-            r = steps32_call<DIMS, INTEG, FIELD, false>(m, f, rule, prw, dim, j0, j1);
-        }
-    } else if (FIELD == FIELD_TONES || far_from_zero(rule)) {
-        r = steps32<DIMS, INTEG, FIELD, true>(m, f, rule, prw, dim, j0, j1);
+        if (!hold_steps<INTEG>(f, dim, m.rotating && prw != 0.0, rule, j0, j1, dt_out, r.p, element))
+            r = steps32_call<DIMS, INTEG, FIELD>(m, f, rule, prw, dim, j0, j1);
     } else {
-        r = steps32<DIMS, INTEG, FIELD, false>(m, f, rule, prw, dim, j0, j1);
+        r = steps32<DIMS, INTEG, FIELD>(m, f, rule, prw, dim, j0, j1);
     }
     for (int s = 1; s < lanes; s <<= 1) r.nsq += __shfl_down_sync(0xffffffffu, r.nsq, s);
     const bool writes = active && lane_in_group == 0;

@@ -34,8 +34,8 @@ SS_D void transform_frame_lt8(double* s, double rw, c64 w) {
     s[7] = X.im;
 }
 
-// Frame phasors restart from sincos after this many steps of their recurrence, so that their drift
-// (about one rounding a step) stays far below the phase's own argument rounding.
+// Frame phasors restart from sincos after this many steps of their recurrence (a power of two), so that their
+// drift (about one rounding a step) stays far below the phase's own argument rounding.
 constexpr int kPhasorSteps = 64;
 
 struct PhasorPair {
@@ -53,11 +53,13 @@ __attribute__((const)) inline __device__ __noinline__ PhasorPair phasor_pair(dou
 
 // Where an interval's steps sample the field and how they weight the samples: the interval's start, the
 // reference's sample offsets and weights of an integrator for steps of dt (I:624-686 Magnus CF4 at the two
-// Gauss points, I:693-752 Heun at the step's ends, I:759-791 Euler at its middle).  A sample's time is t_c + tau
-// with tau = j dt + offset, rounded once each, and the frame's phase is taken at tau, so that the part of the
-// field's phase that is common with it cancels.  Far from time zero (kFollowSteps) the rounding of times shows in
-// the operators, and the samples are taken at the reference's own times instead, the running sum of steps
-// (I:836), with the frame's phase corrected to them (FP64; the FP32-bulk frame turns uniformly).
+// Gauss points, I:693-752 Heun at the step's ends, I:759-791 Euler at its middle).  Samples are taken at the
+// reference's own times, rounded as it rounds them: offsets from the running sum of the steps (I:836), in FP64 at
+// the steps' ends and middles also by way of their distance from the interval's start (I:705-716, another
+// rounding only next to time zero; no edge lies on a Gauss point).  Which side of a field's edge a sample on it falls
+// depends on that, and with a fast field the roundings add up over a call (10 MHz, 10 ns, 10^6 steps: states
+// 8e-9 from those of times j dt).  The frame's phase is taken at the same times (FP64; the FP32-bulk frame turns
+// uniformly), so that the part of the field's phase that is common with it cancels.
 struct StepRule {
     double t_c, dt, off_a, off_b, c0, c1;
 };
@@ -77,63 +79,63 @@ SS_D StepRule step_rule(double t_c, double dt) {
     return r;
 }
 
-// Steps from time zero beyond which an interval is far (FAR below): its samples follow the reference's running
-// sum.  At 10^6 steps the two kinds of times give states 2e-11 apart (a 10 ms spin-one drive at 840 kHz), growing
-// with the time.
-constexpr double kFollowSteps = 1048576.0;
-
-// Far intervals of user fields have a loop of their own, out of line: in one loop their extra arithmetic costs the
-// others 5% (pulse ensemble 2778 -> 2929 us).  Tone fields have the far loop only: they reach the step loops mostly
-// when far, and a step's sines outweigh it (far FP64 tones 579 us inline, 1013 out of line).
-SS_D bool far_from_zero(const StepRule& r) { return fabs(r.t_c) > kFollowSteps * r.dt; }
-
-// What a step loop's field samples need: the rule, the step's number, the frame phasors exp(-i prw tau),
-// prw = P rw with P the power of the frame winding in the xy transform (I:599-613: 2 for spin half, 1 for
-// spin one), at the step's two samples and their rotation by one step, and the table cursors.
+// What a step loop's field samples need: the rule, the step's start, the frame phasors exp(-i prw tau), prw = P rw
+// with P the power of the frame winding in the xy transform (I:599-613: 2 for spin half, 1 for spin one), at the
+// step's two samples and their rotation by one step, and the table cursors.
+//
+// While the times keep their exponent every step of the running sum rounds to the same multiple of their last
+// place, so the phasors turn by that step, and restart at the sum itself.  Measured against correcting the phasors
+// of uniform steps to the sum: the pulse ensemble 3075 -> 2823 us (2784 at uniform times).
 template <int L>
 struct Steps : StepRule {
     c64 wa, wb, wrot;
-    double prw, j, t_fine;
+    double prw, t_fine;
     bool rotating;
+    int restart_steps;
     TableCursor cur[L];
 
     SS_D Steps(const StepRule& rule) : StepRule(rule) {}
-    SS_D double tau(double off) const { return fma(j, dt, off); }
 
     template <int INTEG>
     SS_D void start_phasors() {
-        const PhasorPair p = phasor_pair(-prw * tau(off_a), INTEG != INTEG_EULER ? -prw * tau(off_b) : 0.0);
+        const PhasorPair p = phasor_pair(-prw * ((t_fine + off_a) - t_c),
+                                         INTEG != INTEG_EULER ? -prw * ((t_fine + off_b) - t_c) : 0.0);
         wa = p.a;
         wb = p.b;
     }
-    // Steps from number `first` of an interval that starts at t (steps: how many it has; 0: none).
-    template <int INTEG, bool FAR>
-    SS_D void begin(const MethodConfig& m, double interval_prw, int first, int steps) {
+    // Steps first .. end - 1 of an interval.
+    template <int INTEG>
+    SS_D void begin(const MethodConfig& m, double interval_prw, int first, int end) {
         prw = interval_prw;
         t_fine = t_c;
-        if (FAR)
-            for (int k = 0; k < first; k++) t_fine += dt;
-        j = (double)first;
+        for (int k = 0; k < first; k++) t_fine += dt;
         rotating = m.rotating;
+        restart_steps = kPhasorSteps;
         wa = wb = wrot = c64{1.0, 0.0};
-        if (m.rotating && steps > 0 && prw != 0.0) {
-            sincos_small(-prw * dt, &wrot.im, &wrot.re);
+        if (m.rotating && end > first && prw != 0.0) {
+            const double t_next = t_fine + dt, step = (t_next + dt) - t_next, t_end = fma((double)(end - first), dt, t_fine);
+            // Another exponent on the way, or a first step that rounds otherwise (a tie): where that shows, the
+            // phasors restart at every step.
+            const bool even = step == t_next - t_fine &&
+                              ((__double2hiint(t_fine) ^ __double2hiint(t_end)) & 0xfff00000) == 0;
+            const double furthest = fmax(fabs(t_fine), fabs(t_end));
+            if (!even && fabs(prw) * furthest * (0x1p-52 * (double)(end - first)) > 1e-14) restart_steps = 1;
+            sincos_small(-prw * step, &wrot.im, &wrot.re);
             start_phasors<INTEG>();
         }
 #pragma unroll
         for (int c = 0; c < L; c++) cur[c] = TableCursor{};  // for the increasing sample times of the steps
     }
-    // Before the samples of step n of a lane that began at step n0: the phasors from sincos every
-    // kPhasorSteps steps.
+    // Before the samples of step n of a lane that began at step n0.
     template <int INTEG>
     SS_D void restart(int n, int n0) {
-        if (rotating && prw != 0.0 && (n - n0) % kPhasorSteps == 0) start_phasors<INTEG>();
+        if (rotating && prw != 0.0 && ((n - n0) & (restart_steps - 1)) == 0) start_phasors<INTEG>();
     }
 };
 
 // One step's field samples (FP64) -> frame transform -> the integrator's generators (FP64); the
-// step number and the frame phasors move on.
-template <int FIELD, int L, int INTEG, bool FP64, bool FAR>
+// step's start and the frame phasors move on.
+template <int FIELD, int L, int INTEG, bool FP64>
 SS_D void step_generators(const FieldDesc& f, Steps<L>& st, double* ga, double* gb) {
     double s0[8], s1[8];  // a user field writes all eight channels
 #pragma unroll
@@ -141,30 +143,22 @@ SS_D void step_generators(const FieldDesc& f, Steps<L>& st, double* ga, double* 
         s0[k] = 0.0;
         s1[k] = 0.0;
     }
-    const double ta = st.tau(st.off_a), tb = st.tau(st.off_b);
-    double at_a = st.t_c + ta, at_b = st.t_c + tb;
-    c64 wa = st.wa, wb = st.wb;
-    if constexpr (FAR) {
-        at_a = st.t_fine + st.off_a;
-        at_b = st.t_fine + st.off_b;
-        st.t_fine += st.dt;
-        if (FP64 && st.rotating) {  // to first order: the times differ by a few roundings of t_c
-            const double turn_a = st.prw * ((at_a - st.t_c) - ta), turn_b = st.prw * ((at_b - st.t_c) - tb);
-            wa = c64{fma(turn_a, wa.im, wa.re), fma(-turn_a, wa.re, wa.im)};
-            wb = c64{fma(turn_b, wb.im, wb.re), fma(-turn_b, wb.re, wb.im)};
-        }
+    double at_a = st.t_fine + st.off_a, at_b = st.t_fine + st.off_b;
+    if constexpr (FP64 && INTEG != INTEG_CF4) {
+        at_a = (at_a - st.t_c) + st.t_c;
+        at_b = (at_b - st.t_c) + st.t_c;
     }
+    st.t_fine += st.dt;
     sample_field<FIELD, L>(f, at_a, s0, st.cur);
     if (INTEG != INTEG_EULER) sample_field<FIELD, L>(f, at_b, s1, st.cur);
-    st.j += 1.0;
     if (st.rotating) {  // xy times exp(-i prw tau), z minus prw
-        const c64 xa = c64{s0[0], s0[1]} * wa;
+        const c64 xa = c64{s0[0], s0[1]} * st.wa;
         s0[0] = xa.re;
         s0[1] = xa.im;
         s0[2] -= st.prw;
         st.wa = st.wa * st.wrot;
         if (INTEG != INTEG_EULER) {
-            const c64 xb = c64{s1[0], s1[1]} * wb;
+            const c64 xb = c64{s1[0], s1[1]} * st.wb;
             s1[0] = xb.re;
             s1[1] = xb.im;
             s1[2] -= st.prw;
@@ -227,7 +221,7 @@ SS_D bool hold_steps(const FieldDesc& f, int dim, bool turns, const StepRule& st
 // and products, from the product u of the steps before.  On entry step j's generators are in g and st is at
 // step j + 1.  Out of line, its state passed by value, so that the registers of the common
 // SU(2) loop are allocated without this path's.
-template <int INTEG, int FIELD, bool FAR>
+template <int INTEG, int FIELD>
 __device__ __noinline__ Mat<3> spin_one_quadratic_steps64(const MethodConfig& m, const FieldDesc& f, Steps<4> st,
                                                           Mat<3> u, Generators4 g, int j0, int j, int j1) {
     for (;;) {
@@ -235,7 +229,7 @@ __device__ __noinline__ Mat<3> spin_one_quadratic_steps64(const MethodConfig& m,
         if constexpr (INTEG != INTEG_EULER) spin_one_step64(m, u, g.b);
         if (++j >= j1) return u;
         st.template restart<INTEG>(j, j0);
-        step_generators<FIELD, 4, INTEG, true, FAR>(f, st, g.a, g.b);
+        step_generators<FIELD, 4, INTEG, true>(f, st, g.a, g.b);
     }
 }
 
@@ -250,21 +244,15 @@ SS_D Mat<3> interval_lt8(const MethodConfig& m, const FieldDesc& f, double t_c, 
 #pragma unroll
     for (int c = 0; c < L; c++) cur[c] = TableCursor{};
     const StepRule st = step_rule<INTEG>(t_c, dt);
-    double step = (double)j0, t_fine = t_c;
-    const bool follow = far_from_zero(st);
-    if (follow)
-        for (int j = 0; j < j0; j++) t_fine += dt;
+    double t_fine = t_c;
+    for (int j = 0; j < j0; j++) t_fine += dt;
     auto sample = [&](double* s, double off) {
 #pragma unroll
         for (int k = 0; k < L; k++) s[k] = 0.0;
-        double tau = fma(step, dt, off), at = t_c + tau;
-        if (follow) {
-            at = t_fine + off;
-            tau = at - t_c;
-        }
+        const double tau = (t_fine + off) - t_c;
         c64 w = c64{1.0, 0.0};
         if (m.rotating) sincos(rw * tau, &w.im, &w.re);
-        sample_field<FIELD, L>(f, at, s, cur);
+        sample_field<FIELD, L>(f, tau + t_c, s, cur);
         if (m.rotating) transform_frame_lt8(s, rw, w);
     };
     for (int j = j0; j < j1; j++) {
@@ -279,7 +267,6 @@ SS_D Mat<3> interval_lt8(const MethodConfig& m, const FieldDesc& f, double t_c, 
             for (int k = 0; k < L; k++) g[k] = INTEG == INTEG_CF4 ? st.c1 * s0[k] + st.c0 * s1[k] : st.c0 * s1[k];
             u = matmul(expo_lt8_one(g, m.hypercubes, m.precision), u);
         }
-        step += 1.0;
         t_fine += dt;
     }
     return u;
@@ -404,23 +391,23 @@ struct StepsResult {
 };
 
 // Steps j0 .. j1 - 1 of an interval, one after another.
-template <int DIMS, int INTEG, bool LT_HALF, int FIELD, bool FAR>
+template <int DIMS, int INTEG, bool LT_HALF, int FIELD>
 SS_D StepsResult steps64(const MethodConfig& m, const FieldDesc& f, const StepRule& rule, double prw, int dim, int j0, int j1) {
     constexpr int L = LieDim<DIMS, EXPO_LIE_TROTTER>::value;
     const bool lie_trotter = dim == 3 || LT_HALF;
     Steps<L> st(rule);
-    st.template begin<INTEG, FAR>(m, prw, j0, j1 - j0);
+    st.template begin<INTEG>(m, prw, j0, j1);
     StepsResult r;
     r.p = Su2d{c64{0.0, 0.0}, c64{0.0, 0.0}};
     r.quadratic = false;
     for (int j = j0; j < j1; j++) {
         Generators4 g;
         if (j != j0) st.template restart<INTEG>(j, j0);
-        step_generators<FIELD, L, INTEG, true, FAR>(f, st, g.a, g.b);
+        step_generators<FIELD, L, INTEG, true>(f, st, g.a, g.b);
         if constexpr (DIMS != 2) {
             if (dim == 3 && (g.a[3] != 0.0 || (INTEG != INTEG_EULER && g.b[3] != 0.0))) {
                 r.quadratic = true;
-                r.u = spin_one_quadratic_steps64<INTEG, FIELD, FAR>(
+                r.u = spin_one_quadratic_steps64<INTEG, FIELD>(
                     m, f, st, su2_to_spin_one(c64{1.0 + r.p.am1.re, r.p.am1.im}, r.p.beta), g, j0, j, j1);
                 break;
             }
@@ -432,10 +419,10 @@ SS_D StepsResult steps64(const MethodConfig& m, const FieldDesc& f, const StepRu
 }
 
 // For table fields out of line, so that their cursors' registers are not the piecewise constant path's too.
-template <int DIMS, int INTEG, bool LT_HALF, int FIELD, bool FAR>
+template <int DIMS, int INTEG, bool LT_HALF, int FIELD>
 __device__ __noinline__ StepsResult steps64_call(const MethodConfig& m, const FieldDesc& f, StepRule rule, double prw, int dim,
                                                  int j0, int j1) {
-    return steps64<DIMS, INTEG, LT_HALF, FIELD, FAR>(m, f, rule, prw, dim, j0, j1);
+    return steps64<DIMS, INTEG, LT_HALF, FIELD>(m, f, rule, prw, dim, j0, j1);
 }
 
 // Evolve one output interval.  Every lane of the warp must call this (shuffles use the full mask);
@@ -484,16 +471,10 @@ SS_D void interval64(const MethodConfig& m, const Instance& inst, const FieldDes
                 if constexpr (INTEG != INTEG_EULER) su2_apply64(e, su2_step_element64(m, lie_trotter, gb));
                 return e;
             };
-            if (hold_steps<INTEG>(f, dim, m.rotating && prw != 0.0, rule, j0, j1, dt_out, r.p, element)) {
-            } else if (far_from_zero(rule)) {
-                r = steps64_call<DIMS, INTEG, kLieTrotterHalf, FIELD, true>(m, f, rule, prw, dim, j0, j1);
-            } else {
-                r = steps64_call<DIMS, INTEG, kLieTrotterHalf, FIELD, false>(m, f, rule, prw, dim, j0, j1);
-            }
-        } else if (FIELD == FIELD_TONES || far_from_zero(rule)) {  // tones: here mostly far ones, and slow to sample
-            r = steps64<DIMS, INTEG, kLieTrotterHalf, FIELD, true>(m, f, rule, prw, dim, j0, j1);
+            if (!hold_steps<INTEG>(f, dim, m.rotating && prw != 0.0, rule, j0, j1, dt_out, r.p, element))
+                r = steps64_call<DIMS, INTEG, kLieTrotterHalf, FIELD>(m, f, rule, prw, dim, j0, j1);
         } else {
-            r = steps64<DIMS, INTEG, kLieTrotterHalf, FIELD, false>(m, f, rule, prw, dim, j0, j1);
+            r = steps64<DIMS, INTEG, kLieTrotterHalf, FIELD>(m, f, rule, prw, dim, j0, j1);
         }
         finish_steps<DIMS>(m, dim, r.p, r.u, r.quadratic, lanes, lane_in_group, rw, dt_out, writes, t_c, index, time_out,
                            u_out, product_out);
