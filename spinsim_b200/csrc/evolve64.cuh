@@ -62,6 +62,12 @@ __attribute__((const)) inline __device__ __noinline__ PhasorPair phasor_pair(dou
 // uniformly), so that the part of the field's phase that is common with it cancels.
 struct StepRule {
     double t_c, dt, off_a, off_b, c0, c1;
+
+    // A sample's time from the running sum plus its offset.
+    template <int INTEG, bool FP64>
+    SS_D double sample_time(double t) const {
+        return FP64 && INTEG != INTEG_CF4 ? (t - t_c) + t_c : t;
+    }
 };
 
 template <int INTEG>
@@ -79,13 +85,22 @@ SS_D StepRule step_rule(double t_c, double dt) {
     return r;
 }
 
+// Whether the running sum t + dt + dt ... takes n equal steps: while it keeps its sign and exponent, each rounds to
+// the same multiple of its last place (*step), but for a first one halfway between two.  The sum after j steps is
+// then t + j *step exactly.
+SS_D bool even_steps(double t, double dt, int n, double* step) {
+    const double next = t + dt;
+    *step = (next + dt) - next;
+    const double end = fma((double)n, *step, t);
+    return *step == next - t && ((__double2hiint(t) ^ __double2hiint(end)) & 0xfff00000) == 0;
+}
+
 // What a step loop's field samples need: the rule, the step's start, the frame phasors exp(-i prw tau), prw = P rw
 // with P the power of the frame winding in the xy transform (I:599-613: 2 for spin half, 1 for spin one), at the
 // step's two samples and their rotation by one step, and the table cursors.
 //
-// While the times keep their exponent every step of the running sum rounds to the same multiple of their last
-// place, so the phasors turn by that step, and restart at the sum itself.  Measured against correcting the phasors
-// of uniform steps to the sum: the pulse ensemble 3075 -> 2823 us (2784 at uniform times).
+// The phasors turn by the running sum's own step (even_steps), and restart at the sum itself.  Measured against
+// correcting the phasors of uniform steps to the sum: the pulse ensemble 3075 -> 2823 us (2784 at uniform times).
 template <int L>
 struct Steps : StepRule {
     c64 wa, wb, wrot;
@@ -113,13 +128,11 @@ struct Steps : StepRule {
         restart_steps = kPhasorSteps;
         wa = wb = wrot = c64{1.0, 0.0};
         if (m.rotating && end > first && prw != 0.0) {
-            const double t_next = t_fine + dt, step = (t_next + dt) - t_next, t_end = fma((double)(end - first), dt, t_fine);
-            // Another exponent on the way, or a first step that rounds otherwise (a tie): where that shows, the
-            // phasors restart at every step.
-            const bool even = step == t_next - t_fine &&
-                              ((__double2hiint(t_fine) ^ __double2hiint(t_end)) & 0xfff00000) == 0;
-            const double furthest = fmax(fabs(t_fine), fabs(t_end));
-            if (!even && fabs(prw) * furthest * (0x1p-52 * (double)(end - first)) > 1e-14) restart_steps = 1;
+            // Where the steps are not even and that shows, the phasors restart at every one.
+            double step;
+            if (!even_steps(t_fine, dt, end - first, &step) &&
+                fabs(prw) * fma((double)(end - first), dt, fabs(t_fine)) * (0x1p-52 * (double)(end - first)) > 1e-14)
+                restart_steps = 1;
             sincos_small(-prw * step, &wrot.im, &wrot.re);
             start_phasors<INTEG>();
         }
@@ -143,11 +156,8 @@ SS_D void step_generators(const FieldDesc& f, Steps<L>& st, double* ga, double* 
         s0[k] = 0.0;
         s1[k] = 0.0;
     }
-    double at_a = st.t_fine + st.off_a, at_b = st.t_fine + st.off_b;
-    if constexpr (FP64 && INTEG != INTEG_CF4) {
-        at_a = (at_a - st.t_c) + st.t_c;
-        at_b = (at_b - st.t_c) + st.t_c;
-    }
+    const double at_a = st.template sample_time<INTEG, FP64>(st.t_fine + st.off_a);
+    const double at_b = st.template sample_time<INTEG, FP64>(st.t_fine + st.off_b);
     st.t_fine += st.dt;
     sample_field<FIELD, L>(f, at_a, s0, st.cur);
     if (INTEG != INTEG_EULER) sample_field<FIELD, L>(f, at_b, s1, st.cur);
@@ -179,25 +189,30 @@ struct Generators4 {
 // Steps j0 .. j1 - 1 of an interval whose field is piecewise constant and whose frame does not turn (pulse
 // trains), as runs: the steps between two knots share one element, and their product is its power by
 // squarings; a step with a knot between its samples is a run of its own.  element(ga, gb, n) is the element of
-// n steps of these generators.  False, with nothing done, unless every lane of the warp (which all call
-// this) can take this form.  Bound by latency (the knots' search and the runs' divergence).  A launch of 400
-// pulse trains (4.1e6 output steps of 20, FP32-bulk, 128 registers): 1704 -> 564 us.
+// n steps of these generators.  Every lane of the warp calls this.  False, and p of no use, for lanes that do not
+// take this form: all of them, or those with a sample so near to a knot that its time's roundings decide the side
+// it falls on (a knot on the sample times of Heun or Euler), which only the running sum tells.  Bound by
+// latency (the knots' search and the runs' divergence).  A launch of 400 pulse trains (4.1e6 output steps of 20,
+// FP32-bulk, 128 registers), time evolution and scan: 3059 us step by step, 777 so, 899 with the running sum in here.
 template <int INTEG, typename Element>
 SS_D bool hold_steps(const FieldDesc& f, int dim, bool turns, const StepRule& st, int j0, int j1, double dt_out, Su2d& p,
                      Element element) {
     if (__any_sync(0xffffffffu, turns)) return false;
     HoldChannel ch[3];
     const double first = __shfl_sync(0xffffffffu, st.t_c, 0);
-    if (!hold_channels(f, dim == 2 ? 3 : 4, first, first + 33.0 * dt_out, ch)) return false;
     const double dt = st.dt, last = INTEG == INTEG_EULER ? st.off_a : st.off_b;
-    for (int j = j0, n; j < j1; j += n) {
+    // twice as far as the roundings of a time here and of the running sum (I:836) may be apart
+    const double slack = (double)(j1 + 4) * 0x1p-51 * (fabs(st.t_c) + dt_out);
+    if (!hold_channels(f, dim == 2 ? 3 : 4, first, first + 33.0 * dt_out, slack, ch)) return false;
+    bool near = false;
+    for (int j = j0, n; j < j1 && !near; j += n) {
         const double ta = st.t_c + fma((double)j, dt, st.off_a), tb = st.t_c + fma((double)j, dt, last);
         double sa[3], ga[3], gb[3];
         double until = INFINITY;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            sa[c] = ch[c].at(f, c, ta);
-            until = fmin(until, ch[c].t_hi);
+            sa[c] = ch[c].at(f, c, ta, slack, near);
+            until = fmin(until, ch[c].clear);
         }
         n = 1;
         if (tb < until) {
@@ -208,13 +223,13 @@ SS_D bool hold_steps(const FieldDesc& f, int dim, bool turns, const StepRule& st
         }
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            const double sb = INTEG == INTEG_EULER ? 0.0 : tb < until ? sa[c] : ch[c].at(f, c, tb);
+            const double sb = INTEG == INTEG_EULER ? 0.0 : tb < until ? sa[c] : ch[c].at(f, c, tb, slack, near);
             ga[c] = fma(st.c0, sa[c], st.c1 * sb);
             gb[c] = INTEG == INTEG_HEUN ? st.c0 * sb : fma(st.c1, sa[c], st.c0 * sb);
         }
         su2_apply_power64(p, element(ga, gb, n), n);
     }
-    return true;
+    return !near;
 }
 
 // Steps j .. j1 - 1 of a spin-one interval whose quadratic shift is non-zero: full 3 x 3 exponentials

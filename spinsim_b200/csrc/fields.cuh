@@ -188,29 +188,29 @@ SS_D int64_t warp_seek(const TableChannel& tb, double t) {
 }
 
 // A channel of a piecewise constant field (a zero-order hold, or no table) for sample times that only
-// increase: its value val (gain and bias included) up to its next knot t_hi.  A sample on the knot itself
-// goes to the reference's search.
+// increase: its value val (gain and bias included), for times before `clear`, its next knot less the sample
+// times' slack.
 struct HoldChannel {
     int32_t i;  // the value is that of (time[i], time[i + 1])
-    double t_hi, val;
+    double clear, val;
 
-    SS_D void load(const FieldDesc& f, int c) {
+    SS_D void load(const FieldDesc& f, int c, double slack) {
         const TableChannel& tb = f.tables[c];
         double v = 0.0;
         if (i >= 0 && i + 1 < tb.size) v = __ldg(tb.amplitude + i);
         else if (!tb.zero_boundary) v = __ldg(tb.amplitude + (i < 0 ? 0 : tb.size - 1));
         val = fma(f.gain[c], v, f.bias[c]);
-        t_hi = i + 1 < tb.size ? __ldg(tb.time + i + 1) : INFINITY;
+        clear = i + 1 < tb.size ? __ldg(tb.time + i + 1) - slack : INFINITY;
     }
-    // The value at t (not before the last one's).
-    SS_D double at(const FieldDesc& f, int c, double t) {
-        if (t > t_hi) {
+    // The value at t (not before the last one's); `near` is set when a knot lies within the slack of t.
+    SS_D double at(const FieldDesc& f, int c, double t, double slack, bool& near) {
+        if (t >= clear) {
             const TableChannel& tb = f.tables[c];
-            do i++;
-            while (i + 1 < tb.size && t > __ldg(tb.time + i + 1));
-            load(f, c);
+            while (i + 1 < tb.size && t > __ldg(tb.time + i + 1) + slack) i++;
+            load(f, c, slack);
+            near |= t >= clear;
         }
-        return t == t_hi ? fma(f.gain[c], table_sample(f.tables[c], t), f.bias[c]) : val;
+        return val;
     }
 };
 
@@ -219,13 +219,14 @@ struct HoldChannel {
 // or has many knots before t_end, the end of the warp's intervals, to walk.
 constexpr int kHoldKnots = 32;
 
-SS_D bool hold_channels(const FieldDesc& f, int used, double t_first, double t_end, HoldChannel (&ch)[3]) {
+SS_D bool hold_channels(const FieldDesc& f, int used, double t_first, double t_end, double slack,
+                        HoldChannel (&ch)[3]) {
     if (used > 3 && (f.tables[3].size > 0 || f.bias[3] != 0.0)) return false;
 #pragma unroll
     for (int c = 0; c < 3; c++) {
         const TableChannel& tb = f.tables[c];
         ch[c].i = -1;
-        ch[c].t_hi = INFINITY;
+        ch[c].clear = INFINITY;
         ch[c].val = f.bias[c];
         if (tb.size <= 0) continue;
         if (tb.order != 0 || tb.size >= INT32_MAX) return false;
@@ -235,7 +236,7 @@ SS_D bool hold_channels(const FieldDesc& f, int used, double t_first, double t_e
             ch[c].i = (int32_t)warp_seek(tb, t_first);
             if ((int64_t)ch[c].i + kHoldKnots < tb.size && __ldg(tb.time + ch[c].i + kHoldKnots) < t_end) return false;
         }
-        ch[c].load(f, c);
+        ch[c].load(f, c, slack);
     }
     return true;
 }
