@@ -174,7 +174,7 @@ class ToneField(BuiltinField):
         td = torch.from_numpy(flat).to(device)
         f = _lib.Field()
         f.tones = td.data_ptr()
-        f.n_params = math.ceil(min(max(1.0, float(np.abs(flat[::3]).max())), 1e18))  # the largest |w|
+        f.n_params = math.ceil(min(float(np.fmax.reduce(np.abs(flat[::3]), initial=1.0)), 1e18))  # the largest |w|
         for c in range(8):
             f.tone_start[c] = int(start[c])
             f.tone_count[c] = int(count[c])
