@@ -191,13 +191,14 @@ class Results:
     def _from_block(cls, block, spin_calculator, keep, error):
         """Results in one device block (``_Block``); its tensor views are made on first use."""
         self = cls.__new__(cls)
-        self.__dict__.update(_dev=None, _block=block, spin_calculator=spin_calculator, _keep=keep, _error=error)
+        self.__dict__.update(_dev=None, _block=block, _host=None, spin_calculator=spin_calculator, _keep=keep, _error=error)
         return self
 
     def _device(self):
         dev = self.__dict__["_dev"]
         if dev is None:
             dev = self.__dict__["_dev"] = self.__dict__["_block"].tensors()
+            self.__dict__["_host"] = None  # a caller may write to them: arrays not read yet come from the device
         return dev
 
     @property
@@ -220,9 +221,11 @@ class Results:
     def __getattr__(self, name):
         if name in Results._ARRAYS:
             if self.__dict__["_dev"] is None:
-                # no tensor of it has been handed out: one copy brings all four arrays
-                self.__dict__.update(self.__dict__["_block"].host_arrays())
-                return self.__dict__[name]
+                # no tensor of it has been handed out: one copy brings all four arrays, each an attribute once read
+                if self.__dict__["_host"] is None:
+                    self.__dict__["_host"] = self.__dict__["_block"].host_arrays()
+                value = self.__dict__[name] = self.__dict__["_host"][name]
+                return value
             dev = self._device()
             if name in dev:
                 value = _to_numpy(dev[name])
