@@ -113,7 +113,7 @@ struct EvolveArgs {
                              // product of the tile's operators; null: not written
     const int32_t* scan_begin;  // per instance: its first scan tile (null: one instance, tile 0)
     const struct DmmaConsts* dmma_consts;  // tensor path: per instance, written by dmma_consts_kernel
-                                           // earlier in the launch (null: each tile computes them)
+                                           // earlier in the launch; never null there
     double* rows;  // tensor path: per output step (indexed like time), the interval's lab-frame operator
                    // as its SU(2) pair (a, b), 4 doubles, for the state scan (null: not written)
     Instance single;         // instances == null: the instance,
@@ -153,18 +153,21 @@ SS_HD bool tones_on_tensor_path(const FieldDesc& f, int dim) {
         if (f.tone_count[c] > kBulkTones) return false;
     return !(dim == 3 && (f.bias[3] != 0.0 || f.tone_count[3] > 0));
 }
-// In FP64 also none whose phase w t grows beyond kToneMaxPhase: there the rounding of the reference's sample times,
-// which the per-sample form repeats and these products do not, shows in the operators (at 1.7e5 rad, 27 ms of 1 MHz
-// tones, states 4e-10 apart; at 6e4 rad, 1e-11).  A tone field's n_params is its largest |w|, rounded up; 0, not
-// given, counts as kToneDefaultRate.
+// In FP64 also none whose phase w t grows beyond kToneMaxPhase: there the rounding of each single sample time, at most
+// w t 2^-53, which the per-sample form repeats and these products do not, would show in the states of a resonant drive;
+// nor one for which w K t 2^-53, what the roundings of an interval's running sum can add up to, exceeds kToneMaxDrift.
+// The products follow that sum but where its exponent changes within an interval, to about an eighth of it.  A tone
+// field's n_params is its largest |w|, rounded up; 0, not given, counts as kToneDefaultRate.
 constexpr double kToneMaxPhase = 1e5;
+constexpr double kToneMaxDrift = 2e-9;
 constexpr double kToneDefaultRate = 1e7;
 SS_HD bool tones_on_fp64_tensor_path(const FieldDesc& f, const Instance& inst) {
     const double rate = f.n_params > 0 ? (double)f.n_params : kToneDefaultRate;
     const double first = inst.t0 + inst.dt_out * (double)inst.interval0, last = first + inst.dt_out * (double)inst.n_out;
     const double far = (first < 0 ? -first : first) > (last < 0 ? -last : last) ? (first < 0 ? -first : first)
                                                                               : (last < 0 ? -last : last);
-    return rate * far <= kToneMaxPhase && tones_on_tensor_path(f, inst.dim);
+    return rate * far <= kToneMaxPhase && rate * far * (0x1p-53 * (double)inst.n_fine) <= kToneMaxDrift &&
+           tones_on_tensor_path(f, inst.dim);
 }
 constexpr int kSynthIntervals = 2;          // output intervals per lane, 32 intervals apart
 // Slot-fastest layouts: a warp's 16-byte stores and loads of one quantity for all slots are

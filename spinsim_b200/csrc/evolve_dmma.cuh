@@ -63,6 +63,9 @@ constexpr int kDmmaSegments = 4;                             // lanes (time segm
 // Steps per segment in one table buffer: 5 divides the 25-step segments of K = 100 (1 us output
 // steps of 10 ns), so no phase is a short remainder; 4 was 1% slower there.
 constexpr int kDmmaPhase = SPINSIM_DMMA_PHASE;
+// FP64: the phasor recurrences restart from sincos every 60 pairs, as the step loop of evolve64.cuh does every 64
+// steps: their drift, about a rounding a pair, would grow with K (4e-13 at K = 1e5).
+constexpr int kDmmaRestart = 12;  // phases
 // Largest step size bound theta = h (|B|max + w_max) for which a tile takes the Magnus step.  The
 // Magnus and CF4 steps differ by O(theta^5) per step: measured 4.6e-6 at theta = 6.7 (one 1 us step)
 // and 1e-11 over 10^6 steps at theta = 0.07, i.e. about 3e-10 theta^5 per step, so at theta <= 0.1
@@ -77,12 +80,21 @@ constexpr double kDmmaW0 = (1.5 + kSqrt3) / 3.0, kDmmaW1 = (1.5 - kSqrt3) / 3.0;
 // First pair of segment seg: pair i is the i-th step after the middle of the K and its mirror image.
 SS_D int dmma_segment(int K, int seg) { return (int)(((int64_t)(K / 2) * seg) / kDmmaSegments); }
 
+// How the reference's steps of an interval, at the running sum t_c + dt + dt ... (I:836), lie against t_c + j dt: on
+// average `shift` later, and spaced (1 + stretch) dt about their middle.
+struct StepTimes {
+    double shift, stretch;
+};
+
 struct __align__(16) DmmaShared {
     double table[2][kDmmaPhase][kDmmaChunkDoubles];
     double2 z[kDmmaRecurrences];   // exp(i w delta) of each recurrence at its next pair
     double2 rot[kToneSlots];       // exp(i w dt)
     double2 middle[kToneSlots];    // exp(i w delta) at the middle step's samples
     double w[kToneSlots];          // the tones' frequencies
+    double2 half_step[kToneSlots]; // FP64: exp(i w dt_out / 2)
+    StepTimes times[kDmmaTile];    // FP64: the intervals' times (step_times)
+    double late[kDmmaTile];        // FP64: how far each middle lies from where L puts it
     Su2p warp_product[kDmmaWarps];
     int32_t tile;
     int32_t magnus;                // 1: the tile takes the one-exponential Magnus step
@@ -97,23 +109,42 @@ SS_D void dmma_m8n8k4(double& d0, double& d1, double a, double b) {
 
 static_assert(kDmmaTile == kScanTile, "a CTA tile is one state scan tile (its warps' row products are its partials)");
 
+// Frequency of tone slot (0 for an absent tone).
+SS_D double dmma_frequency(const FieldDesc& f, int slot) {
+    const int c = slot / kBulkTones, tone = slot % kBulkTones;
+    return tone < f.tone_count[c] ? __ldg(f.tones + 3 * (f.tone_start[c] + tone)) : 0.0;
+}
+
+// Pairs before column r's first one (recurrence r = slot * 8 + column), counted from the middle of the interval.
+SS_D double dmma_start(int K, int r) { return (double)dmma_segment(K, (r >> 1) & (kDmmaSegments - 1)) + (K & 1 ? 0.5 : 0.0); }
+
 // Pair recurrence r = slot * 8 + column (column = 2 * segment + Gauss point): the phasor exp(i w delta) of its tone
 // at the column's first distance from the middle of the interval, and the tone's step rotation exp(i w dt).
 SS_D void dmma_recurrence(const FieldDesc& f, int K, double dt, int r, double2* z, double2* rot) {
-    const int gauss = r & 1, seg = (r >> 1) & (kDmmaSegments - 1), slot = r >> 3;
+    const int gauss = r & 1, slot = r >> 3;
     const int c = slot / kBulkTones, tone = slot % kBulkTones;
     *z = make_double2(0.0, 0.0);
     *rot = make_double2(1.0, 0.0);
     if (tone < f.tone_count[c]) {
         const double a = 0.5 * dt * (gauss ? 1.0 + 1.0 / kSqrt3 : 1.0 - 1.0 / kSqrt3);
         const double w = __ldg(f.tones + 3 * (f.tone_start[c] + tone));
-        const double start = (double)dmma_segment(K, seg) + (K & 1 ? 0.5 : 0.0);
         double sn, cs;
-        sincos(w * fma(start, dt, a), &sn, &cs);
+        sincos(w * fma(dmma_start(K, r), dt, a), &sn, &cs);
         *z = make_double2(cs, sn);
         sincos(w * dt, &sn, &cs);
         *rot = make_double2(cs, sn);
     }
+}
+
+// Recurrence r's phasor at its pair `pair`.  Out of line: the recurrences restart from it so rarely that its code
+// should not be the step loop's.
+inline __device__ __noinline__ double2 dmma_restart(const FieldDesc& f, int K, double dt, int r, int pair) {
+    const int slot = r >> 3;
+    if (slot % kBulkTones >= f.tone_count[slot / kBulkTones]) return make_double2(0.0, 0.0);
+    const double a = 0.5 * dt * (r & 1 ? 1.0 + 1.0 / kSqrt3 : 1.0 - 1.0 / kSqrt3);
+    double sn, cs;
+    sincos(dmma_frequency(f, slot) * fma(dmma_start(K, r) + (double)pair, dt, a), &sn, &cs);
+    return make_double2(cs, sn);
 }
 
 // exp(i w tau) of tone slot (1 for an absent tone).
@@ -190,6 +221,29 @@ SS_D double time_rounding(double t0, double dt_out, double i) {
     const double p = __dmul_rn(dt_out, i), ep = __fma_rn(dt_out, i, -p);
     const double s = __dadd_rn(t0, p), b = __dsub_rn(s, t0);
     return -(__dadd_rn(__dsub_rn(t0, __dsub_rn(s, b)), __dsub_rn(p, b)) + ep);
+}
+
+inline __device__ __noinline__ StepTimes step_times(double t_c, double dt, int K) {
+    StepTimes s;
+    double step;
+    if (even_steps(t_c, dt, K, &step)) {
+        s.shift = 0.5 * (double)(K - 1) * (step - dt);
+        s.stretch = (step - dt) / dt;
+        return s;
+    }
+    // the few intervals in which the sum changes its exponent: the line through its deviations
+    double t = t_c, sum = 0.0, moment = 0.0;
+    const double middle = 0.5 * (double)(K - 1);
+    for (int j = 0; j < K; j++) {
+        const double off = (t - t_c) - (double)j * dt;
+        sum += off;
+        moment = fma((double)j - middle, off, moment);
+        t += dt;
+    }
+    const double n = (double)K;
+    s.shift = K > 0 ? sum / n : 0.0;
+    s.stretch = K > 1 ? 12.0 * moment / (n * (n * n - 1.0) * dt) : 0.0;
+    return s;
 }
 
 template <bool B>
@@ -282,48 +336,70 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
     if (threadIdx.x < kToneSlots) {
         sh.rot[threadIdx.x] = cst->rot[threadIdx.x];
         sh.middle[threadIdx.x] = cst->middle[threadIdx.x];
+        if constexpr (PREC == PREC_FP64) sh.half_step[threadIdx.x] = cst->half_step[threadIdx.x];
     }
     if (threadIdx.x == 0) sh.magnus = cst->magnus;
 
     // L of every tone at the middle of every interval of the tile (buffer 1 of the table holds it until the first
-    // refill): thread 4 slot + quarter evaluates interval 8 quarter once and steps to the next seven intervals
-    // with exp(i w dt_out).
+    // refill): thread 4 slot + quarter takes intervals 8 quarter .. 8 quarter + 7, stepping with exp(i w dt_out) from
+    // the call's every eighth interval, so that a piece of a call rounds as the whole does.
     double2* lval = reinterpret_cast<double2*>(&sh.table[1][0][0]);  // [slot][interval of the tile]
     static_assert(sizeof(sh.table[1]) >= sizeof(double2) * kToneSlots * kDmmaTile, "L table fits one buffer");
     if (threadIdx.x < 4 * kToneSlots) {
         const int slot = threadIdx.x >> 2, quarter = threadIdx.x & 3;
         const int c = slot / kBulkTones, tone = slot % kBulkTones;
         const int64_t i0 = inst.interval0 + tile.first + kDmmaRows * quarter;
-        c64 l = c64{0.0, 0.0}, gstep = c64{1.0, 0.0};
-        double w = 0.0;
-        if (tone < f.tone_count[c]) {
-            const double* tn = f.tones + 3 * (f.tone_start[c] + tone);
-            const double amp = f.gain[c] * __ldg(tn + 1);
-            w = __ldg(tn);
-            const double tq = __dadd_rn(inst.t0, __dmul_rn(dt_out, (double)i0));  // as the intervals' own t_c
-            double sn, cs;
-            sincos(fma(w, tq, __ldg(tn + 2)), &sn, &cs);
+        const bool present = tone < f.tone_count[c];
+        const double* tn = f.tones + (present ? 3 * (f.tone_start[c] + tone) : 0);
+        const double w = dmma_frequency(f, slot);
+        c64 l = c64{0.0, 0.0}, h = c64{1.0, 0.0};
+        if (present) {
             const double2 hs = cst->half_step[slot];
-            const c64 h = c64{hs.x, hs.y};
-            l = c64{half_dt * amp * cs, half_dt * amp * sn} * h;
-            gstep = h * h;
+            h = c64{hs.x, hs.y};
         }
+        const c64 gstep = h * h;
         if (quarter == 0) sh.w[slot] = w;
-#pragma unroll
-        for (int r = 0; r < kDmmaRows; r++) {
-            lval[slot * kDmmaTile + kDmmaRows * quarter + r] = make_double2(l.re, l.im);
+#pragma unroll 1
+        for (int64_t i = i0 & ~(int64_t)(kDmmaRows - 1); i < i0 + kDmmaRows; i++) {
+            if (present && (i & (kDmmaRows - 1)) == 0) {
+                const double amp = f.gain[c] * __ldg(tn + 1);
+                const double tq = __dadd_rn(inst.t0, __dmul_rn(dt_out, (double)i));  // as the intervals' own t_c
+                // the phase w tq + phi to twice the precision: its rounding, of which each of the reference's samples has
+                // its own, would be that of all steps of eight intervals
+                const double p = __dmul_rn(w, tq), phi = __ldg(tn + 2), phase = __dadd_rn(p, phi);
+                const double b = __dsub_rn(phase, p);
+                const double rest = __dadd_rn(__dsub_rn(p, __dsub_rn(phase, b)), __dsub_rn(phi, b)) + __fma_rn(w, tq, -p);
+                double sn, cs;
+                sincos(phase, &sn, &cs);
+                l = half_dt * amp * c64{fma(-rest, sn, cs), fma(rest, cs, sn)} * h;
+            }
+            if (i >= i0) lval[slot * kDmmaTile + kDmmaRows * quarter + (int)(i - i0)] = make_double2(l.re, l.im);
             l = l * gstep;
         }
+    } else if constexpr (PREC == PREC_FP64) {  // the last warp meanwhile: each interval's times
+        static_assert(4 * kToneSlots + kDmmaTile == kDmmaThreads, "a thread per interval beside the tones'");
+        const int r = threadIdx.x - 4 * kToneSlots;
+        const int64_t index = inst.interval0 + tile.first + r, from = index & ~(int64_t)(kDmmaRows - 1);
+        const StepTimes times = step_times(__dadd_rn(inst.t0, __dmul_rn(dt_out, (double)index)), dt, K);
+        sh.times[r] = times;
+        sh.late[r] = time_rounding(inst.t0, dt_out, (double)index) - time_rounding(inst.t0, dt_out, (double)from) + times.shift;
     }
     __syncthreads();  // producer phasors, rotations, step choice and L in place
 
     // A operands: L of this lane's interval for tone 4 s + q, its imaginary part for the even sums, real for the
-    // odd; in FP64 corrected (a phase below 1e-10, so to first order) for how the interval's start is rounded,
-    // relative to the warp's first interval, whose phase was taken at its rounded start
-    double late = 0.0;
+    // odd.
+    //
+    // In FP64 corrected for the reference's times.  Its samples are taken at the running sum of the steps (I:836), whose
+    // rounding is the same for all steps of the same exponent and for whole stretches of a call, so that a resonant
+    // drive shows it (1 MHz at 100 steps of 10 ns, states 1.1e-8 off at 10 ms, 5e-12 so; 64 mixed instances 551 -> 574 us).
+    // An interval's samples then lie `shift` later and are stretched about their middle.  The shift, with how the interval's start is rounded relative to the one
+    // whose phase was taken at its rounded start, is a small turn of L.  Evolving with H(t_m + (1 + stretch) tau) is
+    // evolving with H / (1 + stretch) over (1 + stretch) times as long: L and the bias take the factor here, the ends'
+    // extra time is two small elements below.  Both are the interval's own, so pieces of a call round as the whole does.
+    double late = 0.0, scale = 1.0;
     if constexpr (PREC == PREC_FP64) {
-        const int64_t first_index = inst.interval0 + tile.first + kDmmaRows * (threadIdx.x >> 5);
-        late = time_rounding(inst.t0, dt_out, (double)(first_index + g)) - time_rounding(inst.t0, dt_out, (double)first_index);
+        late = sh.late[row];
+        scale = 1.0 - sh.times[row].stretch;
     }
     double even_a[3][2], odd_a[3][2];
 #pragma unroll
@@ -333,8 +409,8 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
             const double2 lv = lval[(c * kBulkTones + 4 * s + q) * kDmmaTile + row];
             if constexpr (PREC == PREC_FP64) {
                 const double turn = late * sh.w[c * kBulkTones + 4 * s + q];
-                even_a[c][s] = active ? fma(turn, lv.x, lv.y) : 0.0;
-                odd_a[c][s] = active ? fma(-turn, lv.y, lv.x) : 0.0;
+                even_a[c][s] = active ? scale * fma(turn, lv.x, lv.y) : 0.0;
+                odd_a[c][s] = active ? scale * fma(-turn, lv.y, lv.x) : 0.0;
             } else {
                 even_a[c][s] = active ? lv.y : 0.0;
                 odd_a[c][s] = active ? lv.x : 0.0;
@@ -355,6 +431,9 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
 #pragma unroll
     for (int c = 0; c < 3; c++) bias[c] = __dmul_rn(half_dt, f.bias[c]);
     bias[2] = __fma_rn(-half_dt, prw, bias[2]);
+    if constexpr (PREC == PREC_FP64)
+#pragma unroll
+        for (int c = 0; c < 3; c++) bias[c] *= scale;
     // Frame phasors at the Gauss points of this segment's steps after the middle: exp(-i P rw delta); those of
     // the mirrored steps before it are their conjugates
     const double start = (double)seg_start + (K & 1 ? 0.5 : 0.0);
@@ -375,6 +454,7 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
             // consumer lane 4 col + tone % 4 of k-step tone / 4: cosines (even sums), then sines
             double* dst = &sh.table[ph & 1][0][(c * 4 + (tone >> 2)) * 32 + 4 * col + (tone & 3)];
             double2 z = sh.z[r];
+            if (PREC == PREC_FP64 && ph > 0 && ph % kDmmaRestart == 0) z = dmma_restart(f, K, dt, r, m0);
             const double2 rt = sh.rot[slot];
             for (int mm = 0; mm < mc; mm++) {
                 dst[mm * kDmmaChunkDoubles] = z.x;
@@ -464,6 +544,12 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
             if (ph + 1 < n_phases) fill(ph + 1);
             const int m0 = ph * kDmmaPhase;
             const int mc = min(kDmmaPhase, n_steps - m0);
+            if (PREC == PREC_FP64 && m.rotating && ph > 0 && ph % kDmmaRestart == 0) {
+                const double at = start + (double)m0;
+                const PhasorPair p = phasor_pair(-prw * fma(at, dt, a_lo), -prw * fma(at, dt, a_hi));
+                wa = p.a;
+                wb = p.b;
+            }
             const double* tb = &sh.table[ph & 1][0][lane];
             // Even and odd sums at the two distances of pair mm (tensor path), issued at the end of pair mm - 1, so
             // they are in flight while the next pair begins.
@@ -516,6 +602,35 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
     // The interval's product, in lane 0 of the quad
     combine_segments<false>(after, q);
     combine_segments<true>(before, q);
+    c64 half_frame = c64{1.0, 0.0};  // the frame's turn over half an output step
+    if (m.rotating) sincos_small(-0.5 * prw * dt_out, &half_frame.im, &half_frame.re);
+    if constexpr (PREC == PREC_FP64) {
+        // The ends' extra time: 1 - i (stretch T / 2) B.sigma / 2, T = K dt, with the ends' samples summed over the quad
+        // (one column would leave seven eighths of a tensor product idle).
+        double first[3], last[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            const double2 z0 = sh.half_step[c * kBulkTones + q], z1 = sh.half_step[c * kBulkTones + 4 + q];
+            double even = fma(even_a[c][0], z0.x, even_a[c][1] * z1.x);
+            double odd = fma(odd_a[c][0], z0.y, odd_a[c][1] * z1.y);
+#pragma unroll
+            for (int s = 1; s < kDmmaSegments; s <<= 1) {
+                even += __shfl_xor_sync(0xffffffffu, even, s);
+                odd += __shfl_xor_sync(0xffffffffu, odd, s);
+            }
+            first[c] = bias[c] + even - odd;
+            last[c] = bias[c] + even + odd;
+        }
+        if (m.rotating) {
+            rotate(first, conj(half_frame));
+            rotate(last, half_frame);
+        }
+        const double n = 0.5 * sh.times[row].stretch * (double)K;
+        Su2d p = Su2d{c64{0.0, -n * first[2]}, c64{n * first[1], -n * first[0]}};
+        su2_apply64(p, before);
+        before = p;
+        su2_apply64(after, Su2d{c64{0.0, -n * last[2]}, c64{n * last[1], -n * last[0]}});
+    }
     su2_apply64(before, after);
     if constexpr (PREC == PREC_FP32_BULK) {
 #pragma unroll
@@ -530,9 +645,11 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
         v.a = c64{1.0 + before.am1.re, before.am1.im};
         v.b = before.beta;
         if (m.rotating) {
-            c64 w;
-            sincos_small(0.5 * prw * dt_out, &w.im, &w.re);
-            v.a = v.a * conj(w);
+            v.a = v.a * half_frame;
+            if constexpr (PREC == PREC_FP64) {  // the phases counted from half an output step and the middle's shift
+                const double x = -prw * sh.times[row].shift;
+                v.b = c64{fma(-x, v.b.im, v.b.re), fma(x, v.b.re, v.b.im)};
+            }
         }
         time_out[idx] = t_c;
         if (norms_out != nullptr) norms_out[idx] = nsq;
