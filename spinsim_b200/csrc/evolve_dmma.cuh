@@ -231,14 +231,24 @@ inline __device__ __noinline__ StepTimes step_times(double t_c, double dt, int K
         s.stretch = (step - dt) / dt;
         return s;
     }
-    // the few intervals in which the sum changes its exponent: the line through its deviations
-    double t = t_c, sum = 0.0, moment = 0.0;
+    // The few intervals in which the sum changes its exponent: the line through its deviations from t_c + j dt, a run
+    // of steps of one exponent at a time.
+    double t = t_c, off = 0.0, sum = 0.0, moment = 0.0;
     const double middle = 0.5 * (double)(K - 1);
-    for (int j = 0; j < K; j++) {
-        const double off = (t - t_c) - (double)j * dt;
-        sum += off;
-        moment = fma((double)j - middle, off, moment);
-        t += dt;
+    for (int j = 0; j < K;) {
+        const double next = t + dt, d = ((next + dt) - next) - dt;
+        const long long power = __double_as_longlong(t) & (long long)0xfff0000000000000ull;  // the power of two below |t|
+        const double edge = __longlong_as_double(t < 0.0 ? power : power + 0x0010000000000000ll);
+        const double room = (edge - t) / (dt + d);
+        const int more = room >= (double)(K - 1 - j) ? K - 1 - j : max(0, (int)room);
+        const double n = (double)more, c = n + 1.0;
+        const double run = c * fma(0.5 * n, d, off);  // steps j .. j + more are late by off, off + d, ...
+        sum += run;
+        moment += fma((double)j - middle, run, 0.5 * n * c * fma((2.0 * n + 1.0) * (1.0 / 3.0), d, off));
+        const double last = fma(n, dt + d, t);
+        t = last + dt;
+        off = fma(n, d, off) + ((t - last) - dt);
+        j += more + 1;
     }
     const double n = (double)K;
     s.shift = K > 0 ? sum / n : 0.0;
@@ -391,7 +401,7 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
     //
     // In FP64 corrected for the reference's times.  Its samples are taken at the running sum of the steps (I:836), whose
     // rounding is the same for all steps of the same exponent and for whole stretches of a call, so that a resonant
-    // drive shows it (1 MHz at 100 steps of 10 ns, states 1.1e-8 off at 10 ms, 5e-12 so; 64 mixed instances 551 -> 574 us).
+    // drive shows it (1 MHz at 100 steps of 10 ns, states 1.1e-8 off at 10 ms, 5e-12 so; 64 mixed instances 551 -> 572 us).
     // An interval's samples then lie `shift` later and are stretched about their middle.  The shift, with how the interval's start is rounded relative to the one
     // whose phase was taken at its rounded start, is a small turn of L.  Evolving with H(t_m + (1 + stretch) tau) is
     // evolving with H / (1 + stretch) over (1 + stretch) times as long: L and the bias take the factor here, the ends'
@@ -454,7 +464,6 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
             // consumer lane 4 col + tone % 4 of k-step tone / 4: cosines (even sums), then sines
             double* dst = &sh.table[ph & 1][0][(c * 4 + (tone >> 2)) * 32 + 4 * col + (tone & 3)];
             double2 z = sh.z[r];
-            if (PREC == PREC_FP64 && ph > 0 && ph % kDmmaRestart == 0) z = dmma_restart(f, K, dt, r, m0);
             const double2 rt = sh.rot[slot];
             for (int mm = 0; mm < mc; mm++) {
                 dst[mm * kDmmaChunkDoubles] = z.x;
@@ -539,17 +548,11 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
     __syncthreads();
     const int n_phases = (n_steps + kDmmaPhase - 1) / kDmmaPhase;
     // The step loop, one copy for each kind of step (both inside one loop do not fit the instruction cache).
-    auto steps = [&](auto magnus) {
-        for (int ph = 0; ph < n_phases; ph++) {
+    auto steps = [&](auto magnus, int from, int to) {
+        for (int ph = from; ph < to; ph++) {
             if (ph + 1 < n_phases) fill(ph + 1);
             const int m0 = ph * kDmmaPhase;
             const int mc = min(kDmmaPhase, n_steps - m0);
-            if (PREC == PREC_FP64 && m.rotating && ph > 0 && ph % kDmmaRestart == 0) {
-                const double at = start + (double)m0;
-                const PhasorPair p = phasor_pair(-prw * fma(at, dt, a_lo), -prw * fma(at, dt, a_hi));
-                wa = p.a;
-                wb = p.b;
-            }
             const double* tb = &sh.table[ph & 1][0][lane];
             // Even and odd sums at the two distances of pair mm (tensor path), issued at the end of pair mm - 1, so
             // they are in flight while the next pair begins.
@@ -596,8 +599,25 @@ SS_D void tile_dmma(const MethodConfig& m, const Instance& inst, const FieldDesc
             __syncthreads();  // buffer (ph & 1) is refilled in phase ph + 1
         }
     };
-    if (PREC == PREC_FP32_BULK && sh.magnus != 0) steps(Flag<true>());
-    else steps(Flag<false>());
+    if constexpr (PREC == PREC_FP64) {
+        for (int from = 0; from < n_phases; from += kDmmaRestart) {
+            if (from > 0) {
+                // buffer (from & 1) is filled: the table's recurrences restart at the next phase (each thread's own)
+                for (int r = threadIdx.x; r < kDmmaRecurrences; r += kDmmaThreads)
+                    sh.z[r] = dmma_restart(f, K, dt, r, (from + 1) * kDmmaPhase);
+                if (m.rotating) {
+                    const double at = start + (double)(from * kDmmaPhase);
+                    const PhasorPair p = phasor_pair(-prw * fma(at, dt, a_lo), -prw * fma(at, dt, a_hi));
+                    wa = p.a;
+                    wb = p.b;
+                }
+            }
+            steps(Flag<false>(), from, min(from + kDmmaRestart, n_phases));
+        }
+    } else {
+        if (sh.magnus != 0) steps(Flag<true>(), 0, n_phases);
+        else steps(Flag<false>(), 0, n_phases);
+    }
 
     // The interval's product, in lane 0 of the quad
     combine_segments<false>(after, q);
