@@ -820,6 +820,18 @@ int check_field(const spinsim_plan* p, const spinsim_field* f) {
 }
 }  // namespace
 
+// Whether an instance of an FP64 tone plan's launch (launch_steps output steps in all) runs on the tensor path.  Where
+// the field lets it (tones_on_fp64_tensor_path), it does, but for launches of few output steps, of many fine steps with
+// few tones each: the tensor path has four lanes for an output step, the per-sample kernel up to 32.  Whole calls, tensor
+// path / per sample, spin one: 256 x 512 steps of 1 / 3 / 6 / 9 tones 85 / 49, 85 / 64, 86 / 83 and 85 / 98 us; of 3 tones
+// 256 x 128 40 / 39, 1024 x 256 55 / 49, 2048 x 256 57 / 68, 256 x 8192 about 900 / 571.  A lane count that the caller fixed was
+// fixed for other kernels too, and says nothing about this choice.
+static bool tensor_path_takes(const spinsim_plan* p, const FieldDesc& f, const Instance& inst, int64_t launch_steps) {
+    if (!tones_on_fp64_tensor_path(f, inst)) return false;
+    const int tones = f.tone_count[0] + f.tone_count[1] + f.tone_count[2];
+    return p->m.lanes != 0 || launch_steps > 1024 || inst.n_fine < 256 || tones > 4;
+}
+
 // ------------------------------------------------------------------ single instance
 static int make_instance(const spinsim_plan* p, double t0, double dt_int, double dt_out, int64_t n_out,
                          const double* psi0, Instance* inst) {
@@ -873,7 +885,7 @@ static int evaluate_impl(const spinsim_plan* p, const spinsim_field* field, doub
     Instance inst;
     rc = make_instance(p, t0, dt_int, dt_out, n_out, psi0, &inst);
     if (rc) return rc;
-    if (p->tensor && tones_on_fp64_tensor_path(*reinterpret_cast<const FieldDesc*>(field), inst)) p = p->tensor;
+    if (p->tensor && tensor_path_takes(p, *reinterpret_cast<const FieldDesc*>(field), inst, n_out)) p = p->tensor;
     if (n_out == 0) return SPINSIM_OK;
     if (!time || !u || (with_scan && !state)) return fail(SPINSIM_ERR_INVALID, "output pointer is null");
     if (with_scan && !psi0) return fail(SPINSIM_ERR_INVALID, "psi0 is null");
@@ -1081,7 +1093,7 @@ struct spinsim_batch {
     Tile* tiles_dev;
     int64_t n_tiles;
     Tile* tensor_tiles_dev = nullptr;  // FP64 tones: the tiles of the instances whose field the tensor path takes
-    int64_t n_tensor_tiles = 0;        // (a launch of its own; an instance's route depends on its field alone)
+    int64_t n_tensor_tiles = 0;        // (a launch of its own)
     int32_t* counter;                  // [2]: the two queues
     int lanes;
     float* step_norms = nullptr;  // FP32-bulk: per output step, the sum of |g|^2 over its fine steps
@@ -1366,9 +1378,11 @@ static int batch_prepare(const spinsim_plan* plan, const spinsim_instance* insta
         const Instance* inst = reinterpret_cast<const Instance*>(instances);
         const int per_warp = tile_intervals(plan, b->lanes);
         std::vector<char> on_path;  // FP64 tones: which instances the tensor path takes
+        int64_t total = 0;
+        for (int i = 0; i < n_instances; i++) total += inst[i].n_out;
         if (plan->tensor)
             for (int i = 0; i < n_instances; i++)
-                on_path.push_back(tones_on_fp64_tensor_path(reinterpret_cast<const FieldDesc*>(fields)[inst[i].field], inst[i]));
+                on_path.push_back(tensor_path_takes(plan, reinterpret_cast<const FieldDesc*>(fields)[inst[i].field], inst[i], total));
         std::vector<Tile> evolve_tiles, tensor_tiles, scan_tiles;
         std::vector<int32_t> begin, end;
         Tile *et, *tt, *stl;
