@@ -71,7 +71,7 @@ typedef struct {
     int32_t precision;         /* SPINSIM_PRECISION_* */
     int32_t threads_per_block; /* 0 = library default (128); else a multiple of 32, <= 128 */
     int32_t max_registers;     /* 0 = library default; else the largest build that fits, up to 168, or
-                                  uncapped above (built-in fields), or passed to the JIT linker (user fields) */
+                                  uncapped above (user fields: one capped build, and uncapped above 168) */
     int32_t lanes;             /* lanes per output interval: 0 = auto, else 1, 2, 4, 8, 16 or 32 */
     int32_t variant;           /* SPINSIM_VARIANT_* (FP32-bulk tone plans; ignored otherwise) */
 } spinsim_plan_desc;

@@ -92,11 +92,12 @@ DMMA_MINB = {1: (3, 4, 5, 6), 0: (3, 4, 5)}
 
 
 def user_minb(v):
-    """Resident CTAs a user-field kernel's register allocation must allow: five for spin half (96 registers; the
-    pulse ensemble's time evolution 2709 -> 2637 us against four CTAs), four with spin one (128; the
-    spin-one Rabi sweep's 179 -> 131 us against 208 registers and two CTAs), except for the
-    eight-generator exponential, whose 3 x 3 temporaries would spill in its inner loop."""
-    return 2 if v[3] == 2 else 5 if v[0] == 2 else 4
+    """Resident CTAs that the register allocation of a user-field kernel's images must allow, the default image's first:
+    five for spin half (96 registers; the pulse ensemble's time evolution 2709 -> 2637 us against four CTAs), four
+    with spin one (128; the spin-one Rabi sweep's 179 -> 131 us against 208 registers and two CTAs), except for the
+    eight-generator exponential, whose 3 x 3 temporaries would spill in its inner loop.  And two (no cap) for
+    fields of many live values."""
+    return (2,) if v[3] == 2 else (5, 2) if v[0] == 2 else (4, 2)
 
 
 def gen_sources():
@@ -117,18 +118,19 @@ def gen_sources():
                 units.append(("sass", name, src))
                 reg_decl.append(f'extern "C" const void* spinsim_kget_{name}(void);')
                 builtin_rows.append(f"    {{{v[0]}, {v[1]}, {v[2]}, {v[3]}, {field}, {v[4]}, {minb}, spinsim_kget_{name}}},")
-        name = vname(v)
-        src = os.path.join(GEN, f"u_{name}.cu")
-        body = ("#define SPINSIM_USER_FIELD 1\n"
-                '#include "evolve_kernel.cuh"\n'
-                f'extern "C" __global__ void __launch_bounds__(spinsim::kEvolveThreadsMax, {user_minb(v)}) '
-                f"spinsim_evolve_user(const __grid_constant__ spinsim::EvolveArgs a) {{\n"
-                f"    spinsim::evolve_body<{tmpl(v, 0)}>(a);\n}}\n")
-        write_if_changed(src, body)
-        units.append(("lto", name, src))
-        reg_decl.append(f'extern "C" const unsigned char spinsim_blob_{name}_begin[], spinsim_blob_{name}_end[];')
-        user_rows.append(f"    {{{v[0]}, {v[1]}, {v[2]}, {v[3]}, {v[4]}, spinsim_blob_{name}_begin, "
-                         f"spinsim_blob_{name}_end}},")
+        for minb in user_minb(v):
+            name = f"{vname(v)}_b{minb}"
+            src = os.path.join(GEN, f"u_{name}.cu")
+            body = ("#define SPINSIM_USER_FIELD 1\n"
+                    '#include "evolve_kernel.cuh"\n'
+                    f'extern "C" __global__ void __launch_bounds__(spinsim::kEvolveThreadsMax, {minb}) '
+                    f"spinsim_evolve_user(const __grid_constant__ spinsim::EvolveArgs a) {{\n"
+                    f"    spinsim::evolve_body<{tmpl(v, 0)}>(a);\n}}\n")
+            write_if_changed(src, body)
+            units.append(("lto", name, src))
+            reg_decl.append(f'extern "C" const unsigned char spinsim_blob_{name}_begin[], spinsim_blob_{name}_end[];')
+            user_rows.append(f"    {{{v[0]}, {v[1]}, {v[2]}, {v[3]}, {v[4]}, {minb}, spinsim_blob_{name}_begin, "
+                             f"spinsim_blob_{name}_end}},")
     # Magnus CF4 tone kernels with the field samples on the FP64 tensor path (one per spin mix, precision and
     # register budget; the exponentiators do not enter them).
     dmma_rows = []

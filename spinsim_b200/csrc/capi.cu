@@ -61,7 +61,7 @@ struct BuiltinEntry {
     kernel_getter get;
 };
 struct UserEntry {
-    int dims, integ, expo_h, expo_o, prec;
+    int dims, integ, expo_h, expo_o, prec, minb;
     const unsigned char* begin;
     const unsigned char* end;
 };
@@ -129,11 +129,10 @@ int load_jitlink() {
 enum { JL_INPUT_LTOIR = 3, JL_INPUT_FATBIN = 4 };
 
 int jit_link(const void* kernel_fatbin, size_t kernel_size, const void* user_ltoir, size_t user_size,
-             int max_registers, std::vector<char>* cubin) {
+             std::vector<char>* cubin) {
     int rc = load_jitlink();
     if (rc) return rc;
     std::vector<std::string> opts = {"-arch=sm_100a", "-lto", "-O3"};
-    if (max_registers > 0) opts.push_back("-maxrregcount=" + std::to_string(max_registers));
     std::vector<const char*> optp;
     for (auto& s : opts) optp.push_back(s.c_str());
     void* h = nullptr;
@@ -161,13 +160,12 @@ int jit_link(const void* kernel_fatbin, size_t kernel_size, const void* user_lto
     return SPINSIM_OK;
 }
 
-// The last kernels linked, by everything that goes into a link (the built-in kernel's image, the register cap and
-// the field's whole LTO-IR), most recent first: another plan of the same field, which a program that makes a
+// The last kernels linked, by everything that goes into a link (the built-in kernel's image and the field's whole
+// LTO-IR), most recent first: another plan of the same field, which a program that makes a
 // simulator per call asks for, takes a copy. Even from its disk cache nvJitLink needs milliseconds, more the
 // larger the kernel's image. At most kLinkedKept entries.
 struct Linked {
     const void* kernel;
-    int max_registers;
     std::string field;
     std::vector<char> cubin;
 };
@@ -176,11 +174,11 @@ std::mutex g_linked_mutex;
 std::list<Linked> g_linked;
 
 int linked_cubin(const void* kernel_fatbin, size_t kernel_size, const void* user_ltoir, size_t user_size,
-                 int max_registers, std::vector<char>* cubin) {
+                 std::vector<char>* cubin) {
     try {
         const std::string field((const char*)user_ltoir, user_size);
         auto is_this = [&](const Linked& k) {
-            return k.kernel == kernel_fatbin && k.max_registers == max_registers && k.field == field;
+            return k.kernel == kernel_fatbin && k.field == field;
         };
         {
             std::lock_guard<std::mutex> lock(g_linked_mutex);
@@ -191,11 +189,11 @@ int linked_cubin(const void* kernel_fatbin, size_t kernel_size, const void* user
                 return SPINSIM_OK;
             }
         }
-        const int rc = jit_link(kernel_fatbin, kernel_size, user_ltoir, user_size, max_registers, cubin);
+        const int rc = jit_link(kernel_fatbin, kernel_size, user_ltoir, user_size, cubin);
         if (rc) return rc;
         std::lock_guard<std::mutex> lock(g_linked_mutex);
         if (std::none_of(g_linked.begin(), g_linked.end(), is_this))
-            g_linked.push_front(Linked{kernel_fatbin, max_registers, field, *cubin});
+            g_linked.push_front(Linked{kernel_fatbin, field, *cubin});
         if (g_linked.size() > kLinkedKept) g_linked.pop_back();
         return SPINSIM_OK;
     } catch (const std::bad_alloc&) {
@@ -376,26 +374,41 @@ extern "C" int spinsim_plan_create(const spinsim_plan_desc* desc, const void* fi
             }
         }
     } else {
-        const UserEntry* u = nullptr;
+        // The default image's registers are capped (96 for spin half, 128 with spin one), which a field of many live
+        // values outgrows.  Fields of 25 / 49 / 81 live doubles, 2048 instances of 200 x 50 steps, spin half: 1157 / 1721 /
+        // 3881 us there, 1087 / 1689 / 2496 in the uncapped image (the last in the table); spin one 1163 / 1766 / 2631 and
+        // 1144 / 1722 / 2519.  A budget above 168 takes the uncapped one, and so does, without a budget, a spin-half
+        // field that makes the default one spill (300 to 376 bytes of local memory, 40 to 72 without).
+        const UserEntry *capped = nullptr, *uncapped = nullptr;
         for (const UserEntry& x : kUser)
-            if (x.dims == d.spin_dim && x.integ == d.integration && x.expo_h == eh && x.expo_o == eo && x.prec == d.precision)
-                u = &x;
-        if (u) {
-            std::vector<char> cubin;
-            int rc = linked_cubin(u->begin, (size_t)(u->end - u->begin), field_ltoir, field_ltoir_size, d.max_registers, &cubin);
-            if (rc) {
-                delete p;
-                return rc;
+            if (x.dims == d.spin_dim && x.integ == d.integration && x.expo_h == eh && x.expo_o == eo && x.prec == d.precision) {
+                if (!capped) capped = &x;
+                uncapped = &x;
             }
+        auto load = [&](const UserEntry* u) -> int {
+            if (p->lib) cudaLibraryUnload(p->lib);
+            p->lib = nullptr;
+            std::vector<char> cubin;
+            int rc = linked_cubin(u->begin, (size_t)(u->end - u->begin), field_ltoir, field_ltoir_size, &cubin);
+            if (rc) return rc;
             e = cudaLibraryLoadData(&p->lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0);
             cudaKernel_t k = nullptr;
             if (e == cudaSuccess) e = cudaLibraryGetKernel(&k, p->lib, "spinsim_evolve_user");
-            if (e != cudaSuccess) {
+            if (e != cudaSuccess) return fail(SPINSIM_ERR_LINK, "loading the linked module failed: %s", cudaGetErrorString(e));
+            p->func = (const void*)k;
+            return SPINSIM_OK;
+        };
+        if (capped) {
+            int rc = load(d.max_registers > 168 ? uncapped : capped);
+            cudaFuncAttributes attr;
+            if (!rc && d.max_registers <= 0 && d.spin_dim == 2 && cudaFuncGetAttributes(&attr, p->func) == cudaSuccess &&
+                attr.localSizeBytes > 200)
+                rc = load(uncapped);
+            if (rc) {
                 if (p->lib) cudaLibraryUnload(p->lib);
                 delete p;
-                return fail(SPINSIM_ERR_LINK, "loading the linked module failed: %s", cudaGetErrorString(e));
+                return rc;
             }
-            p->func = (const void*)k;
         }
     }
     if (!p->func) {
