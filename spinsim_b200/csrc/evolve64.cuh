@@ -235,13 +235,19 @@ SS_D bool hold_steps(const FieldDesc& f, int dim, bool turns, const StepRule& st
 // Steps j .. j1 - 1 of a spin-one interval whose quadratic shift is non-zero: full 3 x 3 exponentials
 // and products, from the product u of the steps before.  On entry step j's generators are in g and st is at
 // step j + 1.  Out of line, its state passed by value, so that the registers of the common
-// SU(2) loop are allocated without this path's.
+// SU(2) loop are allocated without this path's; loops are kept rolled, since a user field's kernel is linked when
+// its simulator is made (with the other rolled loops of the 3 x 3 path an image of 567 -> 455 KB, linked in 0.8 ->
+// 0.3 to 0.7 s, and no slower: 4001 x 50 steps 37.6 -> 37.0 us).
 template <int INTEG, int FIELD>
 __device__ __noinline__ Mat<3> spin_one_quadratic_steps64(const MethodConfig& m, const FieldDesc& f, Steps<4> st,
                                                           Mat<3> u, Generators4 g, int j0, int j, int j1) {
     for (;;) {
-        spin_one_step64(m, u, g.a);
-        if constexpr (INTEG != INTEG_EULER) spin_one_step64(m, u, g.b);
+#pragma unroll 1
+        for (int e = 0; e < (INTEG == INTEG_EULER ? 1 : 2); e++) {
+            spin_one_step64(m, u, g.a);
+#pragma unroll
+            for (int c = 0; c < 4; c++) g.a[c] = g.b[c];
+        }
         if (++j >= j1) return u;
         st.template restart<INTEG>(j, j0);
         step_generators<FIELD, 4, INTEG, true>(f, st, g.a, g.b);
@@ -352,7 +358,9 @@ SS_D void finish_interval(const MethodConfig& m, V v, double rw, double dt_out, 
     }
     if (product_out == nullptr) return;
     const int lane = threadIdx.x & 31;
-#pragma unroll
+    // unrolled for the pairs (400 pulse trains 789 -> 777 us); 3 x 3 products would be most of a kernel's code
+    constexpr int kUnroll = sizeof(V) == sizeof(Su2p) ? 5 : 1;
+#pragma unroll kUnroll
     for (int s = 1; s < 32; s <<= 1) {
         const V later = shfl_down_operator(v, s);
         if ((lane & (2 * s - 1)) == 0) v = later_times(later, v);

@@ -200,10 +200,8 @@ SS_D Mat<3> expo_lt_one_m1(const double* g, int hypercubes, double precision) {
     r.a[1][2] = sa * ((eq * epc) * ez);           // exp(i(q - p + z))
     cem = cos_exp_m1(0.5 * a, z - q);
     r.a[2][2] = cem * (cem + c64{2.0, 0.0});
-    for (int h = 0; h < hypercubes; h++) {
-        r = square_m1(r);
-        r = square_m1(r);
-    }
+#pragma unroll 1
+    for (int h = 0; h < 2 * hypercubes; h++) r = square_m1(r);
     return r;
 }
 
