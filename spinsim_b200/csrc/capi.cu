@@ -782,6 +782,7 @@ int launch_scan(const Instance* inst_dev, const Instance* single, const ScanBuff
 
 // early: the launch may start before the preceding kernel (the tensor path's constants) completes.
 int launch_evolve(const spinsim_plan* p, EvolveArgs a, int64_t tiles, cudaStream_t s, bool early = false) {
+    if (p->cta_tiles && !a.dmma_consts) return fail(SPINSIM_ERR_INVALID, "the tensor path's constants are missing");
     int64_t blocks = p->cta_tiles ? tiles : (tiles * 32 + p->block - 1) / p->block;
     if (a.tile_counter) {  // persistent: fill the device once, warps pull tiles from the queue
         const int64_t resident = (int64_t)p->sm_count * p->blocks_per_sm;

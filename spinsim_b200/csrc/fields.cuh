@@ -99,8 +99,7 @@ SS_D double table_sample(const TableChannel& tb, double ts) {
 // output interval).  The interval [time[i], time[i+1]] that holds a sample strictly inside it is
 // unique, so advancing the cursor finds the same index as the reference's search; a sample that
 // lands exactly on a table time (or outside the table) goes to the reference's search, which picks
-// among the touching intervals as the reference does.  Results are therefore identical to
-// table_sample; the cursor only removes the bisection's chain of dependent loads.
+// among the touching intervals as the reference does.  The cursor removes the bisection's chain of dependent loads.
 //
 // A cursor also keeps the channel (gain and bias included) on (t_lo, t_hi): its constant value (a zero-order
 // hold, or a channel without a table, on the whole line), or the coefficients of its linear or cubic piece in
