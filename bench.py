@@ -85,12 +85,11 @@ def instances(ss, specs):
 FLOPS_FP64_PLAIN = {2: 278, 3: 278}
 FLOPS_BULK = {2: {"fp64": 175, "fp32": 36}, 3: {"fp64": 175, "fp32": 36}}
 # DRAM bytes (read + write) of one full-size FP32-bulk time-evolution launch of this workload (the
-# tensor-path kernel at 96 registers, writing the scan's tile partials and each output step's SU(2)
+# tensor-path kernel at 128 registers, writing the scan's tile partials and each output step's SU(2)
 # pair beside U: 46 MB of the writes are that scan scratch, not outputs), from one capture of
 # `ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none -k regex:evolve_dmma -c 1`
-# on `bench.py --workload profile --profile-size full --precision fp32_bulk --max-registers 96 --variant 0`.
-# The capture is of the kernel with 192 sample flops per step; what it reads and writes has not changed since.
-TRAFFIC_BYTES_PER_LAUNCH = 7328000 + 137223936
+# on `bench.py --workload profile --profile-size full --precision fp32_bulk --max-registers 128 --variant 0`.
+TRAFFIC_BYTES_PER_LAUNCH = 8372992 + 137942016
 
 
 def algorithmic_bytes(specs):
