@@ -838,12 +838,13 @@ int check_field(const spinsim_plan* p, const spinsim_field* f) {
 // the field lets it (tones_on_fp64_tensor_path), it does, but for launches of few output steps, of many fine steps with
 // few tones each: the tensor path has four lanes for an output step, the per-sample kernel up to 32.  Whole calls, tensor
 // path / per sample, spin one: 256 x 512 steps of 1 / 3 / 6 / 9 tones 85 / 49, 85 / 64, 86 / 83 and 85 / 98 us; of 3 tones
-// 256 x 128 40 / 39, 1024 x 256 55 / 49, 2048 x 256 57 / 68, 256 x 8192 about 900 / 571.  A lane count that the caller fixed was
-// fixed for other kernels too, and says nothing about this choice.
+// 256 x 128 40 / 39, 1024 x 256 55 / 49, 2048 x 256 57 / 68, 256 x 8192 about 900 / 571.  A caller who fixed fewer lanes
+// gets the tensor path's four (4 x 1000 steps of 3 tones: 129 us, per sample with 16 lanes 166).
 static bool tensor_path_takes(const spinsim_plan* p, const FieldDesc& f, const Instance& inst, int64_t launch_steps) {
     if (!tones_on_fp64_tensor_path(f, inst)) return false;
     const int tones = f.tone_count[0] + f.tone_count[1] + f.tone_count[2];
-    return p->m.lanes != 0 || launch_steps > 1024 || inst.n_fine < 256 || tones > 4;
+    const bool all_lanes = p->m.lanes == 0 || p->m.lanes == 32;
+    return !all_lanes || launch_steps > 1024 || inst.n_fine < 256 || tones > 4;
 }
 
 // ------------------------------------------------------------------ single instance

@@ -25,7 +25,9 @@ def test_both_routes(cuda, spin, n, k, tones, tensor):
     args = (0.0, (n + 0.5) * dt_out, 10e-9, dt_out, sq.plus_z)
     time, u, state, _ = O.evaluate(sq.dimension, O.Field(8), p, *args)
     batch = Batch([Instance(sq, *args, field=field)])
-    assert batch.launch_info()["tile_intervals"] == (32 if tensor else 1)
+    for lanes, per_sample in ((0, not tensor), (32, not tensor), (16, False)):
+        info = Batch([Instance(sq, *args, field=field)], lanes=lanes).launch_info()
+        assert info["tile_intervals"] == (1 if per_sample else 32)
     batch.run()
     for r in (batch.result(0), ss.Simulator(field, sq).evaluate(*args)):
         assert np.array_equal(r.time, time)
